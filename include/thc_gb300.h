@@ -99,8 +99,8 @@ int thc_ctx_destroy(thc_ctx* ctx);
 /* Run on a caller stream (a cudaStream_t); NULL restores the context's own stream. */
 int thc_ctx_set_stream(thc_ctx* ctx, void* cuda_stream);
 /* Named numeric options: "slices_p", "slices_z", "slices_m" (sliced-GEMM depths of the
- * P, zeta and Coulomb products, 2..6); "gemm_tc" (1 = tcgen05 tensor-core kernel, the
- * default; 0 = warp-level mma.sync kernel); "km_prune" (1 = spatially pruned k-means
+ * P, zeta and Coulomb products, 2..6); "gemm_tc" (1 = tcgen05 tensor-core kernels, the
+ * default; 0 = warp-level mma.sync kernel, and FP64 FMAs for the FP64 products); "km_prune" (1 = spatially pruned k-means
  * assignment, the default; 0 = exhaustive scan -- both exact); "graphs" (1 = replay the
  * k-means iteration block as a CUDA graph, the default); "tc_bk" (k-step per
  * pipeline stage of the tensor-core kernel: 32, the default, or 16; setting it turns the

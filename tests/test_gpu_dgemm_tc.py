@@ -1,0 +1,81 @@
+"""The FP64 path's products on the tensor cores (csrc/dgemm_tc.cu) at the edges of their tiles:
+the matrices against the oracle, the two routes (option gemm_tc) against each other, and an
+orbital value that is not finite."""
+import numpy as np
+import pytest
+
+import oracle
+from thcpp_gb300 import capi, synth
+
+pytestmark = pytest.mark.gpu
+
+_SYS = {}
+
+
+def _system(mesh):
+    if mesh not in _SYS:
+        lat, atoms = synth.diamond_supercell(1)
+        s = synth.make_system(f"edge{mesh}", lat, atoms, mesh, 32, 8, 4321, 55)
+        _SYS[mesh] = (s, oracle.kmeans_system(s).idx)
+    return _SYS[mesh]
+
+
+def _cplx(a):
+    return a[..., 0] + 1j * a[..., 1]
+
+
+def _rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+# Points on either side of the 128-row and 64-column tile edges; meshes whose N_g and half
+# spectrum are odd, below and above a multiple of the tiles.
+@pytest.mark.parametrize("mesh", [(24, 24, 24), (23, 25, 27)])
+@pytest.mark.parametrize("nmu", [63, 127, 128, 129, 193, 256])
+def test_isdf_tile_edges(gpu_ctx_fp64, mesh, nmu):
+    s, idx_all = _system(mesh)
+    idx = np.ascontiguousarray(np.sort(np.random.default_rng(nmu).permutation(idx_all)[:nmu]))
+    pm = s.phi[idx]
+    # A relative perturbation eps of Z and C moves zeta, and with it M, by cond(C) eps.
+    tol = np.linalg.cond((pm @ pm.T) ** 2) * np.finfo(float).eps
+    ref = oracle.isdf_real(s.phi, idx, s.mesh, s.coulG)
+    got = {}
+    for tc in (1, 0):
+        gpu_ctx_fp64.set_option("gemm_tc", tc)
+        try:
+            got[tc] = gpu_ctx_fp64.isdf(s.phi, idx, s.mesh, s.coulG)
+        finally:
+            gpu_ctx_fp64.set_option("gemm_tc", 1)
+        assert got[tc]["status"] == 0
+        assert _rel(_cplx(got[tc]["M"]), ref["M"]) < tol
+    assert _rel(_cplx(got[1]["M"]), _cplx(got[0]["M"])) < tol
+
+
+def test_negative_weights_and_symmetry(gpu_ctx_fp64):
+    """A Coulomb kernel with both signs: the product keeps its weights on one side."""
+    s, idx = _system((24, 24, 24))
+    v = s.coulG * np.where(np.arange(s.ng) % 7 == 3, -0.5, 1.0)
+    r = gpu_ctx_fp64.isdf(s.phi, idx, s.mesh, v, raise_on_error=False)
+    ref = oracle.isdf_real(s.phi, idx, s.mesh, v)
+    pm = s.phi[idx]
+    tol = np.linalg.cond((pm @ pm.T) ** 2) * np.finfo(float).eps
+    assert _rel(_cplx(r["M"]), ref["M"]) < tol
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_non_finite_orbital(gpu_ctx_fp64, value):
+    """A value that is not finite, at a point that is no interpolating point, spoils every
+    interpolating vector there and so M, on either route."""
+    s, idx = _system((24, 24, 24))
+    phi = s.phi.copy()
+    g = int(np.setdiff1d(np.arange(s.ng), idx)[100])
+    phi[g, 5] = value
+    for tc in (1, 0):
+        gpu_ctx_fp64.set_option("gemm_tc", tc)
+        try:
+            r = gpu_ctx_fp64.isdf(phi, idx, s.mesh, s.coulG, raise_on_error=False)
+            z = gpu_ctx_fp64.interpolating_vectors(s.ng, s.nmu) if r["status"] == 0 else None
+        finally:
+            gpu_ctx_fp64.set_option("gemm_tc", 1)
+        assert r["status"] == capi.THC_ERR_NOT_PD and r["stats"].chol_m_info == 1
+        assert z is None and not np.isfinite(r["M"][..., 0]).any()

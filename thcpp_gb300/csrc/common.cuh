@@ -67,6 +67,10 @@ enum Slot : int {
   WS_ORB,           // (N_o + N_occ) x N_mu x 2 orbital outputs staged for a host copy
   WS_REFINE,        // 3 x nmu x nmu doubles: refinement polynomial, L^{-1} T (mixed)
   WS_EQUIL,         // nmu doubles + nmu ints: power-of-two equilibration of C (mixed)
+  WS_T64_A,         // digits of dgemm's tensor-core route
+  WS_T64_B,
+  WS_T64_E,         // its row exponents and maxima
+  WS_T64_ERR,       // its error flag
   WS_NSLOTS
 };
 
@@ -101,7 +105,9 @@ struct Ctx {
   // zeta_hat): 4 slices leave 1.3e-6 on M at N_g 1.26e6 (a bias from the dropped level-4
   // pairs on the diagonal), 5 slices 2.7e-7.
   int slices_m = 5;
-  int gemm_tc = 1;      // 1: tcgen05 sliced GEMM, 0: mma.sync sliced GEMM
+  // 1: tcgen05 GEMMs; 0: mma.sync sliced GEMM (mixed path) and FP64 FMAs (dgemm).
+  int gemm_tc = 1;
+  int* tc64_err = nullptr;   // device flag: a bounded wait of dgemm's tensor-core route gave up
   int km_prune = 1;     // 1: spatially pruned k-means assign, 0: exhaustive
   int use_graphs = 1;   // capture the k-means iteration block in a CUDA graph
   // k-step per pipeline stage of the tensor-core GEMM: 32 (2-3 stages of all slices, the

@@ -356,6 +356,11 @@ static void launch_dgemm(const GemmArgs& g, cudaStream_t s)
 int dgemm(Ctx* c, const GemmArgs& g_in)
 {
   if (g_in.M <= 0 || g_in.N <= 0) return THC_OK;
+  if (dgemm_tc_fits(c, g_in)) {
+    bool done = false;
+    const int st = dgemm_tc(c, g_in, &done);
+    if (st || done) return st;
+  }
   GemmArgs g = g_in;
   if (g.ksplit <= 1 && !g.part) {
     // Tile and split-K so that the grid covers the SMs about twice.
@@ -384,10 +389,13 @@ int dgemm(Ctx* c, const GemmArgs& g_in)
   else if (g.tile == 32) launch_dgemm<32>(g, c->stream);
   else launch_dgemm<64>(g, c->stream);
   THC_LAUNCHED(c, "dgemm");
-  if (g.ksplit > 1) {
-    dgemm_reduce<<<(unsigned)cdiv(g.M * g.N, 256), 256, 0, c->stream>>>(g);
-    THC_LAUNCHED(c, "dgemm_reduce");
-  }
+  return g.ksplit > 1 ? dgemm_reduce_partials(c, g) : THC_OK;
+}
+
+int dgemm_reduce_partials(Ctx* c, const GemmArgs& g)
+{
+  dgemm_reduce<<<(unsigned)cdiv(g.M * g.N, 256), 256, 0, c->stream>>>(g);
+  THC_LAUNCHED(c, "dgemm_reduce");
   return THC_OK;
 }
 

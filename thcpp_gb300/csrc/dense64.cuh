@@ -21,6 +21,8 @@ struct GemmArgs {
   long long ldc = 0;
   const double* dk = nullptr;
   int dk_shift = 0;
+  const double* dkr = nullptr;       // sqrt(dk), where A == B and no dk is negative: lets the
+                                     // tensor-core route cut one operand for both sides
   double alpha = 1.0, beta = 0.0;
   int mode = GEMM_STORE;
   int lower_only = 0;
@@ -36,6 +38,7 @@ struct GemmArgs {
   int lower_offset = 0;              // lower_only keeps n <= m + lower_offset (C's own indices)
   int no_split = 0;                  // no split of K (no shared partial buffer: a GEMM that
                                      // runs beside others on a second stream)
+  int fma_only = 0;                  // keep the FMA kernel (dgemm_tc_fits)
   int tile = 64;                     // CTA tile edge (64, 32 or 16; chosen by dgemm)
 };
 
@@ -50,6 +53,22 @@ struct CholStatus {
 // that the grid covers the GPU (the FP64 pipe of one SM is narrow, so small GEMMs must spread
 // over many SMs); split partials are summed in split order (deterministic).
 int dgemm(Ctx* c, const GemmArgs& g);
+// Products the tensor-core route takes (dgemm_tc.cu): at least this much work, no skip flag,
+// no aliasing, no known-zero triangle and no caller's split.  Below it the FMA kernel's one
+// launch is as fast as the cut of two operands and the product (97 x 1001 x 200, 3.9e7: 50 us
+// against 36; 130 x 130 x 1000, 3.4e7: 52 against 46; 130 x 200 x 1000 row-contiguous, 5.2e7:
+// 80 against 85; 256 x 4096 x 32, 6.7e7: 73 against 31).
+constexpr double kDgemmTcFlops = 4e7;
+constexpr size_t kDgemmTcBytes = (size_t)3 << 30;   // digit buffers: larger products run in panels
+bool dgemm_tc_fits(const Ctx* c, const GemmArgs& g);
+// Runs g on the tensor cores; *done = false (and THC_OK) when it does not take it (no room
+// for the digits), and the caller runs the FMA kernel.
+int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done);
+// Clears the device flag that a bounded wait of the kernel sets (c->tc64_err).  Every entry
+// point whose products may take this route calls it first and reads the flag at its end.
+int dgemm_tc_begin(Ctx* c);
+// Split-K partials summed in split order, then the epilogue, into C.
+int dgemm_reduce_partials(Ctx* c, const GemmArgs& g);
 // Cholesky with GEMM panels; dinv receives the inverted NB x NB diagonal blocks
 // (NB = 64: ceil(n/64) x 64 x 64 doubles).
 int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholStatus* cs,

@@ -262,6 +262,7 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   double* orb_dev = out_orb ? (orb_host ? stage : out_orb) : nullptr;
   double* occ_dev = out_orb_occ ? (occ_host ? stage + 2LL * nmu * no : out_orb_occ) : nullptr;
   THC_CUDA(c, cudaMemsetAsync(scr, 0, 1024, s));
+  if ((st = dgemm_tc_begin(c))) return st;
   THC_CUDA(c, cudaEventRecord(c->ev0, s));
   gather_pairs<<<(int)cdiv((long long)nmu * no, 256), 256, 0, s>>>(phi, ng, no, idx, nmu, pmu,
                                                                   pmu_rot, orb_dev, bad);
@@ -370,11 +371,14 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   THC_CUDA(c, cudaEventRecord(c->ev1, s));
   if (out_M) THC_CUDA(c, cudaMemcpyAsync(out_M, mcx, sizeof(double) * 2 * nn, cudaMemcpyDefault, s));
   GjStatus hg{};
-  int hbad = 0;
+  int hbad = 0, herr = 0;
+  THC_CUDA(c, cudaMemcpyAsync(&herr, c->tc64_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hg, gs, sizeof(GjStatus), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaStreamSynchronize(s));
   if (hbad) return set_error(c, THC_ERR_ARG, "thc_isdf_half_complex: interpolating index out of range");
+  if (herr)
+    return set_error(c, THC_ERR_TIMEOUT, "thc_isdf_half_complex: tensor-core GEMM wait timed out");
   if (stats) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);

@@ -60,9 +60,11 @@ __global__ void gather_rows(const double* __restrict__ phi, long long ng, int no
   }
 }
 
-// Half-spectrum Coulomb weights: dsym = w (v(G) + v(-G))/2, danti = w (v(G) - v(-G))/2.
+// Half-spectrum Coulomb weights: dsym = w (v(G) + v(-G))/2, danti = w (v(G) - v(-G))/2, and
+// root = sqrt|dsym|, for a product that takes half the weight on each side.
 __global__ void coulomb_weights(const double* __restrict__ v, int n0, int n1, int n2,
-                                double* dsym, double* danti, int* n_anti)
+                                double* dsym, double* danti, double* root, int* n_anti,
+                                int* n_neg)
 {
   int nc = n2 / 2 + 1;
   long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -75,7 +77,10 @@ __global__ void coulomb_weights(const double* __restrict__ v, int n0, int n1, in
   double vp = v[((long long)k0 * n1 + k1) * n2 + k2];
   double vn = v[((long long)j0 * n1 + j1) * n2 + j2];
   double w = (k2 == 0 || (n2 % 2 == 0 && k2 == n2 / 2)) ? 1.0 : 2.0;
-  dsym[e] = w * 0.5 * (vp + vn);
+  const double d = w * 0.5 * (vp + vn);
+  dsym[e] = d;
+  root[e] = sqrt(fabs(d));
+  if (d < 0.0) atomicAdd(n_neg, 1);
   double a = w * 0.5 * (vp - vn);
   danti[e] = a;
   if (a != 0.0) atomicAdd(n_anti, 1);
@@ -307,7 +312,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   double* zt = (double*)ws_get(c, WS_ZT, sizeof(double) * nmu * ng);
   double* zeta = (double*)ws_get(c, WS_ZETA, sizeof(double) * nmu * ng);
   double* zhat = (double*)ws_get(c, WS_ZHAT, sizeof(double) * 2 * nmu * nc);
-  double* dsym = (double*)ws_get(c, WS_DSYM, sizeof(double) * nc);
+  double* dsym = (double*)ws_get(c, WS_DSYM, 2 * sizeof(double) * nc);   // and their roots
   double* danti = (double*)ws_get(c, WS_DANTI, sizeof(double) * nc);
   double* Mw = (double*)ws_get(c, WS_M, sizeof(double) * 4 * nn);  // Re M lower, X, complex M
   double* Lw = (double*)ws_get(c, WS_L, sizeof(double) * 2 * nn);
@@ -326,6 +331,8 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   double* zero = dmean + 3;
   int* bad = (int*)(scr + 512);
   int* n_anti = bad + 1;
+  int* n_neg = bad + 2;
+  double* droot = dsym + nc;
   // Orbital outputs: written in place on the device, else staged for the host copy.
   double* orb_dev = nullptr;
   double* occ_dev = nullptr;
@@ -339,8 +346,15 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   if (out_orb) orb_dev = orb_host ? orb_stage : out_orb;
   if (half && out_orb_occ) occ_dev = occ_host ? orb_stage + 2 * (long long)nmu * no : out_orb_occ;
   THC_CUDA(c, cudaMemsetAsync(scr + 512, 0, 64, s));
+  if ((st = dgemm_tc_begin(c))) return st;
   THC_CUDA(c, cudaEventRecord(c->ev0, s));
 
+  // The Coulomb weights depend on the kernel only: with them first, their counts reach the
+  // host with C's factorisation status and cost no wait of their own.
+  coulomb_weights<<<(int)cdiv(nc, 256), 256, 0, s>>>(coul, n0, n1, n2, dsym, danti, droot, n_anti,
+                                                     n_neg);
+  THC_LAUNCHED(c, "coulomb_weights");
+  int h_counts[2] = {0, 0};            // n_anti, n_neg
   gather_rows<<<(int)cdiv((long long)nmu * kw, 256), 256, 0, s>>>(phi, ng, kw, idx, nmu, phimu,
                                                                   cplx ? nullptr : orb_dev, bad);
   THC_LAUNCHED(c, "gather_rows");
@@ -451,6 +465,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   CholStatus hcs{};
   if ((st = factor(shift_rel > 0.0 ? shift_rel : 0.0))) return st;
   shifted = shift_rel > 0.0;
+  THC_CUDA(c, cudaMemcpyAsync(h_counts, n_anti, sizeof(h_counts), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hcs, cs, sizeof(CholStatus), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaStreamSynchronize(s));
   if (hcs.flag) {
@@ -495,10 +510,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   }
   // FFT of every interpolating vector.
   if ((st = fft_forward(c, n0, n1, n2, nmu, CUFFT_D2Z, zeta, zhat))) return st;
-  coulomb_weights<<<(int)cdiv(nc, 256), 256, 0, s>>>(coul, n0, n1, n2, dsym, danti, n_anti);
-  THC_LAUNCHED(c, "coulomb_weights");
-  int h_anti = 0;
-  THC_CUDA(c, cudaMemcpyAsync(&h_anti, n_anti, sizeof(int), cudaMemcpyDeviceToHost, s));
+  const int h_anti = h_counts[0];
   // Re M (lower) = sum_k zh[mu,k] dsym[k/2] zh[nu,k] over interleaved (re, im) pairs.
   double* mre = Mw;
   double* xim = Mw + nn;
@@ -509,18 +521,11 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
     g.A = zhat; g.sam = 2 * nc; g.sak = 1;
     g.B = zhat; g.sbn = 2 * nc; g.sbk = 1;
     g.dk = dsym; g.dk_shift = 1;
+    g.dkr = h_counts[1] ? nullptr : droot;
     g.C = mre; g.ldc = nmu; g.lower_only = 1;
     if (2 * nc > 0x7fffffffLL) return set_error(c, THC_ERR_SHAPE, "thc_isdf: mesh too large");
-    // Long K, small output: split K over CTAs (deterministic reduction in split order).
-    long long tiles = cdiv(nmu, 64) * (cdiv(nmu, 64) + 1) / 2;
-    g.ksplit = (int)std::max<long long>(1, std::min<long long>(cdiv(2 * 152, tiles), cdiv(2 * nc, 4096)));
-    if (g.ksplit > 1) {
-      g.part = (double*)ws_get(c, WS_PART, sizeof(double) * g.ksplit * nn);
-      if (!g.part) return set_error(c, THC_ERR_NOMEM, "thc_isdf: split-K buffer");
-    }
     if ((st = dgemm(c, g))) return st;
   }
-  THC_CUDA(c, cudaStreamSynchronize(s));
   if (h_anti > 0) {
     // X = sum_c zh_re[mu,c] danti[c] zh_im[nu,c];  Im M = X - X^T.
     GemmArgs g;
@@ -559,13 +564,15 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   if (out_L && !half)
     THC_CUDA(c, cudaMemcpyAsync(out_L, Lout, sizeof(double) * 2 * nn, cudaMemcpyDefault, s));
   CholStatus hm{};
-  int hbad = 0;
+  int hbad = 0, herr = 0;
+  THC_CUDA(c, cudaMemcpyAsync(&herr, c->tc64_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hm, csm, sizeof(CholStatus), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
   double hshift = 0.0;
   THC_CUDA(c, cudaMemcpyAsync(&hshift, shift_dev, sizeof(double), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaStreamSynchronize(s));
   if (hbad) return set_error(c, THC_ERR_ARG, "thc_isdf: interpolating index out of range");
+  if (herr) return set_error(c, THC_ERR_TIMEOUT, "thc_isdf: tensor-core GEMM wait timed out");
   c->zeta_last = zeta;
   c->zeta_elem = sizeof(double);
   c->zeta_ng = ng;

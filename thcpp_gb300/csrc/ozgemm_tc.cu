@@ -25,7 +25,6 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
-#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cmath>
@@ -36,134 +35,18 @@
 
 #include "common.cuh"
 #include "ozgemm.cuh"
+#include "tc_ptx.cuh"
 
 namespace thc {
 
 namespace {
 
-constexpr int TBM = 128;
 constexpr int kChunkK = 512;            // exact levels are drained every 512 k
 constexpr int kStageBudget = 200 * 1024;  // shared memory for the stage buffers (BN = 128)
 constexpr int kStageBudget64 = 80 * 1024;  // the same for BN = 64 (two CTAs per SM)
 constexpr int kSmemGuard = 16 * 1024;   // slack after the buffers (descriptor reads stay inside)
 constexpr int TEPI_WARPS = 8;
 constexpr int TTHREADS = 32 * (2 + TEPI_WARPS);
-constexpr long long kDrainLimit = 1LL << 22;   // teardown waits after an abort
-
-__device__ __forceinline__ uint32_t su32(const void* p)
-{
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(su32(b)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(su32(b)), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* b)
-{
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(su32(b)) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity)
-{
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(su32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait: false (and *abort set) when the barrier phase does not complete within
-// `limit` polls (the context option "spin_limit"; 0 gives up at once).
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort,
-                                          long long limit)
-{
-  for (long long i = 0; i < limit; i++) {
-    if (mbar_try(b, parity)) return true;
-    if (*abort) return false;
-  }
-  *abort = 1;
-  return false;
-}
-
-// Teardown wait after an abort: polls a phase a bounded number of times, whatever *abort.
-__device__ __forceinline__ void mbar_drain(uint64_t* b, uint32_t parity)
-{
-  for (long long i = 0; i < kDrainLimit; i++)
-    if (mbar_try(b, parity)) return;
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,
-                                            uint64_t* bar)
-{
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
-          su32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(su32(bar))
-      : "memory");
-}
-
-// UMMA shared-memory descriptor, K-major with the rows of one tile BK bf16 (2 BK bytes)
-// long: BK = 32 uses the 64-byte swizzle (8-row groups 512 B apart), BK = 16 the 32-byte
-// swizzle (groups 256 B apart).
-template <int BK>
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr)
-{
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
-  d |= (uint64_t)1 << 16;                       // leading byte offset (unused when swizzled)
-  d |= (uint64_t)((8 * 2 * BK) >> 4) << 32;     // stride byte offset: one 8-row group
-  d |= (uint64_t)1 << 46;                       // descriptor version
-  d |= (uint64_t)(BK == 32 ? 4 : 6) << 61;      // layout: 64- or 32-byte swizzle
-  return d;
-}
-
-// kind::f16 instruction descriptor: D f32, A/B bf16, both K-major, M = 128, N = BN.
-template <int BN>
-__host__ __device__ constexpr uint32_t idesc()
-{
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-         ((uint32_t)(TBM >> 4) << 24);
-}
-
-template <int BN>
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t acc)
-{
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc<BN>()), "r"(acc));
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar)
-{
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                   su32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v)
-{
-  uint32_t r[8];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
-}
 
 // Error-free transformations in FP32 (Knuth's TwoSum; Dekker's FastTwoSum for |a| >= |b|).
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
@@ -996,27 +879,12 @@ __global__ void __launch_bounds__(TTHREADS, 1)
   }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 get_encoder()
-{
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    cudaDriverEntryPointQueryResult q;
-    void* p = nullptr;
-    // The entry point with the ABI of CUDA 12.0, which the PFN type above describes.
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
-                                         &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-  }
-  return fn;
-}
-
 // 2-D map of a slice buffer: rows of `width` bf16 (kpad for plain storage, 32 for tiled),
 // box bk x box_rows with the swizzle that matches the UMMA descriptor (sdesc<bk>).
 int make_map(Ctx* c, CUtensorMap* map, const void* base, long long width, long long rows,
              int box_rows, int bk)
 {
-  auto enc = get_encoder();
+  auto enc = tensor_map_encoder();
   if (!enc) return set_error(c, THC_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
   // Row coordinates are 32-bit in the copy instruction.
   if (rows > 0x7fffffffLL) return set_error(c, THC_ERR_SHAPE, "ozgemm_tc: slice buffer too tall");
