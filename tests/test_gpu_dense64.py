@@ -1,7 +1,6 @@
-"""The FP64 path's products on the tensor cores (csrc/dgemm_tc.cu) at the edges of their tiles:
-the matrices against the oracle, the two routes (option gemm_tc) against each other, and an
-orbital value that is not finite."""
-import numpy as np
+"""The FP64 dense kernels at the edges of their tiles: products on the tensor cores
+(csrc/dgemm_tc.cu) against the oracle and the FMA route (option gemm_tc), an orbital value that
+is not finite, and the Cholesky (csrc/dense64.cu) with a breakdown at every kind of position."""
 import pytest
 
 import oracle
@@ -47,6 +46,9 @@ def test_isdf_tile_edges(gpu_ctx_fp64, mesh, nmu):
         finally:
             gpu_ctx_fp64.set_option("gemm_tc", 1)
         assert got[tc]["status"] == 0
+        L = _cplx(got[tc]["L"])
+        # The factor's backward error: n eps, for the blocked loop as for the plain one.
+        assert _rel(L @ L.conj().T, _cplx(got[tc]["M"])) < nmu * np.finfo(float).eps
         assert _rel(_cplx(got[tc]["M"]), ref["M"]) < tol
     assert _rel(_cplx(got[1]["M"]), _cplx(got[0]["M"])) < tol
 
@@ -79,3 +81,17 @@ def test_non_finite_orbital(gpu_ctx_fp64, value):
             gpu_ctx_fp64.set_option("gemm_tc", 1)
         assert r["status"] == capi.THC_ERR_NOT_PD and r["stats"].chol_m_info == 1
         assert z is None and not np.isfinite(r["M"][..., 0]).any()
+
+
+# Positions at the edges of the Cholesky's panels (4 columns), of the warp that owns the rows
+# (32) and of its blocks (64).
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("pos", [1, 3, 4, 31, 32, 36, 63, 64, 67, 127, 129])
+def test_breakdown_position(gpu_ctx_fp64, gpu_ctx_mixed, prec, pos):
+    """A repeated interpolating point makes C singular at that pivot, in any block."""
+    ctx = gpu_ctx_fp64 if prec == "fp64" else gpu_ctx_mixed
+    s, idx_all = _system((24, 24, 24))
+    idx = np.ascontiguousarray(np.random.default_rng(7).permutation(idx_all)[:130])
+    idx[pos] = idx[pos - 1]
+    r = ctx.isdf(s.phi, idx, s.mesh, s.coulG)
+    assert r["stats"].chol_c_info == pos + 1 and r["stats"].rank_deficient == 1

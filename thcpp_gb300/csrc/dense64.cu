@@ -122,122 +122,154 @@ __global__ void dgemm_reduce(GemmArgs g)
 
 // ---- Cholesky (lower, in place, row-major) --------------------------------------
 
-// Diagonal block edge of the blocked Cholesky.  The serial part (the diagonal blocks, one
-// SM each) is a latency chain of NB dependent steps per block; 32 x 32 blocks (a quarter of
-// the FP64 work per block) measured no faster at n = 256 (the factorisations of C and M:
-// 0.95 ms against 0.99 ms, and the triangular inverse 0.26 ms against 0.16 ms with twice the
-// block rows), so both edges stay available and 64 is used.
-inline int chol_nb(int) { return 64; }
+// Edge of the diagonal blocks of the blocked Cholesky.
+constexpr int NB = 64;
 
 // 1/sqrt(d) for a positive normal d: an FP32 seed y0 (relative error e0 < 2^-22), then one
 // third-order step of the binomial series for (1 - e)^(-1/2), e = 1 - d y0^2:
-// y = y0 (1 + e/2 + 3e^2/8), which leaves O(e0^3) -- below FP64 rounding.  Five dependent
-// FP64 operations instead of a square root and a division: the pivot is on the critical
-// path of every Cholesky step, and FP64 latency is long on this part.
+// y = y0 (1 + e/2 + 3e^2/8), which leaves O(e0^3) -- below FP64 rounding.  Four dependent
+// FP64 operations: the pivot is on the critical path of every Cholesky step, and FP64 latency
+// is long on this part.  The two conversions are integer arithmetic for the same reason.
 __device__ __forceinline__ double rsqrt_fast(double d)
 {
   const long long db = __double_as_longlong(d);
   const int ed = (int)((db >> 52) & 0x7ff);
   if (ed < 1023 - 100 || ed > 1023 + 100) return 1.0 / sqrt(d);   // outside FP32's range
-  const double y = (double)rsqrtf((float)d);
+  // (float)d, rounded to nearest even.
+  const long long half = db + 0x0fffffffLL + ((db >> 29) & 1);
+  const float f = __uint_as_float((unsigned)(half >> 29) - 0xc0000000u);   // exponent - 896
+  const int yb = __float_as_int(rsqrtf(f));
+  const double y = __hiloint2double((yb >> 3) + (896 << 20), yb << 29);
   const double e = __fma_rn(-d * y, y, 1.0);
   return __fma_rn(y * e, __fma_rn(0.375, e, 0.5), y);
 }
 
-// Factor the diagonal block at (k0, k0) and invert its triangle: writes L_kk into A
-// (upper part zeroed) and L_kk^{-1} into dinv (nb x nb, row-major, zero above the diagonal).
-// Pivots at or below thr stop the factorisation (info = global 1-based index).
-// Right-looking, two barriers per column j: (1) column j of L (a_ij r_j, r_j = 1/sqrt(d_j))
-// and row j of V = L^{-1} (v_jc r_j) are scaled in place; (2) the trailing triangle takes
-// a_ic -= a_ij a_cj (c > j) and the rows of V below j take v_ic -= a_ij v_jc (c <= j).  The
-// FP64 pipe (two lanes per clock per SM on this part, whatever the active mask) bounds the
-// block's ~nb^3/3 FMAs, so phase (2) runs as one flat list of work items with every lane
-// busy (a triangle ordered by decreasing column makes the items of step j a prefix).  The
-// thread that updates the next pivot a_{j+1,j+1} forms its reciprocal root at once.
-template <int NB>
-__global__ void __launch_bounds__(256) potrf_diag_inv(double* A, long long ld, int n, int k0,
-                                                      const double* thr_p, CholStatus* cs,
-                                                      double* dinv)
+// The diagonal block at (k0, k0), on one SM: a chain of 64 pivots.  A warp's FP64 instruction
+// holds its quarter of the SM's pipe for 64 clocks whatever its active lanes, and a dependent
+// one follows no sooner; a pivot is eight of them (reciprocal root, scaling, next pivot) and
+// two shuffles behind the last.  So the chain runs on one warp with as little beside it as
+// possible: panels of four columns, a lane per row, the pivot and the multipliers going
+// between lanes by shuffles; a second warp on another quarter follows column by column with
+// the rows the first has no lane for; then all warps bring the next panel's columns up to
+// date, and while that panel runs the other warps update the columns behind it.  Every element
+// takes its FMAs in the order of the columns, as the plain right-looking loop does, so the
+// factor has that loop's bits.  Measured 40 us (the chain alone would be 25); that loop, with a
+// barrier pair per column and the inverse's triangle in the same block, took 100 us, panels of
+// 16 columns on one warp 94 us.  All of N_mu = 256: 0.50 -> 0.25 ms.
+// Pivots at or below thr stop the factorisation (info = global 1-based index).  Writes L_kk into
+// A (upper part zeroed) and the pivots' reciprocal roots, the diagonal of L_kk^{-1}, into dinv.
+constexpr int CP = 4;                        // panel width
+constexpr int CS = NB + 2;                   // shared row length: 16-byte rows, spread banks
+__global__ void __launch_bounds__(256) chol_diag(double* A, long long ld, int n, int k0,
+                                                 const double* thr_p, CholStatus* cs, double* dinv)
 {
   if (cs->flag) return;
   const double thr = thr_p ? *thr_p : 0.0;
-  extern __shared__ double dsm[];                       // 2 x NB x (NB + 1) doubles
-  double (*a)[NB + 1] = reinterpret_cast<double (*)[NB + 1]>(dsm);
-  double (*v)[NB + 1] = reinterpret_cast<double (*)[NB + 1]>(dsm + NB * (NB + 1));
-  __shared__ double rr[NB], piv[NB];
-  __shared__ unsigned short tri[NB * (NB - 1) / 2];     // (i << 8) | c, c descending
+  __shared__ __align__(16) double a[NB][CS];
+  __shared__ double rr[NB];
+  __shared__ int bad;
   const int nb = min(NB, n - k0);
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-    int r = e / NB, c = e % NB;
-    a[r][c] = (r < nb && c < nb) ? A[(long long)(k0 + r) * ld + k0 + c] : (r == c ? 1.0 : 0.0);
-    v[r][c] = r == c ? 1.0 : 0.0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  {
+    double v[16];                            // all loads in flight at once
+    const int c = threadIdx.x & 63, r0 = threadIdx.x >> 6;
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      const int r = r0 + 4 * q;
+      v[q] = (r < nb && c <= r) ? A[(long long)(k0 + r) * ld + k0 + c] : (r == c ? 1.0 : 0.0);
+    }
+#pragma unroll
+    for (int q = 0; q < 16; q++) a[r0 + 4 * q][c] = v[q];
   }
-  // Column c (1 <= c < nb) holds items (c..nb-1, c); columns nb-1, nb-2, ... come first, so
-  // column c starts at T(c) = sum_{c' > c} (nb - c') = (nb - 1 - c)(nb - c) / 2.
-  for (int c = 1 + (int)threadIdx.x; c < nb; c += blockDim.x) {
-    const int base = (nb - 1 - c) * (nb - c) / 2;
-    for (int i = c; i < nb; i++) tri[base + (i - c)] = (unsigned short)((i << 8) | c);
-  }
+  if (threadIdx.x == 0) bad = 0;
   double pmin = cs->min_piv, pmax = cs->max_piv;
-  __syncthreads();
-  auto pivot = [&](int j, double d) {
-    piv[j] = d;
-    rr[j] = d > 0.0 ? rsqrt_fast(d) : 1.0;
-  };
-  if (threadIdx.x == 0) pivot(0, a[0][0]);
-  __syncthreads();
-  bool bad = false;
   // d > thr (thr >= 0) as an integer comparison of the bit patterns, which order like the
-  // values for non-negative doubles (a negative d compares below): the FP64 pipe is the
-  // scarce resource here, and every thread takes this test every step.
+  // values for non-negative doubles (a negative d compares below).
   const long long thr_bits = __double_as_longlong(thr > 0.0 ? thr : 0.0);
-  for (int j = 0; j < nb; j++) {
-    const double d = piv[j];                             // the same value in every thread
-    const long long db = __double_as_longlong(d);
-    if (!(db > thr_bits && ((db >> 52) & 0x7ff) != 0x7ff)) {
-      if (threadIdx.x == 0) {
-        cs->flag = 1;
-        cs->info = k0 + j + 1;
+  __syncthreads();
+  // a[i][c] -= sum_j a[i][j] a[c][j] over panel columns j = c0 .. c0 + 3, in order.
+  auto update = [&](int i, int c, int c0) {
+    double v = a[i][c];
+    const double2 x0 = *(const double2*)&a[i][c0], x1 = *(const double2*)&a[i][c0 + 2];
+    const double2 y0 = *(const double2*)&a[c][c0], y1 = *(const double2*)&a[c][c0 + 2];
+    v = __fma_rn(-x0.x, y0.x, v);
+    v = __fma_rn(-x0.y, y0.y, v);
+    v = __fma_rn(-x1.x, y1.x, v);
+    v = __fma_rn(-x1.y, y1.y, v);
+    a[i][c] = v;
+  };
+  for (int c0 = 0; c0 < nb; c0 += CP) {
+    if (warp == 0) {
+      const int row = c0 + lane;
+      double x[CP];
+#pragma unroll
+      for (int q = 0; q < CP; q++) x[q] = row < NB ? a[row][c0 + q] : 0.0;
+      bool stop = false;
+#pragma unroll
+      for (int q = 0; q < CP; q++) {
+        const int j = c0 + q;
+        if (j >= nb) stop = true;
+        if (!stop) {
+          const double d = __shfl_sync(0xffffffffu, x[q], q);
+          const long long db = __double_as_longlong(d);
+          if (db > thr_bits && ((db >> 52) & 0x7ff) != 0x7ff) {
+            const double r = rsqrt_fast(d);
+            x[q] = __dmul_rn(x[q], r);
+            if (lane == 0) rr[j] = r;
+            if (row < NB && lane >= q) a[row][j] = x[q];
+#pragma unroll
+            for (int c = q + 1; c < CP; c++)
+              x[c] = __fma_rn(-x[q], __shfl_sync(0xffffffffu, x[q], c), x[c]);
+            // The smallest and largest pivot, compared as bit patterns (all are positive).
+            if (db < __double_as_longlong(pmin)) pmin = d;
+            if (db > __double_as_longlong(pmax)) pmax = d;
+          } else {
+            if (lane == 0) {
+              cs->flag = 1;
+              cs->info = k0 + j + 1;
+              bad = 1;
+            }
+            stop = true;
+          }
+        }
+        // Column j is in shared memory (or there is none): warp 1 may go on.
+        __syncwarp();
+        asm volatile("bar.arrive %0, 64;\n" ::"r"(1 + q) : "memory");
       }
-      bad = true;
-      break;
-    }
-    if (threadIdx.x == 0) {
-      pmin = fmin(pmin, d);
-      pmax = fmax(pmax, d);
-    }
-    const double r = rr[j];
-    // (1) scale column j of L (rows j..nb-1) and row j of V (columns 0..j)
-    {
-      const int t = threadIdx.x, na = nb - j;
-      if (t < na) a[j + t][j] *= r;
-      else if (t - na <= j) v[j][t - na] *= r;
+    } else if (warp == 1) {
+      const int row = c0 + 32 + lane;
+      double x[CP];
+#pragma unroll
+      for (int q = 0; q < CP; q++) x[q] = row < NB ? a[row][c0 + q] : 0.0;
+#pragma unroll
+      for (int q = 0; q < CP; q++) {
+        asm volatile("bar.sync %0, 64;\n" ::"r"(1 + q) : "memory");
+        if (c0 + 32 >= NB || c0 + q >= nb || *(volatile int*)&bad) continue;
+        x[q] = __dmul_rn(x[q], rr[c0 + q]);
+#pragma unroll
+        for (int c = q + 1; c < CP; c++) x[c] = __fma_rn(-x[q], a[c0 + c][c0 + q], x[c]);
+      }
+#pragma unroll
+      for (int q = 0; q < CP; q++)
+        if (row < NB) a[row][c0 + q] = x[q];
+    } else if (c0 > 0 && warp != 4) {
+      // The panel before this one, on the columns behind this one (not by warp 4, which shares
+      // its quarter of the FP64 pipe with the chain).  Item e of the triangle's list, columns
+      // from the last one back: column 63 - u holds items u (u + 1) / 2 .. + u.
+      const int w = NB - c0 - CP;
+      for (int e = (int)threadIdx.x - (warp < 4 ? 64 : 96); e < w * (w + 1) / 2; e += 160) {
+        int u = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+        if (u * (u + 1) / 2 > e) u--;
+        if ((u + 1) * (u + 2) / 2 <= e) u++;
+        update(63 - (e - u * (u + 1) / 2), 63 - u, c0 - CP);
+      }
     }
     __syncthreads();
-    // (2) the trailing triangle (T(j) items) and the rows of V below j ((nb-1-j)(j+1) items)
-    const int ntri = (nb - 1 - j) * (nb - j) / 2;
-    const int nrect = (nb - 1 - j) * (j + 1);
-    const int pe = ntri - (nb - 1 - j);                  // item (j+1, j+1): the next pivot
-    const int w = j + 1;                                 // rectangle row length
-    const float rw = 1.0f / (float)w;
-    for (int e = threadIdx.x; e < ntri + nrect; e += blockDim.x) {
-      if (e < ntri) {
-        const unsigned code = tri[e];
-        const int i = code >> 8, c = code & 255;
-        const double nv = __fma_rn(-a[i][j], a[c][j], a[i][c]);
-        a[i][c] = nv;
-        if (e == pe) pivot(j + 1, nv);
-      } else {
-        // q = r w + c without an integer division: the FP32 quotient of q < 2^12 is off by
-        // at most one, which the two corrections fix.
-        const int q = e - ntri;
-        int r = (int)((float)q * rw);
-        int c = q - r * w;
-        if (c < 0) { r--; c += w; }
-        if (c >= w) { r++; c -= w; }
-        const int i = j + 1 + r;
-        v[i][c] = __fma_rn(-a[i][j], v[j][c], v[i][c]);
-      }
+    if (bad) break;
+    // The next panel's columns, by this panel: an element a thread.
+    {
+      const int i = threadIdx.x & 63, c = c0 + CP + (threadIdx.x >> 6);
+      if (c < NB && i >= c) update(i, c, c0);
     }
     __syncthreads();
   }
@@ -246,11 +278,152 @@ __global__ void __launch_bounds__(256) potrf_diag_inv(double* A, long long ld, i
     cs->max_piv = pmax;
   }
   if (bad) return;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    int r = e / nb, c = e % nb;
+  const int c = threadIdx.x & 63;
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int r = (threadIdx.x >> 6) + 4 * q;
+    if (r >= nb || c >= nb) continue;
     A[(long long)(k0 + r) * ld + k0 + c] = c <= r ? a[r][c] : 0.0;
-    dinv[(long long)r * nb + c] = c <= r ? v[r][c] : 0.0;
+    if (r == c) dinv[(long long)r * nb + r] = rr[r];
   }
+}
+
+// L_kk^{-1} (nb x nb, row-major, zero above the diagonal) from the factored block and the
+// reciprocal roots on dinv's diagonal: the columns are independent forward substitutions, a
+// warp each on SMs of their own (inside the diagonal kernel they took two thirds of its FP64
+// work).  Column c: v_j *= r_j, then v_i -= l_ij v_j for i > j, j ascending.
+constexpr int IW = 4;                        // columns a block: one warp to each FP64 quarter
+__global__ void __launch_bounds__(32 * IW) chol_diag_inv(const double* A, long long ld, int n,
+                                                         int k0, const CholStatus* cs, double* dinv)
+{
+  if (cs->flag) return;
+  __shared__ double a[NB][NB + 1];
+  __shared__ double rr[NB];
+  const int nb = min(NB, n - k0);
+  const int lane = threadIdx.x & 31, c = blockIdx.x * IW + (threadIdx.x >> 5);
+  {
+    const int q = threadIdx.x & 63, r0 = threadIdx.x >> 6;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      double v[16];
+#pragma unroll
+      for (int t = 0; t < 16; t++) {
+        const int r = r0 + 2 * t + 32 * h;
+        v[t] = (r < nb && q < r) ? A[(long long)(k0 + r) * ld + k0 + q] : 0.0;
+      }
+#pragma unroll
+      for (int t = 0; t < 16; t++) a[r0 + 2 * t + 32 * h][q] = v[t];
+    }
+    if (threadIdx.x < nb) rr[threadIdx.x] = dinv[(long long)threadIdx.x * nb + threadIdx.x];
+  }
+  __syncthreads();
+  if (c >= nb) return;
+  double v0 = lane == c ? 1.0 : 0.0, v1 = lane + 32 == c ? 1.0 : 0.0;
+  // Rows 0-31, then (where they take part at all) rows 32-63 by every column.
+  for (int j = c; j < min(nb, 32); j++) {
+    const double vj = __dmul_rn(__shfl_sync(0xffffffffu, v0, j), rr[j]);
+    const double t0 = __fma_rn(-a[lane][j], vj, v0);       // a is zero on and above the diagonal
+    v1 = __fma_rn(-a[lane + 32][j], vj, v1);
+    v0 = lane == j ? vj : (lane > j ? t0 : v0);
+  }
+  for (int j = max(c, 32); j < nb; j++) {
+    const double vj = __dmul_rn(__shfl_sync(0xffffffffu, v1, j - 32), rr[j]);
+    const double t1 = __fma_rn(-a[lane + 32][j], vj, v1);
+    v1 = lane + 32 == j ? vj : (lane + 32 > j ? t1 : v1);
+  }
+  if (lane < nb && lane != c) dinv[(long long)lane * nb + c] = lane > c ? v0 : 0.0;
+  if (lane + 32 < nb && lane + 32 != c) dinv[(long long)(lane + 32) * nb + c] = lane + 32 > c ? v1 : 0.0;
+}
+
+// L_panel = A_panel L_kk^{-T} in place, rows k0 + 64 .. n: a CTA owns R whole rows, so that
+// nothing it overwrites is read elsewhere (the general GEMM went through partials and a second
+// launch).  Two threads an entry sum k below and above 32, the order of that GEMM's split.
+template <int R>
+__global__ void __launch_bounds__(128 * R) chol_panel(double* P, long long ld, int rows,
+                                                      const double* __restrict__ dinv,
+                                                      const int* flag)
+{
+  if (*flag) return;
+  __shared__ __align__(16) double v[NB][CS];
+  __shared__ __align__(16) double x[R][NB];
+  constexpr int T = 128 * R, LD = NB * NB / 2 / T;
+  {
+    double2 t[LD];
+#pragma unroll
+    for (int q = 0; q < LD; q++) t[q] = __ldg((const double2*)dinv + threadIdx.x + q * T);
+    if (threadIdx.x < NB * R) {
+      const long long row = blockIdx.x * (long long)R + threadIdx.x / NB;
+      x[threadIdx.x / NB][threadIdx.x % NB] = row < rows ? P[row * ld + threadIdx.x % NB] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < LD; q++) {
+      const int e = 2 * (threadIdx.x + q * T);
+      *(double2*)&v[e / NB][e % NB] = t[q];
+    }
+  }
+  __syncthreads();
+  const int h = threadIdx.x & 1, c = (threadIdx.x >> 1) & (NB - 1), r = threadIdx.x / (2 * NB);
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < NB / 2; k += 2) {
+    const double2 p = *(const double2*)&x[r][32 * h + k], q = *(const double2*)&v[c][32 * h + k];
+    s = __fma_rn(p.x, q.x, s);
+    s = __fma_rn(p.y, q.y, s);
+  }
+  const double s1 = __shfl_down_sync(0xffffffffu, s, 1);
+  const long long row = blockIdx.x * (long long)R + r;
+  if (h == 0 && row < rows) P[row * ld + c] = __dadd_rn(__dadd_rn(0.0, s), s1);
+}
+
+// C[m, n] -= sum_{k < 64} L[m, k] L[n, k] for n <= m (C and L row-major with ld): the small
+// trailing updates.  A CTA of 256 threads owns 8 x 16 entries, two threads each for k below and
+// above 32, added in that order as the general GEMM's split does; small tiles, because an SM
+// takes two FMAs a clock and 192 rows are 1.2e6 of them.  (That GEMM and the sum of its
+// partials were two launches of 12 and 4 us at 192 rows.)
+constexpr int RM = 8, RN = 16;
+__global__ void __launch_bounds__(256) chol_rank64(const double* __restrict__ L, double* C,
+                                                   long long ld, int rows, const int* flag)
+{
+  // Tile t: row block i of 8 reaches column block i / 2 of 16; 2 q (q + 1) / 2 tiles lie
+  // before row blocks 2q and 2q + 1, which have q + 1 each.
+  const int t = blockIdx.x;
+  int q = (int)((sqrtf(4.f * (float)t + 1.f) - 1.f) * 0.5f);
+  while (q * (q + 1) > t) q--;
+  while ((q + 1) * (q + 2) <= t) q++;
+  const int rest = t - q * (q + 1);
+  const int m0 = (2 * q + (rest > q ? 1 : 0)) * RM, n0 = (rest > q ? rest - q - 1 : rest) * RN;
+  if (m0 >= rows || *flag) return;
+  __shared__ __align__(16) double x[RM][CS], y[RN][CS];
+  {
+    double2 v[3];
+#pragma unroll
+    for (int s = 0; s < 3; s++) {             // 24 rows of 32 pairs
+      const int e = threadIdx.x + 256 * s, r = e >> 5, k = 2 * (e & 31);
+      const int row = r < RM ? m0 + r : n0 + r - RM;
+      const double* p = L + (long long)row * ld + k;
+      v[s] = row < rows ? make_double2(p[0], p[1]) : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+      const int e = threadIdx.x + 256 * s, r = e >> 5, k = 2 * (e & 31);
+      *(double2*)(r < RM ? &x[r][k] : &y[r - RM][k]) = v[s];
+    }
+  }
+  const int h = threadIdx.x & 1, j = (threadIdx.x >> 1) & (RN - 1), i = threadIdx.x / (2 * RN);
+  const int m = m0 + i, n = n0 + j;
+  const bool own = h == 0 && m < rows && n <= m;
+  double* cp = C + (long long)m * ld + n;
+  const double old = own ? *cp : 0.0;
+  __syncthreads();
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < NB / 2; k += 2) {
+    const double2 a = *(const double2*)&x[i][32 * h + k], b = *(const double2*)&y[j][32 * h + k];
+    s = __fma_rn(a.x, b.x, s);
+    s = __fma_rn(a.y, b.y, s);
+  }
+  const double s1 = __shfl_down_sync(0xffffffffu, s, 1);
+  if (own) *cp = __dadd_rn(old, -__dadd_rn(__dadd_rn(0.0, s), s1));
 }
 
 __global__ void set_identity_k(double* A, long long ld, int n)
@@ -353,6 +526,20 @@ static void launch_dgemm(const GemmArgs& g, cudaStream_t s)
   else dgemm_kernel<false, false, T><<<grid, 256, 0, s>>>(g);
 }
 
+// Tile and split of K so that the grid covers the SMs about twice.
+static void choose_tile(GemmArgs& g)
+{
+  const long long want = 2LL * 152;
+  auto tiles = [&](int t) {
+    long long mt = cdiv(g.M, t), nt = cdiv(g.N, t);
+    return g.lower_only ? (mt * nt + mt) / 2 : mt * nt;
+  };
+  g.tile = tiles(64) >= want / 2 ? 64 : (tiles(32) >= want / 2 ? 32 : 16);
+  long long split = std::min<long long>(cdiv(want, tiles(g.tile)), std::max(1, g.K / 32));
+  if (g.no_split) split = 1;
+  g.ksplit = (int)std::max<long long>(1, std::min<long long>(split, cdiv(g.K, BK)));
+}
+
 int dgemm(Ctx* c, const GemmArgs& g_in)
 {
   if (g_in.M <= 0 || g_in.N <= 0) return THC_OK;
@@ -363,26 +550,11 @@ int dgemm(Ctx* c, const GemmArgs& g_in)
   }
   GemmArgs g = g_in;
   if (g.ksplit <= 1 && !g.part) {
-    // Tile and split-K so that the grid covers the SMs about twice.
-    const long long want = 2LL * 152;
-    auto tiles = [&](int t) {
-      long long mt = cdiv(g.M, t), nt = cdiv(g.N, t);
-      return g.lower_only ? (mt * nt + mt) / 2 : mt * nt;
-    };
-    g.tile = tiles(64) >= want / 2 ? 64 : (tiles(32) >= want / 2 ? 32 : 16);
-    long long split = std::min<long long>(cdiv(want, tiles(g.tile)), std::max(1, g.K / 32));
-    if (g.aliased) split = std::max<long long>(split, 2);
-    if (g.no_split) {
-      if (g.aliased) return set_error(c, THC_ERR_ARG, "dgemm: aliased operands need a split");
-      split = 1;
-    }
-    g.ksplit = (int)std::max<long long>(1, std::min<long long>(split, cdiv(g.K, BK)));
+    choose_tile(g);
     if (g.ksplit > 1) {
       g.part = (double*)ws_get(c, WS_DPART, sizeof(double) * g.ksplit * g.M * g.N);
       if (!g.part) return set_error(c, THC_ERR_NOMEM, "dgemm: split-K partials");
     }
-  } else if (g.aliased && g.ksplit <= 1) {
-    return set_error(c, THC_ERR_ARG, "dgemm: aliased operands need split-K partials");
   }
   ProfScope prof(c, "dgemm");
   if (g.tile == 16) launch_dgemm<16>(g, c->stream);
@@ -399,6 +571,20 @@ int dgemm_reduce_partials(Ctx* c, const GemmArgs& g)
   return THC_OK;
 }
 
+// C -= L L^T over a panel of 64 columns: the kernel for it where the general GEMM would split K
+// in two (fewer tiles than twice the SMs), else that GEMM.
+static int rank64_update(Ctx* c, const GemmArgs& g)
+{
+  GemmArgs t = g;
+  choose_tile(t);
+  if (t.ksplit != 2 || g.K != NB) return dgemm(c, g);
+  const long long q = cdiv(g.M, 2 * RM);
+  chol_rank64<<<(unsigned)(q * (q + 1)), 256, 0, c->stream>>>(g.A, g.C, g.ldc, (int)g.M,
+                                                             g.skip_flag);
+  THC_LAUNCHED(c, "chol_rank64");
+  return THC_OK;
+}
+
 // Blocked Cholesky whose panel solve is a GEMM with the inverted diagonal block; the
 // inverted diagonal blocks are kept in dinv (nblk x 64 x 64) for the triangular inverse.
 int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholStatus* cs,
@@ -406,7 +592,6 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
 {
   ProfScope prof(c, "potrf_inv");
   cudaStream_t s = c->stream;
-  const int NB = chol_nb(n);
   // Look-ahead (n >= 512, with the context's second stream): after block k's panel, the
   // next diagonal block is updated first, on the main stream, and factored there while the
   // rest of block k's trailing update runs on the second stream; the next panel waits for
@@ -418,15 +603,10 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
   for (int k0 = 0; k0 < n; k0 += NB) {
     int nb = std::min(NB, n - k0);
     double* di = dinv + (long long)(k0 / NB) * NB * NB;
-    const int smem = 2 * NB * (NB + 1) * (int)sizeof(double);
-    if (NB == 32) {
-      THC_CUDA(c, cudaFuncSetAttribute(potrf_diag_inv<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      potrf_diag_inv<32><<<1, 256, smem, s>>>(A, ld, n, k0, thr, cs, di);
-    } else {
-      THC_CUDA(c, cudaFuncSetAttribute(potrf_diag_inv<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      potrf_diag_inv<64><<<1, 256, smem, s>>>(A, ld, n, k0, thr, cs, di);
-    }
-    THC_LAUNCHED(c, "potrf_diag_inv");
+    chol_diag<<<1, 256, 0, s>>>(A, ld, n, k0, thr, cs, di);
+    THC_LAUNCHED(c, "chol_diag");
+    chol_diag_inv<<<NB / IW, 32 * IW, 0, s>>>(A, ld, n, k0, cs, di);
+    THC_LAUNCHED(c, "chol_diag_inv");
     int rest = n - k0 - nb;
     if (rest <= 0) break;
     if (trail_pending) {     // the panel rows below were updated on the second stream
@@ -434,16 +614,12 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
       trail_pending = false;
     }
     {
-      // L_panel = A_panel L_kk^{-T}, in place (each CTA owns its rows; N = nb <= 64).
-      GemmArgs g{};
-      g.M = rest; g.N = nb; g.K = nb;
-      g.A = A + (long long)(k0 + nb) * ld + k0; g.sam = ld; g.sak = 1;
-      g.B = di; g.sbn = nb; g.sbk = 1;
-      g.C = A + (long long)(k0 + nb) * ld + k0; g.ldc = ld;
-      g.skip_flag = &cs->flag;
-      g.aliased = 1;
-      int st = dgemm(c, g);
-      if (st) return st;
+      double* panel = A + (long long)(k0 + nb) * ld + k0;
+      // Rows a CTA: two while their blocks find an SM at once, else four, which share the copy
+      // of the inverse block.
+      if (rest <= 608) chol_panel<2><<<(unsigned)cdiv(rest, 2), 256, 0, s>>>(panel, ld, rest, di, &cs->flag);
+      else chol_panel<4><<<(unsigned)cdiv(rest, 4), 512, 0, s>>>(panel, ld, rest, di, &cs->flag);
+      THC_LAUNCHED(c, "chol_panel");
     }
     const double* l21 = A + (long long)(k0 + nb) * ld + k0;
     if (!la) {
@@ -454,7 +630,7 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
       g.C = A + (long long)(k0 + nb) * ld + k0 + nb; g.ldc = ld;
       g.alpha = -1.0; g.beta = 1.0; g.lower_only = 1; g.mode = GEMM_STORE;
       g.skip_flag = &cs->flag;
-      int st = dgemm(c, g);
+      int st = rank64_update(c, g);
       if (st) return st;
       continue;
     }
@@ -468,7 +644,7 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
       g.C = A + (long long)(k0 + nb) * ld + k0 + nb; g.ldc = ld;
       g.alpha = -1.0; g.beta = 1.0; g.lower_only = 1; g.mode = GEMM_STORE;
       g.skip_flag = &cs->flag;
-      int st = dgemm(c, g);
+      int st = rank64_update(c, g);
       if (st) return st;
     }
     if (rest > nb1) {
@@ -500,14 +676,13 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
 
 // X = L^{-1} (lower, n x n, ld) from the factor L and its inverted diagonal blocks, block row
 // by block row: X_ii = dinv_i, X[i, 0:i] = -dinv_i (L[i, 0:i] X[0:i, 0:i]), with the block
-// edge NB = chol_nb(n) that potrf_inv used.  T is an NB x n scratch.  Then Cinv = X^T X.
+// edge NB that potrf_inv used.  T is an NB x n scratch.  Then Cinv = X^T X.
 int chol_inverse(Ctx* c, const double* L, long long ld, int n, const double* dinv, double* X,
                  double* T, double* Cinv, const CholStatus* cs)
 {
   ProfScope prof(c, "chol_inverse");
   cudaStream_t s = c->stream;
   THC_CUDA(c, cudaMemsetAsync(X, 0, sizeof(double) * (size_t)n * ld, s));
-  const int NB = chol_nb(n);
   int nblk = (n + NB - 1) / NB;
   for (int bi = 0; bi < nblk; bi++) {
     int i0 = bi * NB, nb = std::min(NB, n - i0);

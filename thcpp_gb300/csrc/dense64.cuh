@@ -29,7 +29,6 @@ struct GemmArgs {
   const int* skip_flag = nullptr;   // if non-null and set, the kernel does nothing
   int ksplit = 1;                    // > 1: K is split over blockIdx.z into FP64 partials
   double* part = nullptr;            // ksplit x M x N partial buffer (row-major, ld = N)
-  int aliased = 0;                   // C overlaps A or B: products go through partials
   // Known zeros: A(m, k) = 0 for k < m (a_zero_below) / B(k, n) = 0 for k < n
   // (b_zero_below), as for a lower-triangular factor read transposed / as it is.  A tile
   // then starts its k loop at its first row / column: the skipped terms are exact zeros,
@@ -54,7 +53,7 @@ struct CholStatus {
 // over many SMs); split partials are summed in split order (deterministic).
 int dgemm(Ctx* c, const GemmArgs& g);
 // Products the tensor-core route takes (dgemm_tc.cu): at least this much work, no skip flag,
-// no aliasing, no known-zero triangle and no caller's split.  Below it the FMA kernel's one
+// no known-zero triangle and no caller's split.  Below it the FMA kernel's one
 // launch is as fast as the cut of two operands and the product (97 x 1001 x 200, 3.9e7: 50 us
 // against 36; 130 x 130 x 1000, 3.4e7: 52 against 46; 130 x 200 x 1000 row-contiguous, 5.2e7:
 // 80 against 85; 256 x 4096 x 32, 6.7e7: 73 against 31).

@@ -834,7 +834,7 @@ int cut_operand(Ctx* c, const CutSrc& a, const Digits& d, unsigned* rowmax, int*
 
 bool dgemm_tc_fits(const Ctx* c, const GemmArgs& g)
 {
-  if (!c->gemm_tc || g.fma_only || g.skip_flag || g.aliased || g.a_zero_below || g.b_zero_below ||
+  if (!c->gemm_tc || g.fma_only || g.skip_flag || g.a_zero_below || g.b_zero_below ||
       g.lower_offset || g.no_split || g.ksplit > 1 || g.part || (g.lower_only && g.M != g.N))
     return false;
   return 2.0 * (double)g.M * (double)g.N * (double)g.K >= kDgemmTcFlops && g.K >= 8;
