@@ -1,6 +1,7 @@
 """The FP64 dense kernels at the edges of their tiles: products on the tensor cores
 (csrc/dgemm_tc.cu) against the oracle and the FMA route (option gemm_tc), an orbital value that
 is not finite, and the Cholesky (csrc/dense64.cu) with a breakdown at every kind of position."""
+import numpy as np
 import pytest
 
 import oracle
