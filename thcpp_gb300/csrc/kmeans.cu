@@ -79,7 +79,6 @@ struct KmState {
   double slack32;                        // absolute slack of the FP32 candidate bound
   int diff_exact;                        // st->diff came from the sequential sum
   int ticket;                            // blocks of km_sums finished this iteration
-  int scan_ticket;                       // blocks of km_colscan finished this iteration
   int nwin;                              // windows of the exact sums this iteration
 };
 
@@ -98,7 +97,7 @@ struct KmBufs {
   double* cen;     // [2][3][nmu]
   float* cen32;    // [2][3][nmu]
   int* labels;     // [2][ng]
-  int* hist;       // [nmu][nb]
+  int* hist;       // [nb][nmu]: a block's counts are one run, for the scan and the scatter
   int* total;      // [nmu]
   int* start;      // [nmu]
   int* member;     // [ng]
@@ -114,6 +113,7 @@ struct KmBufs {
   int* bcount;     // [nbins_max] counts, then offsets, then cursors
   int nbins_max;
   float* pf;       // [3][ng] FP32 coordinates in the binned order (pf[d][t] of point perm[t])
+  float* box;      // [tiles][6] bounding boxes of its 256-point tiles (min x, y, z, max x, y, z)
   // Window-parallel exact sums (nwin_max == 0: the one-kernel km_sums path).
   const double* tq;   // [4][ng] rho_i, rho_i x_i, rho_i y_i, rho_i z_i in point order
   double* sv;         // [4][ng] the same terms in sorted (cluster, ascending point) order
@@ -273,10 +273,14 @@ __global__ void km_bin_count(const double* __restrict__ grid, KmBufs b)
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= b.ng) return;
   const KmState* st = b.st;
+  // Boustrophedon order: every second row runs backwards, so consecutive bins touch and a
+  // tile of 256 points never spans the cell (a tile over a row's end kept nearly every
+  // centroid: 142 us an iteration at N_g 373248, N_mu 2048).
   int bin = 0;
   for (int d = 0; d < 3; d++) {
     int q = (int)((grid[3 * i + d] - st->blo[d]) * st->binv[d]);
     q = q < 0 ? 0 : (q >= st->nbin[d] ? st->nbin[d] - 1 : q);
+    if (bin & 1) q = st->nbin[d] - 1 - q;
     bin = bin * st->nbin[d] + q;
   }
   b.pbin[i] = bin;
@@ -333,27 +337,6 @@ __global__ void km_bin_scatter(KmBufs b)
   b.pf[2 * b.ng + pos] = b.fz[i];
 }
 
-// Ordered block-wide compaction of `flag` over the block's threads: returns this thread's
-// slot (or -1) and adds the block's count to *total (all threads see the new total).
-__device__ __forceinline__ int block_compact(bool flag, int* wsum, int* total)
-{
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  unsigned bal = __ballot_sync(0xffffffffu, flag);
-  if (lane == 0) wsum[wid] = __popc(bal);
-  __syncthreads();
-  int before = *total;
-  for (int w = 0; w < wid; w++) before += wsum[w];
-  int slot = flag ? before + __popc(bal & ((1u << lane) - 1u)) : -1;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = *total;
-    for (int w = 0; w < nw; w++) t += wsum[w];
-    *total = t;
-  }
-  __syncthreads();
-  return slot;
-}
-
 // A final label of the pruned assign kernels, with the counting sort's histogram entry
 // (cluster k, block of kBP consecutive point indices) and the changed-label count: the
 // separate histogram pass is not needed on this path.
@@ -361,7 +344,7 @@ __device__ __forceinline__ void put_label(const KmBufs& b, int it, long long i, 
                                           unsigned& changed)
 {
   b.labels[(size_t)(it & 1) * b.ng + i] = k;
-  atomicAdd(&b.hist[(size_t)k * b.nb + i / kBP], 1);
+  atomicAdd(&b.hist[(size_t)(i / kBP) * b.nmu + k], 1);
   if (it > 0 && b.labels[(size_t)((it + 1) & 1) * b.ng + i] != k) changed++;
 }
 
@@ -372,110 +355,26 @@ __device__ __forceinline__ void flush_changed(KmState* st, unsigned changed)
   if ((threadIdx.x & 31) == 0 && changed) atomicAdd(&st->changed, (unsigned long long)changed);
 }
 
-constexpr int kPruneMax = 2048;   // candidate centroids kept in shared memory per tile
+constexpr int kPruneMax = 1024;   // candidate centroids kept in shared memory per tile
 
-// FP64 assign with exact spatial pruning.  A tile is 256 consecutive points of the
-// binned order.  With lb(c) / ub(c) the smallest / largest squared distance from centroid
-// c to the tile's bounding box and U = min_c ub(c), every point's nearest centroid has
-// squared distance <= U; a centroid with lb(c) > U (1 + 1e-9) is farther from every point
-// of the tile than its nearest centroid by a relative margin far above the rounding of
-// either bound or of the distance itself, so it can neither win nor tie after sqrt.  The
-// kept centroids are scanned in ascending index order with the exact semantics.
-__global__ void __launch_bounds__(kAssignThreads) km_assign64p(KmBufs b)
-{
-  const KmState* st = b.st;
-  if (st->done) return;
-  int it = st->iter;
-  const double* cx = b.cen + (size_t)(it & 1) * 3 * b.nmu;
-  const double* cy = cx + b.nmu;
-  const double* cz = cy + b.nmu;
-  extern __shared__ unsigned char sm[];
-  int* cand = (int*)sm;
-  double* ccx = (double*)(sm + sizeof(int) * kPruneMax);
-  double* ccy = ccx + kPruneMax;
-  double* ccz = ccy + kPruneMax;
-  __shared__ double red[3][2][kAssignThreads / 32];
-  __shared__ double uw[kAssignThreads / 32];
-  __shared__ int wsum[kAssignThreads / 32];
-  __shared__ int ncand;
-  long long t = blockIdx.x * (long long)kAssignThreads + threadIdx.x;
-  bool valid = t < b.ng;
-  long long i = valid ? b.perm[t] : 0;
-  double g[3] = {0, 0, 0};
-  if (valid) { g[0] = b.gx[i]; g[1] = b.gy[i]; g[2] = b.gz[i]; }
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double lo[3], hi[3];
-  for (int d = 0; d < 3; d++) {
-    double mn = valid ? g[d] : CUDART_INF, mx = valid ? g[d] : -CUDART_INF;
-    for (int off = 16; off; off >>= 1) {
-      mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, off));
-      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    }
-    if (lane == 0) { red[d][0][wid] = mn; red[d][1][wid] = mx; }
-  }
-  if (threadIdx.x == 0) ncand = 0;
-  __syncthreads();
-  for (int d = 0; d < 3; d++) {
-    lo[d] = red[d][0][0];
-    hi[d] = red[d][1][0];
-    for (int w = 1; w < kAssignThreads / 32; w++) {
-      lo[d] = fmin(lo[d], red[d][0][w]);
-      hi[d] = fmax(hi[d], red[d][1][w]);
-    }
-  }
-  // U = min over centroids of the largest squared distance to the box.
-  double u = CUDART_INF;
-  for (int k = threadIdx.x; k < b.nmu; k += kAssignThreads) {
-    double c3[3] = {cx[k], cy[k], cz[k]}, ub = 0.0;
-    for (int d = 0; d < 3; d++) {
-      double a = c3[d] - lo[d], e = c3[d] - hi[d];
-      ub += fmax(a * a, e * e);
-    }
-    u = fmin(u, ub);
-  }
-  for (int off = 16; off; off >>= 1) u = fmin(u, __shfl_xor_sync(0xffffffffu, u, off));
-  if (lane == 0) uw[wid] = u;
-  __syncthreads();
-  double U = uw[0];
-  for (int w = 1; w < kAssignThreads / 32; w++) U = fmin(U, uw[w]);
-  double cut = U * (1.0 + 1e-9);
-  for (int kb = 0; kb < b.nmu; kb += kAssignThreads) {
-    int k = kb + threadIdx.x;
-    bool keep = false;
-    double c3[3] = {0, 0, 0};
-    if (k < b.nmu) {
-      c3[0] = cx[k]; c3[1] = cy[k]; c3[2] = cz[k];
-      double lb = 0.0;
-      for (int d = 0; d < 3; d++) {
-        double v = fmax(0.0, fmax(lo[d] - c3[d], c3[d] - hi[d]));
-        lb += v * v;
-      }
-      keep = lb <= cut;
-    }
-    int slot = block_compact(keep, wsum, &ncand);
-    if (slot >= 0 && slot < kPruneMax) {
-      cand[slot] = k; ccx[slot] = c3[0]; ccy[slot] = c3[1]; ccz[slot] = c3[2];
-    }
-  }
-  __syncthreads();   // every thread reads every candidate written above
-  int nc = ncand;
-  ArgMin am;
-  am.init();
-  if (nc <= kPruneMax) {
-    if (valid)
-      for (int j = 0; j < nc; j++) am.push(d2_exact(ccx[j], ccy[j], ccz[j], g[0], g[1], g[2]), cand[j]);
-  } else if (valid) {
-    for (int k = 0; k < b.nmu; k++) am.push(d2_exact(cx[k], cy[k], cz[k], g[0], g[1], g[2]), k);
-  }
-  unsigned changed = 0;
-  if (valid) put_label(b, it, i, am.k, changed);
-  flush_changed(const_cast<KmState*>(st), changed);
-}
-
-// FP32 filter with pruning.  Bounds are computed in FP32 with a relative margin 1e-4 and
-// an absolute slack 1e-4 |a|^2, far above their FP32 rounding, so the FP64 nearest
-// centroid is always kept; the margin test and the FP64 recheck then work as in km_assign32.
-__global__ void __launch_bounds__(kAssignThreads) km_assign32p(KmBufs b)
+// Assign with exact spatial pruning, for both precisions: FP32 filters, FP64 decides.
+//
+// A tile is 256 consecutive points of the binned order, its bounding box (b.box) made once per
+// call.  With lb(c) / ub(c) the smallest / largest squared distance from centroid c to the box
+// and U = min_c ub(c), a centroid with lb(c) > U (1 + 1e-4) + slack, slack = 1e-4 |a|^2, is
+// farther from every point of the tile than its nearest centroid by a margin far above the
+// rounding of the FP32 bounds and of the FP64 distance, so it can neither win nor tie after
+// sqrt.  Of the kept centroids, in ascending index order, each thread takes the nearest in FP32
+// with the gap to the second: with u = 2^-24,
+//   |d2_32 - d2_64| <= u (2 |d| |a| + 5 d2) + O(u^2),   a_i = |c_i| + |g_i|,
+// so a gap above E(m1) + E(m2), E(m) = 2u (2 sqrt(m) |a| + 5 m) (a factor 2 for the O(u^2)
+// terms), proves that every other centroid is strictly farther in FP64, hence also after sqrt.
+// Other points are resolved at once in FP64 by their whole warp, one at a time, with the
+// reference's semantics.  The labels are those of an FP64 scan, whose 64 clocks an operation
+// and warp this part cannot afford (17 points a thread and 48 centroids took 52 us).  The test
+// itself is FP32 too, its terms raised by 1e-5 to cover its rounding: in FP64 its two roots
+// cost more than the scan (9 of 21 us at N_g 110592, N_mu 256).
+__global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
 {
   KmState* st = b.st;
   if (st->done) return;
@@ -488,41 +387,35 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign32p(KmBufs b)
   float* ccx = (float*)(sm + sizeof(int) * kPruneMax);
   float* ccy = ccx + kPruneMax;
   float* ccz = ccy + kPruneMax;
-  __shared__ float red[3][2][kAssignThreads / 32];
-  __shared__ float uw[kAssignThreads / 32];
-  __shared__ int wsum[kAssignThreads / 32];
-  __shared__ int ncand;
+  unsigned* kept = (unsigned*)(ccz + kPruneMax);        // 32 centroids a word
+  constexpr int kW = kAssignThreads / 32;
+  __shared__ float uw[kW];
+  __shared__ int wsum[kW];
   long long t = blockIdx.x * (long long)kAssignThreads + threadIdx.x;
   bool valid = t < b.ng;
   long long i = valid ? b.perm[t] : 0;
   float g[3] = {0, 0, 0};
   if (valid) { g[0] = b.pf[t]; g[1] = b.pf[b.ng + t]; g[2] = b.pf[2 * b.ng + t]; }
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float lo[3], hi[3];
   for (int d = 0; d < 3; d++) {
-    float mn = valid ? g[d] : INFINITY, mx = valid ? g[d] : -INFINITY;
-    for (int off = 16; off; off >>= 1) {
-      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    }
-    if (lane == 0) { red[d][0][wid] = mn; red[d][1][wid] = mx; }
+    lo[d] = b.box[(size_t)blockIdx.x * 6 + d];
+    hi[d] = b.box[(size_t)blockIdx.x * 6 + 3 + d];
   }
-  if (threadIdx.x == 0) ncand = 0;
-  __syncthreads();
-  for (int d = 0; d < 3; d++) {
-    lo[d] = red[d][0][0];
-    hi[d] = red[d][1][0];
-    for (int w = 1; w < kAssignThreads / 32; w++) {
-      lo[d] = fminf(lo[d], red[d][0][w]);
-      hi[d] = fmaxf(hi[d], red[d][1][w]);
-    }
-  }
+  // Warp w owns the words w nwords / kW .. of 32 consecutive centroids each, so that the
+  // compaction keeps the index order with one exchange of counts.
+  const int nwords = (b.nmu + 31) >> 5;
+  const int w0 = wid * nwords / kW, w1 = (wid + 1) * nwords / kW;
   float u = INFINITY;
-  for (int k = threadIdx.x; k < b.nmu; k += kAssignThreads) {
-    float c3[3] = {cx[k], cy[k], cz[k]}, ub = 0.f;
+#pragma unroll 4
+  for (int w = w0; w < w1; w++) {
+    const int k = w * 32 + lane;
+    if (k >= b.nmu) continue;
+    const float c3[3] = {cx[k], cy[k], cz[k]};
+    float ub = 0.f;
     for (int d = 0; d < 3; d++) {
-      float a = c3[d] - lo[d], e = c3[d] - hi[d];
-      ub += fmaxf(a * a, e * e);
+      const float p = c3[d] - lo[d], q = c3[d] - hi[d];
+      ub += fmaxf(p * p, q * q);
     }
     u = fminf(u, ub);
   }
@@ -530,28 +423,43 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign32p(KmBufs b)
   if (lane == 0) uw[wid] = u;
   __syncthreads();
   float U = uw[0];
-  for (int w = 1; w < kAssignThreads / 32; w++) U = fminf(U, uw[w]);
-  float cut = U * (1.0f + 1e-4f) + (float)st->slack32;
-  for (int kb = 0; kb < b.nmu; kb += kAssignThreads) {
-    int k = kb + threadIdx.x;
+  for (int w = 1; w < kW; w++) U = fminf(U, uw[w]);
+  const float cut = U * (1.0f + 1e-4f) + (float)st->slack32;
+  int count = 0;
+#pragma unroll 4
+  for (int w = w0; w < w1; w++) {
+    const int k = w * 32 + lane;
     bool keep = false;
-    float c3[3] = {0, 0, 0};
     if (k < b.nmu) {
-      c3[0] = cx[k]; c3[1] = cy[k]; c3[2] = cz[k];
+      const float c3[3] = {cx[k], cy[k], cz[k]};
       float lb = 0.f;
       for (int d = 0; d < 3; d++) {
-        float v = fmaxf(0.f, fmaxf(lo[d] - c3[d], c3[d] - hi[d]));
+        const float v = fmaxf(0.f, fmaxf(lo[d] - c3[d], c3[d] - hi[d]));
         lb += v * v;
       }
       keep = lb <= cut;
     }
-    int slot = block_compact(keep, wsum, &ncand);
-    if (slot >= 0 && slot < kPruneMax) {
-      cand[slot] = k; ccx[slot] = c3[0]; ccy[slot] = c3[1]; ccz[slot] = c3[2];
-    }
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) kept[w] = bal;
+    count += __popc(bal);
   }
-  __syncthreads();   // every thread reads every candidate written above
-  int nc = ncand;
+  if (lane == 0) wsum[wid] = count;
+  __syncthreads();
+  int nc = 0, slot = 0;
+  for (int w = 0; w < kW; w++) {
+    if (w == wid) slot = nc;
+    nc += wsum[w];
+  }
+  if (nc <= kPruneMax)
+    for (int w = w0; w < w1; w++) {
+      const unsigned bal = kept[w];
+      if (bal >> lane & 1) {
+        const int k = w * 32 + lane, q = slot + __popc(bal & ((1u << lane) - 1u));
+        cand[q] = k; ccx[q] = cx[k]; ccy[q] = cy[k]; ccz[q] = cz[k];
+      }
+      slot += __popc(bal);
+    }
+  __syncthreads();
   bool amb = false;
   unsigned changed = 0;
   if (valid) {
@@ -561,9 +469,10 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign32p(KmBufs b)
       for (int j = 0; j < nc; j++) {
         float dx = ccx[j] - g[0], dy = ccy[j] - g[1], dz = ccz[j] - g[2];
         float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
-        if (d2 < m1) { m2 = m1; m1 = d2; k1 = cand[j]; }
+        if (d2 < m1) { m2 = m1; m1 = d2; k1 = j; }
         else if (d2 < m2) { m2 = d2; }
       }
+      k1 = nc ? cand[k1] : 0;
     } else {
       for (int k = 0; k < b.nmu; k++) {
         float dx = cx[k] - g[0], dy = cy[k] - g[1], dz = cz[k] - g[2];
@@ -572,11 +481,11 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign32p(KmBufs b)
         else if (d2 < m2) { m2 = d2; }
       }
     }
-    const double uu = 5.9604644775390625e-08;
-    double a = st->abound;
-    double e1 = 2.0 * uu * (2.0 * sqrt((double)m1) * a + 5.0 * (double)m1);
-    double e2 = 2.0 * uu * (2.0 * sqrt((double)m2) * a + 5.0 * (double)m2);
-    if ((double)m2 - (double)m1 > e1 + e2 + 1e-300) put_label(b, it, i, k1, changed);
+    // 2u (2 |a| (sqrt m1 + sqrt m2) + 5 (m1 + m2)), every factor rounded up.
+    const float a = (float)st->abound * 1.00001f;
+    const float e = 1.1920929e-07f * 1.00001f *
+                    (2.f * a * (sqrtf(m1) + sqrtf(m2)) + 5.00001f * (m1 + m2));
+    if ((m2 - m1) * 0.99999f > e + 1e-30f) put_label(b, it, i, k1, changed);
     else amb = true;
   }
   // FP64 rescue of the near ties, at once and by the whole warp, one point at a time: the
@@ -723,7 +632,7 @@ __global__ void km_recheck(KmBufs b)
   }
 }
 
-// Per-block label histogram (sparse write into the zeroed hist[k][block]) and the
+// Per-block label histogram (sparse write into the zeroed hist[block][k]) and the
 // count of labels that changed since the previous iteration.
 __global__ void km_hist(KmBufs b)
 {
@@ -753,7 +662,7 @@ __global__ void km_hist(KmBufs b)
   if ((threadIdx.x & 31) == 0 && changed) atomicAdd(&st->changed, (unsigned long long)changed);
   __syncthreads();
   for (int k = threadIdx.x; k < b.nmu; k += blockDim.x)
-    if (sh[k]) b.hist[(size_t)k * b.nb + blockIdx.x] = sh[k];
+    if (sh[k]) b.hist[(size_t)blockIdx.x * b.nmu + k] = sh[k];
 }
 
 // Exclusive block-wide scan of one int per thread (all threads of the block).
@@ -781,81 +690,99 @@ __device__ int block_exscan(int v, int* warp_sums)
   return warp_sums[wid] + x - v;
 }
 
-// Exclusive scan of the cluster totals into cluster start offsets (one block); with the
-// window-parallel sums also the window table: cluster k's terms are cut into windows of
-// kSegWin, numbered consecutively from wbase[k].
-__device__ void kscan_block(KmBufs& b)
+// Start offsets of the clusters from their totals, by the whole block into shared memory
+// (base); with `publish` also start[] and, for the window-parallel sums, the window table:
+// cluster k's terms are cut into windows of kSegWin, numbered consecutively from wbase[k].
+// Every scatter block scans for itself: nmu totals are a few loads a thread, where a single
+// block between two kernels made all others wait for its round trips (3 us).
+__device__ void kscan_block(KmBufs& b, int* base, bool publish)
 {
   __shared__ int warp_sums[32];
-  int n = b.nmu;
-  int per = (n + blockDim.x - 1) / blockDim.x;
-  int lo = threadIdx.x * per, hi = min(n, lo + per);
+  const int n = b.nmu;
+  const int per = (n + blockDim.x - 1) / blockDim.x;
+  // Totals through shared memory, so that the loads are coalesced.
+  for (int k = threadIdx.x; k < n; k += blockDim.x) base[k] = b.total[k];
+  __syncthreads();
+  const int lo = min(n, (int)threadIdx.x * per), hi = min(n, lo + per);
   int s = 0, nw = 0;
   for (int k = lo; k < hi; k++) {
-    int t = __ldcg(b.total + k);
-    s += t;
-    nw += (t + kSegWin - 1) / kSegWin;
+    s += base[k];
+    nw += (base[k] + kSegWin - 1) / kSegWin;
   }
   int run = block_exscan(s, warp_sums);
-  int wrun = b.nwin_max ? block_exscan(nw, warp_sums) : 0;
+  int wrun = publish && b.nwin_max ? block_exscan(nw, warp_sums) : 0;
   for (int k = lo; k < hi; k++) {
-    const int t = __ldcg(b.total + k);
-    b.start[k] = run;
-    if (b.nwin_max) {
-      b.wbase[k] = wrun;
-      for (int j = 0; j * kSegWin < t; j++) {
-        KmWin w;
-        w.pos = run + j * kSegWin;
-        w.cnt = min(kSegWin, t - j * kSegWin);
-        w.first = run;
-        w.k = k;
-        b.win[wrun++] = w;
+    const int t = base[k];
+    base[k] = run;
+    if (publish) {
+      b.start[k] = run;
+      if (b.nwin_max) {
+        b.wbase[k] = wrun;
+        for (int j = 0; j * kSegWin < t; j++) {
+          KmWin w;
+          w.pos = run + j * kSegWin;
+          w.cnt = min(kSegWin, t - j * kSegWin);
+          w.first = run;
+          w.k = k;
+          b.win[wrun++] = w;
+        }
       }
     }
     run += t;
   }
-  if (b.nwin_max && hi == n && lo < hi) {
+  if (publish && b.nwin_max && hi == n && lo < hi) {
     b.wbase[n] = wrun;
     b.st->nwin = wrun;
   }
-  if (b.nwin_max && n == 0 && threadIdx.x == 0) b.st->nwin = 0;
+  __syncthreads();
 }
 
-// One warp per cluster: exclusive scan of its block counts (in place) and its total.  The
-// last block to finish (a ticket in the state) turns the totals into start offsets.
-__global__ void __launch_bounds__(256) km_colscan(KmBufs b)
+// Exclusive scan of every cluster's block counts (in place) and its total.  A CTA owns 32
+// clusters, a lane each, so that every access is one run; its 32 warps take consecutive
+// stretches of the blocks: sums first, a scan of the 32 sums per cluster, then the prefixes.
+// (A warp per cluster over a [cluster][block] table was 8.2 us at 216 blocks of 256 clusters,
+// 18 at 729 of 2048.)
+constexpr int kScanWarps = 32;
+__global__ void __launch_bounds__(32 * kScanWarps) km_colscan(KmBufs b)
 {
-  KmState* st = b.st;
-  if (st->done) return;
-  __shared__ int last;
-  int lane = threadIdx.x & 31;
-  long long k = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  if (b.st->done) return;
+  __shared__ int part[kScanWarps][33];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  const int per = (b.nb + kScanWarps - 1) / kScanWarps;
+  const int j0 = min(b.nb, wid * per), j1 = min(b.nb, j0 + per);
+  int* h = b.hist + k;
+  int sum = 0;
   if (k < b.nmu) {
-    int* h = b.hist + (size_t)k * b.nb;
-    int carry = 0;
-    for (int c = 0; c < b.nb; c += 32) {
-      int j = c + lane;
-      int v = j < b.nb ? h[j] : 0;
-      int x = v;
-      for (int off = 1; off < 32; off <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, off);
-        if (lane >= off) x += y;
-      }
-      if (j < b.nb) h[j] = carry + x - v;
-      carry += __shfl_sync(0xffffffffu, x, 31);
+#pragma unroll 8
+    for (int j = j0; j < j1; j++) sum += h[(size_t)j * b.nmu];
+  }
+  part[wid][lane] = sum;
+  __syncthreads();
+  {
+    const int v = part[lane][wid];           // warp `wid` scans cluster `wid` of the CTA
+    int x = v;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, off);
+      if (lane >= off) x += y;
     }
-    if (lane == 0) b.total[k] = carry;
+    part[lane][wid] = x - v;
+    if (lane == 31 && blockIdx.x * 32 + wid < b.nmu) b.total[blockIdx.x * 32 + wid] = x;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(&st->scan_ticket, 1) == (int)gridDim.x - 1;
+  if (k < b.nmu) {
+    int run = part[wid][lane];
+    for (int j = j0; j < j1; j += 8) {
+      int v[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = j + q < j1 ? h[(size_t)(j + q) * b.nmu] : 0;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        if (j + q < j1) h[(size_t)(j + q) * b.nmu] = run;
+        run += v[q];
+      }
+    }
   }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  kscan_block(b);
-  if (threadIdx.x == 0) st->scan_ticket = 0;
 }
 
 // Stable scatter of point indices into per-cluster member lists.  The block's labels and
@@ -872,8 +799,24 @@ __global__ void __launch_bounds__(256) km_scatter(KmBufs b)
   __shared__ int spos[kBP];
   const int* lab = b.labels + (size_t)(it & 1) * b.ng;
   const long long blk = (long long)blockIdx.x * kBP;
-  for (int k = threadIdx.x; k < b.nmu; k += blockDim.x)
-    base[k] = b.start[k] + b.hist[(size_t)k * b.nb + blockIdx.x];
+  kscan_block(b, base, blockIdx.x == 0);
+  int* h = b.hist + (size_t)blockIdx.x * b.nmu;
+  for (int k0 = threadIdx.x; k0 < b.nmu; k0 += 8 * blockDim.x) {
+    int v[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int k = k0 + q * blockDim.x;
+      v[q] = k < b.nmu ? h[k] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int k = k0 + q * blockDim.x;
+      if (k < b.nmu) {
+        base[k] += v[q];
+        h[k] = 0;              // for the next iteration's counts
+      }
+    }
+  }
   for (int t = threadIdx.x; t < kBP; t += blockDim.x) {
     long long i = blk + t;
     int l = i < b.ng ? lab[i] : -1;
@@ -1229,8 +1172,8 @@ __global__ void __launch_bounds__(1024) km_normdiff_exact(KmBufs b)
 }
 
 // Bounding box of each 256-point tile of the binned order, from the FP32 coordinates (for
-// the pruned map_to_grid).
-__global__ void km_tile_boxes(KmBufs b, float* box)
+// the pruned assign and map_to_grid; once per call).
+__global__ void km_tile_boxes(KmBufs b)
 {
   __shared__ float red[6][8];
   long long t = blockIdx.x * 256LL + threadIdx.x;
@@ -1251,7 +1194,7 @@ __global__ void km_tile_boxes(KmBufs b, float* box)
     int d = threadIdx.x;
     float v = red[d][0];
     for (int w = 1; w < 8; w++) v = d < 3 ? fminf(v, red[d][w]) : fmaxf(v, red[d][w]);
-    box[(long long)blockIdx.x * 6 + d] = v;
+    b.box[(long long)blockIdx.x * 6 + d] = v;
   }
 }
 
@@ -1517,6 +1460,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   b.gx = g64; b.gy = g64 + ng; b.gz = g64 + 2 * ng; b.rho = g64 + 3 * ng;
   b.fx = g32; b.fy = g32 + ng; b.fz = g32 + 2 * ng;
   b.pf = g32 + 3 * ng;
+  b.box = (float*)part_s;   // 6 floats per tile: at most 12 N_mu N_g / 1024 bytes from N_mu 8 on
   b.cen = cen; b.cen32 = cen32; b.labels = labels; b.hist = hist; b.total = tot;
   b.start = tot + nmu; b.member = member; b.terms = terms; b.recheck = recheck;
   b.log = logb; b.st = st;
@@ -1547,8 +1491,10 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   THC_LAUNCHED(c, "km_prep");
   km_finish_prep<<<1, 1, 0, s>>>(st, ng, nbins_max);
   THC_LAUNCHED(c, "km_finish_prep");
-  // Spatial binning of the grid (once per call): perm lists the points bin by bin.
-  const bool prune = c->km_prune && nmu >= 64;
+  // Spatial binning of the grid (once per call): perm lists the points bin by bin.  From 8
+  // centroids on, where the tile boxes fit the map's partials (part_s): at N_g 4320, N_mu 48
+  // the pruned map takes 25 us against 530, the assign 6 against 52 (FP64).
+  const bool prune = c->km_prune && nmu >= 8;
   if (prune) {
     THC_CUDA(c, cudaMemsetAsync(b.bcount, 0, sizeof(int) * 2 * (size_t)nbins_max, s));
     km_bin_count<<<(int)cdiv(ng, 256), 256, 0, s>>>(grid, b);
@@ -1557,16 +1503,13 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
     THC_LAUNCHED(c, "km_bin_scan");
     km_bin_scatter<<<(int)cdiv(ng, 256), 256, 0, s>>>(b);
     THC_LAUNCHED(c, "km_bin_scatter");
+    km_tile_boxes<<<(int)cdiv(ng, 256), 256, 0, s>>>(b);
+    THC_LAUNCHED(c, "km_tile_boxes");
   }
-  const size_t prune64_smem = (size_t)kPruneMax * (sizeof(int) + 3 * sizeof(double));
-  const size_t prune32_smem = (size_t)kPruneMax * (sizeof(int) + 3 * sizeof(float));
-  if (prune) {
-    THC_CUDA(c, cudaFuncSetAttribute(km_assign64p, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)prune64_smem));
-    THC_CUDA(c, cudaFuncSetAttribute(km_assign32p, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)prune32_smem));
-  }
-
+  // Candidates (index and FP32 coordinates) and a bit per centroid.
+  const size_t prune_smem = (size_t)kPruneMax * (sizeof(int) + 3 * sizeof(float)) +
+                            sizeof(unsigned) * (size_t)cdiv(nmu, 32);
+  THC_CUDA(c, cudaMemsetAsync(hist, 0, sizeof(int) * (size_t)nmu * b.nb, s));
   const bool mixed = c->precision == THC_PREC_MIXED;
   int nassign = (int)cdiv(ng, kAssignThreads);
   size_t hist_smem = sizeof(int) * nmu;
@@ -1581,24 +1524,23 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   // One k-means iteration; every kernel reads the iteration index from device state and
   // returns at once after convergence, so the same launch sequence serves any iteration.
   auto iteration = [&](bool prof) -> int {
-    // The pruned assign kernels count the histogram themselves (put_label).
-    THC_CUDA(c, cudaMemsetAsync(hist, 0, sizeof(int) * (size_t)nmu * b.nb, s));
-    if (mixed) {
+    // The pruned assign counts the histogram itself (put_label); the scatter clears it.
+    if (prune) {
+      ProfScope p(prof ? c : nullptr, "km_assign");
+      km_assign_p<<<nassign, kAssignThreads, prune_smem, s>>>(b);
+      THC_LAUNCHED(c, "km_assign_p");
+    } else if (mixed) {
       {
         ProfScope p(prof ? c : nullptr, "km_assign");
-        if (prune) km_assign32p<<<nassign, kAssignThreads, prune32_smem, s>>>(b);
-        else km_assign32<<<nassign, kAssignThreads, 0, s>>>(b);
+        km_assign32<<<nassign, kAssignThreads, 0, s>>>(b);
       }
       THC_LAUNCHED(c, "km_assign32");
-      if (!prune) {   // the pruned kernel rescues its near ties itself
-        km_recheck<<<152 * 4, 256, 0, s>>>(b);
-        THC_LAUNCHED(c, "km_recheck");
-      }
+      km_recheck<<<152 * 4, 256, 0, s>>>(b);
+      THC_LAUNCHED(c, "km_recheck");
     } else {
       {
         ProfScope p(prof ? c : nullptr, "km_assign");
-        if (prune) km_assign64p<<<nassign, kAssignThreads, prune64_smem, s>>>(b);
-        else km_assign64<<<nassign, kAssignThreads, 0, s>>>(b);
+        km_assign64<<<nassign, kAssignThreads, 0, s>>>(b);
       }
       THC_LAUNCHED(c, "km_assign64");
     }
@@ -1606,7 +1548,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
       km_hist<<<b.nb, 256, hist_smem, s>>>(b);
       THC_LAUNCHED(c, "km_hist");
     }
-    km_colscan<<<(int)cdiv((long long)nmu * 32, 256), 256, 0, s>>>(b);
+    km_colscan<<<(int)cdiv(nmu, 32), 32 * kScanWarps, 0, s>>>(b);
     THC_LAUNCHED(c, "km_colscan");
     km_scatter<<<b.nb, 256, hist_smem, s>>>(b);
     THC_LAUNCHED(c, "km_scatter");
@@ -1670,7 +1612,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
     const int nblock = std::min(kCheckEvery, max_it - launched);
     if (gexec && nblock == kCheckEvery) {
       THC_CUDA(c, cudaGraphLaunch(gexec, s));
-      c->launches += (mixed ? 6LL : 5LL) * kCheckEvery;  // kernels per captured iteration
+      c->launches += (prune ? 5LL : mixed ? 7LL : 6LL) * kCheckEvery;  // kernels per captured iteration
     } else {
       for (int k = 0; k < nblock; k++) {
         int rc = iteration(!fixed);
@@ -1704,11 +1646,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   int* dups = (int*)(part_i + (size_t)nmu * nch);
   THC_CUDA(c, cudaMemsetAsync(dups, 0, sizeof(int), s));
   if (prune) {
-    int ntiles = (int)cdiv(ng, 256);
-    float* box = (float*)part_s;   // 6 floats per tile fit in the partials buffer
-    km_tile_boxes<<<ntiles, 256, 0, s>>>(b, box);
-    THC_LAUNCHED(c, "km_tile_boxes");
-    km_map_pruned<<<nmu, kMapThreads, 0, s>>>(b, box, ntiles, didx);
+    km_map_pruned<<<nmu, kMapThreads, 0, s>>>(b, b.box, (int)cdiv(ng, 256), didx);
     THC_LAUNCHED(c, "km_map_pruned");
   } else {
     dim3 mg((unsigned)nch, (unsigned)cdiv(nmu, 256));
@@ -1756,7 +1694,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
     stats->duplicates = hd;
     stats->final_diff = hs.diff;
     stats->pct_changed = hs.pct;
-    stats->rechecked = hs.rechecked_total;
+    stats->rechecked = mixed ? hs.rechecked_total : 0;
     stats->device_ms = ms;
   }
   return THC_OK;
