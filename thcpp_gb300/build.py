@@ -20,7 +20,7 @@ BUILD = os.path.join(PKG, "_build")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libthc_gb300.so")
 
-CUDA_SOURCES = ["capi.cu", "kmeans.cu", "dense64.cu", "dgemm_tc.cu", "isdf.cu", "mixed.cu", "ozgemm.cu",
+CUDA_SOURCES = ["capi.cu", "kmeans.cu", "dense64.cu", "dgemm_tc.cu", "fft_tc.cu", "isdf.cu", "mixed.cu", "ozgemm.cu",
                 "ozgemm_tc.cu", "noalloc.cu", "synthgen.cu", "qrcp.cu", "halfc.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 HOST = os.path.join(PKG, "host")

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fft_tc.cuh"
 #include "ozgemm.cuh"
 #include "isdf.cuh"
 
@@ -223,6 +224,7 @@ int thc_ctx_destroy(thc_ctx* h)
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
   for (auto& kv : c->plans) cufftDestroy(kv.second);
+  thc::dft_release(c);
   for (int s = 0; s < thc::WS_NSLOTS; s++)
     if (c->ws[s]) cudaFreeAsync(c->ws[s], c->stream);
   cudaStreamSynchronize(c->stream);

@@ -90,6 +90,9 @@ struct Ctx {
   size_t ws_bytes[WS_NSLOTS] = {};
   std::map<std::tuple<int, int, int, int, int>, cufftHandle> plans;  // (n0,n1,n2,batch,type)
   std::map<std::tuple<int, int, int, int, int>, size_t> plan_work;   // their work-area bytes
+  // Digits of the DFT matrices of fft_tc.cu, by (n, real): device memory of the context's.
+  struct Dft { void* p; long long rows_pad, kpad; };
+  std::map<std::pair<int, int>, Dft> dft;
   // 4 KB pinned host scratch for asynchronous device-to-host flags.  Users (never live at
   // the same time within one call): bytes [0, 32) the k-means done flags of two blocks in
   // flight (kmeans.cu) or the CholStatus of C (mixed.cu); bytes [kPinnedCounts, +8) the

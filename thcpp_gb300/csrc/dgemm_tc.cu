@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "dense64.cuh"
+#include "digits64.cuh"
 #include "ozgemm.cuh"
 #include "tc_ptx.cuh"
 
@@ -40,7 +41,6 @@ namespace thc {
 
 namespace {
 
-constexpr int kNS = 7;                   // base-256 digits of an operand
 constexpr int kLv = 8;                   // levels, one accumulator each
 constexpr int kPeriod = 6;               // stages between drains: 192 k
 constexpr int kBN = 64;                  // tile width (128 x 64: eight TMEM slots of 64 columns)
@@ -58,112 +58,8 @@ static_assert(kSmem <= 227 * 1024, "shared memory");
 static_assert(kStageBytes % 1024 == 0, "stage alignment");
 
 constexpr long long kPair = 0x8b400000LL;  // 257 x the bits of 1.5 2^23, modulo 2^32
-constexpr int kNonFinite = 1 << 28;      // exponent mark of a row that holds an Inf or NaN
 
-// ---- cutting an operand into digits -----------------------------------------------------
-
-// A row's exponent e, |x| < 2^e for every entry, comes from the largest exponent field:
-// entries are scanned by the high word of |x| (NaN and Inf above every finite value).  A
-// scaled row takes the largest sum of the two fields, at most one above the exact exponent,
-// which keeps the FP64 multiply (two a clock on this part) out of the first pass.
-__device__ __forceinline__ unsigned abs_hi(double x)
-{
-  return (unsigned)__double2hiint(x) & 0x7fffffffu;
-}
-
-__device__ __forceinline__ int field_of(double x, double s)
-{
-  const int ex = (int)(abs_hi(x) >> 20), es = (int)(abs_hi(s) >> 20);
-  return (ex == 0x7ff || es == 0x7ff) ? kNonFinite : ex + es;
-}
-
-// e from the maximum of abs_hi (plain rows) or of field_of (scaled rows).
-template <bool SC>
-__device__ __forceinline__ int row_exponent(unsigned mx)
-{
-  if (SC) return (int)mx - 2044 > 1024 ? kNonFinite : max((int)mx - 2044, -1021);
-  const int E = (int)(mx >> 20);
-  return E == 0x7ff ? kNonFinite : max(E, 1) - 1022;
-}
-
-// R = round(x 2^{55 - e}) (half away from zero) plus the bias 128 in each of its six low
-// bytes, as two words: byte i of R then is digit 6 - i plus 128 (balanced digits in one
-// addition), and the bits from 48 on are digit 0.  base = 1022 + e.  32-bit funnel shifts;
-// a row marked kNonFinite shifts everything out (R = 0).
-__device__ __forceinline__ void cut(double x, int base, unsigned& blo, unsigned& bhi)
-{
-  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
-  const int E = (int)((h & 0x7fffffffu) >> 20);
-  const unsigned m = (h & 0xfffffu) | (E ? 0x100000u : 0u);
-  unsigned qh = __funnelshift_l(l, m, 3), ql = l << 3;          // 8 x mantissa
-  unsigned k = (unsigned)(base - max(E, 1));                    // >= 0: |x| < 2^e
-  if (k >= 32) { ql = qh; qh = 0; k -= 32; }
-  ql = __funnelshift_rc(ql, qh, k);
-  qh = k >= 32 ? 0u : qh >> k;
-  const unsigned long long q = (((unsigned long long)qh << 32 | ql) + 1) >> 1;
-  const unsigned neg = (unsigned)((int)h >> 31);
-  const unsigned long long r = (q ^ ((unsigned long long)neg << 32 | neg)) +
-                               (0x0000808080808080ULL + (neg & 1u));
-  blo = (unsigned)r;
-  bhi = (unsigned)(r >> 32);
-}
-
-// Digits of two neighbouring columns as a BF16 pair, from byte n of their biased words:
-// b - 128 = (128 + b mod 128) - (b < 128 ? 256 : 128), both terms BF16 bit patterns.
-__device__ __forceinline__ unsigned digit_pair(unsigned w0, unsigned w1, int n)
-{
-  const unsigned x = __byte_perm(w0, w1, (unsigned)(n | n << 4 | (4 + n) << 8 | (4 + n) << 12));
-  const unsigned a = (x & 0x007f007fu) | 0x43004300u, c = (~x & 0x00800080u) | 0x43004300u;
-  const __nv_bfloat162 d = __hsub2(*(const __nv_bfloat162*)&a, *(const __nv_bfloat162*)&c);
-  return *(const unsigned*)&d;
-}
-
-// Digit storage: [k / 32][digit][row][32] BF16, rows padded to 128 and k to 32 with zeros,
-// so that the 16-k tile of 128 rows and all digits is one box of a 3-D tensor map.
-struct Digits {
-  __nv_bfloat16* s = nullptr;
-  int* e = nullptr;
-  long long rows_pad = 0, kpad = 0;
-};
-
-// Cuts columns k .. k + 7 of row r: one 16-byte store per digit.
-__device__ __forceinline__ void store8(const Digits& o, long long r, long long k, int base,
-                                       const double (&v)[8])
-{
-  unsigned lo[8], hi[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) cut(v[j], base, lo[j], hi[j]);
-  __nv_bfloat16* p = o.s + (k >> 5) * (kNS * o.rows_pad * 32) + r * 32 + (k & 31);
-  const long long step = o.rows_pad * 32;
-  unsigned w[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    // (float)(hi >> 16) without the conversion pipe: |digit 0| <= 128.
-    const float f0 = __int_as_float(0x4b400000 + ((int)hi[2 * q] >> 16)) - 12582912.f;
-    const float f1 = __int_as_float(0x4b400000 + ((int)hi[2 * q + 1] >> 16)) - 12582912.f;
-    const __nv_bfloat162 d = __floats2bfloat162_rn(f0, f1);
-    w[q] = *(const unsigned*)&d;
-  }
-  *(uint4*)p = make_uint4(w[0], w[1], w[2], w[3]);
-#pragma unroll
-  for (int i = 1; i < kNS; i++) {
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      w[q] = i < 3 ? digit_pair(hi[2 * q], hi[2 * q + 1], 2 - i)
-                   : digit_pair(lo[2 * q], lo[2 * q + 1], 6 - i);
-    *(uint4*)(p + i * step) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-}
-
-// Where an operand's element (row r, index k) lies and what multiplies it.
-struct CutSrc {
-  const double* x;
-  long long rows, sr, sk;    // x[r sr + k sk]
-  int k0, K;                 // the panel's first k and its length
-  const double* scale;       // SC: indexed (k0 + k) >> shift
-  int shift;
-  bool vec;                  // sk == 1, rows 16-byte aligned
-};
+// ---- cutting an operand into digits (digits64.cuh) --------------------------------------
 
 __device__ __forceinline__ void load8(const CutSrc& a, long long r, int k, double (&v)[8])
 {
@@ -796,7 +692,6 @@ int digit_map(Ctx* c, CUtensorMap* map, const Digits& d, int box_rows)
   return THC_OK;
 }
 
-// Digits of one operand's panel (k0, K) into d.
 template <bool SC>
 int cut_operand_t(Ctx* c, const CutSrc& a, const Digits& d, unsigned* rowmax, int* flag)
 {
@@ -823,14 +718,68 @@ int cut_operand_t(Ctx* c, const CutSrc& a, const Digits& d, unsigned* rowmax, in
   return THC_OK;
 }
 
-int cut_operand(Ctx* c, const CutSrc& a, const Digits& d, unsigned* rowmax, int* flag)
+}  // namespace
+
+int digits_cut(Ctx* c, const CutSrc& a, const Digits& d, unsigned* rowmax, int* flag)
 {
   ProfScope prof(c, "slice64");
   return a.scale ? cut_operand_t<true>(c, a, d, rowmax, flag)
                  : cut_operand_t<false>(c, a, d, rowmax, flag);
 }
 
-}  // namespace
+int digits_product(Ctx* c, const Digits& a, const Digits& b, const GemmArgs& g)
+{
+  int sms = 0, st;
+  THC_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  THC_CUDA(c, cudaFuncSetAttribute(dgemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kSmem));
+  Args t;
+  t.M = g.M; t.N = g.N;
+  t.stages = (int)(a.kpad / kBK);
+  t.ea = a.e; t.eb = b.e;
+  t.C = g.C; t.ldc = g.ldc; t.alpha = g.alpha; t.beta = g.beta;
+  t.lower = g.lower_only;
+  t.error = c->tc64_err;
+  t.spin_limit = c->spin_limit;
+  t.mtn = cdiv(g.M, TBM);
+  t.ntn = cdiv(g.N, kBN);
+  t.tiles = g.lower_only ? (t.mtn - 1) * t.mtn + std::min(2 * t.mtn, t.ntn) : t.mtn * t.ntn;
+  // Split of K: waves x (k tiles per item + ~3 k tiles' worth of fill and final drain).
+  const int kt = t.stages;
+  int best = 1;
+  double cost = 0.0;
+  for (int z = 1; z <= std::min(kt, 256); z++) {
+    const int pk = (int)cdiv(kt, z);
+    if ((size_t)z * g.M * g.N * 8 > ((size_t)1 << 30) && z > 1) break;
+    const double w = (double)cdiv(t.tiles * cdiv(kt, pk), sms) * (pk + 3) + (z > 1 ? 2.0 : 0.0);
+    if (z == 1 || w < 0.98 * cost) { cost = w; best = z; }
+  }
+  t.kt_per = (int)cdiv(kt, best);
+  t.ksplit = (int)cdiv(kt, t.kt_per);
+  t.part = nullptr;
+  if (t.ksplit > 1) {
+    t.part = (double*)ws_get(c, WS_DPART, sizeof(double) * t.ksplit * g.M * g.N);
+    if (!t.part) { t.ksplit = 1; t.kt_per = kt; }
+  }
+  t.square = t.ksplit == 1 && g.mode == GEMM_SQUARE;
+  t.scaled = t.ksplit == 1 && g.alpha != 1.0;
+  t.added = t.ksplit == 1 && g.beta != 0.0;
+  CUtensorMap ma, mb;
+  if ((st = digit_map(c, &ma, a, TBM)) || (st = digit_map(c, &mb, b, kBN))) return st;
+  const unsigned grid = (unsigned)std::min<long long>(t.tiles * t.ksplit, sms);
+  {
+    ProfScope prof(c, "dgemm_tc");
+    dgemm_tc_kernel<<<grid, kThreads, kSmem, c->stream>>>(ma, mb, t);
+    THC_LAUNCHED(c, "dgemm_tc");
+  }
+  if (t.ksplit > 1) {
+    GemmArgs p = g;
+    p.ksplit = t.ksplit;
+    p.part = t.part;
+    return dgemm_reduce_partials(c, p);
+  }
+  return THC_OK;
+}
 
 bool dgemm_tc_fits(const Ctx* c, const GemmArgs& g)
 {
@@ -878,8 +827,6 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
   int* nonfin = (int*)flags;
   int sms = 0;
   THC_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  THC_CUDA(c, cudaFuncSetAttribute(dgemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kSmem));
   auto vec = [](const double* p, long long sr, long long sk) {
     return sk == 1 && sr % 2 == 0 && (uintptr_t)p % 16 == 0;
   };
@@ -891,7 +838,7 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
     {
       CutSrc a{g.A, g.M, g.sam, g.sak, k0, K, same ? dkr : g.dk, g.dk_shift,
                vec(g.A, g.sam, g.sak)};
-      if ((st = cut_operand(c, a, da, rowmax, nonfin))) return st;
+      if ((st = digits_cut(c, a, da, rowmax, nonfin))) return st;
     }
     for (long long n0 = 0; n0 < g.N; n0 += npan) {
       GemmArgs p = g;
@@ -905,52 +852,9 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
         db.rows_pad = oz_pad_mn(p.N);
         db.e = eb_own;
         CutSrc b{p.B, p.N, g.sbn, g.sbk, k0, K, nullptr, 0, vec(p.B, g.sbn, g.sbk)};
-        if ((st = cut_operand(c, b, db, rowmax, nonfin))) return st;
+        if ((st = digits_cut(c, b, db, rowmax, nonfin))) return st;
       }
-      Args t;
-      t.M = p.M; t.N = p.N;
-      t.stages = (int)(da.kpad / kBK);
-      t.ea = da.e; t.eb = db.e;
-      t.C = p.C; t.ldc = p.ldc; t.alpha = p.alpha; t.beta = p.beta;
-      t.lower = p.lower_only;
-      t.error = c->tc64_err;
-      t.spin_limit = c->spin_limit;
-      t.mtn = cdiv(p.M, TBM);
-      t.ntn = cdiv(p.N, kBN);
-      t.tiles = p.lower_only ? (t.mtn - 1) * t.mtn + std::min(2 * t.mtn, t.ntn) : t.mtn * t.ntn;
-      // Split of K: waves x (k tiles per item + ~3 k tiles' worth of fill and final drain).
-      const int kt = t.stages;
-      int best = 1;
-      double cost = 0.0;
-      for (int z = 1; z <= std::min(kt, 256); z++) {
-        const int pk = (int)cdiv(kt, z);
-        if ((size_t)z * p.M * p.N * 8 > ((size_t)1 << 30) && z > 1) break;
-        const double w = (double)cdiv(t.tiles * cdiv(kt, pk), sms) * (pk + 3) + (z > 1 ? 2.0 : 0.0);
-        if (z == 1 || w < 0.98 * cost) { cost = w; best = z; }
-      }
-      t.kt_per = (int)cdiv(kt, best);
-      t.ksplit = (int)cdiv(kt, t.kt_per);
-      t.part = nullptr;
-      if (t.ksplit > 1) {
-        t.part = (double*)ws_get(c, WS_DPART, sizeof(double) * t.ksplit * p.M * p.N);
-        if (!t.part) { t.ksplit = 1; t.kt_per = kt; }
-      }
-      t.square = t.ksplit == 1 && p.mode == GEMM_SQUARE;
-      t.scaled = t.ksplit == 1 && p.alpha != 1.0;
-      t.added = t.ksplit == 1 && p.beta != 0.0;
-      CUtensorMap ma, mb;
-      if ((st = digit_map(c, &ma, da, TBM)) || (st = digit_map(c, &mb, db, kBN))) return st;
-      const unsigned grid = (unsigned)std::min<long long>(t.tiles * t.ksplit, sms);
-      {
-        ProfScope prof(c, "dgemm_tc");
-        dgemm_tc_kernel<<<grid, kThreads, kSmem, c->stream>>>(ma, mb, t);
-        THC_LAUNCHED(c, "dgemm_tc");
-      }
-      if (t.ksplit > 1) {
-        p.ksplit = t.ksplit;
-        p.part = t.part;
-        if ((st = dgemm_reduce_partials(c, p))) return st;
-      }
+      if ((st = digits_product(c, da, db, p))) return st;
       fix_nonfinite<<<(unsigned)(2 * sms), 256, 0, c->stream>>>(p, k0, K, da.e, db.e, nonfin);
       THC_LAUNCHED(c, "fix_nonfinite");
     }

@@ -13,9 +13,10 @@
 // C has full rank for a sensible point set but no symmetry, so the reference's QR solve is
 // replaced by the inverse from Gauss-Jordan elimination with partial pivoting (one pivot
 // kernel and one elimination kernel per column, on [C | I]; N_mu^3 complex FMAs, small next
-// to the N_mu^2 N_g of the products), then X = C^{-1} Z as four real FP64 GEMMs.  Complex
-// values are (re, im) pairs; P and Z are kept as separate real and imaginary N_mu x N_g
-// matrices so that every product is a real GEMM of dense64.cu.
+// to the N_mu^2 N_g of the products), then X = C^{-1} Z.  Complex values are (re, im) pairs; P
+// and Z are kept as their real N_mu x N_g matrix and the imaginary one behind it, so that every
+// complex product is one real GEMM (of twice the rows, or the terms) with each operand cut
+// once.  IVMG(G) = IVG(-G), so one transform serves both.
 #include <cuda_runtime.h>
 #include <cufft.h>
 
@@ -24,6 +25,7 @@
 
 #include "common.cuh"
 #include "dense64.cuh"
+#include "fft_tc.cuh"
 #include "isdf.cuh"
 
 namespace thc {
@@ -193,6 +195,44 @@ __global__ void conj_interleave(const double* __restrict__ xr, const double* __r
   z[2 * e + 1] = -xi[e];
 }
 
+// The left operand of M from the forward spectra: the backward transform of a field at G is its
+// forward one at -G.  left1 = (re, -im) and left2 = (im, re) of IVMG(G) = IVG(-G), so that over
+// (re, im) pairs left1 . IVG = Re(IVMG IVG) and left2 . IVG = Im; vs = v in the spectrum's order
+// (zyx: kz, ky, kx with kx fastest, as fft_tc leaves it; else kz fastest).
+__global__ void left_spectra(const double2* __restrict__ ivg, const double* __restrict__ v, int n0,
+                             int n1, int n2, bool zyx, int nmu, double2* left1, double2* left2,
+                             double* vs)
+{
+  const long long ng = (long long)n0 * n1 * n2;
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (e >= ng) return;
+  const int d0 = zyx ? n0 : n2;                       // fastest axis, then n1, then the other
+  const int f = (int)(e % d0), k1 = (int)(e / d0 % n1), sl = (int)(e / d0 / n1);
+  const int ds = zyx ? n2 : n0;
+  const long long m = ((long long)((ds - sl) % ds) * n1 + (n1 - k1) % n1) * d0 + (d0 - f) % d0;
+  if (blockIdx.y == 0) vs[e] = zyx ? v[((long long)f * n1 + k1) * n2 + sl] : v[e];
+  for (int mu = blockIdx.y; mu < nmu; mu += gridDim.y) {
+    const double2 p = ivg[mu * ng + m];
+    left1[mu * ng + e] = make_double2(p.x, -p.y);
+    left2[mu * ng + e] = make_double2(p.y, p.x);
+  }
+}
+
+// [Re C^-1, -Im C^-1] over [Im C^-1, Re C^-1] (2n x 2n) from the right half of [C | I] after the
+// elimination: with Z's real rows over its imaginary ones, one real product gives X's.
+__global__ void inverse_pairs(const double* __restrict__ aug, int n, double* out)
+{
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (e >= (long long)n * n) return;
+  const int r = (int)(e / n), c = (int)(e % n);
+  const double re = aug[2 * ((long long)r * 2 * n + n + c)];
+  const double im = aug[2 * ((long long)r * 2 * n + n + c) + 1];
+  out[(long long)r * 2 * n + c] = re;
+  out[(long long)r * 2 * n + n + c] = -im;
+  out[(long long)(n + r) * 2 * n + c] = im;
+  out[(long long)(n + r) * 2 * n + n + c] = re;
+}
+
 __global__ void interleave(const double* __restrict__ re, const double* __restrict__ im,
                            long long n, double* out)
 {
@@ -254,9 +294,9 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
     return set_error(c, THC_ERR_NOMEM, "thc_isdf_half_complex: workspace allocation failed");
   double* pmu = rows;
   double* pmu_rot = pmu + 2LL * nmu * no;
-  double* omu = pmu_rot + 2LL * nmu * no;
+  double* omu = pmu_rot + 2LL * nmu * no;   // each followed by its rotation
   double* omu_rot = omu + 2LL * nmu * nocc;
-  double *pr = prpi, *pi = prpi + nmg, *qr = qrqi, *qi = qrqi + nmg;
+  double *pr = prpi, *pi = prpi + nmg, *qr = qrqi, *qi = qrqi + nmg;   // Re and Im
   GjStatus* gs = (GjStatus*)scr;
   int* bad = (int*)(scr + 512);
   double* orb_dev = out_orb ? (orb_host ? stage : out_orb) : nullptr;
@@ -277,22 +317,17 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
     THC_CUDA(c, cudaMemcpyAsync(out_orb_occ, occ_dev, sizeof(double) * 2 * nmu * nocc,
                                 cudaMemcpyDeviceToHost, s));
   // Re(a^H b) and Im(a^H b) as real dot products over the (re, im) pairs: a . b and
-  // rot(a) . b with rot(a) = (-im, re).
-  auto pseudo_dm = [&](const double* amu, const double* arot, const double* full, int k,
-                       double* re, double* im) -> int {
+  // rot(a) . b with rot(a) = (-im, re), whose rows follow a's; so do the results'.
+  auto pseudo_dm = [&](const double* amu, const double* full, int k, double* out) -> int {
     GemmArgs g;
-    g.M = nmu; g.N = ng; g.K = 2 * k;
+    g.M = 2LL * nmu; g.N = ng; g.K = 2 * k;
     g.A = amu; g.sam = 2 * k; g.sak = 1;
     g.B = full; g.sbn = 2 * k; g.sbk = 1;
-    g.C = re; g.ldc = ng;
-    int r = dgemm(c, g);
-    if (r) return r;
-    g.A = arot;
-    g.C = im;
+    g.C = out; g.ldc = ng;
     return dgemm(c, g);
   };
-  if ((st = pseudo_dm(pmu, pmu_rot, phi, no, pr, pi))) return st;
-  if ((st = pseudo_dm(omu, omu_rot, occ, nocc, qr, qi))) return st;
+  if ((st = pseudo_dm(pmu, phi, no, prpi))) return st;
+  if ((st = pseudo_dm(omu, occ, nocc, qrqi))) return st;
   half_product<<<(int)cdiv(nmg, 256), 256, 0, s>>>(pr, pi, qr, qi, nmg);
   THC_LAUNCHED(c, "half_product");
   // C^{-1} by Gauss-Jordan elimination on [C | I].
@@ -305,31 +340,30 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   }
   c->launches += 2LL * nmu;
   THC_LAUNCHED(c, "gj_eliminate");
-  // X = C^{-1} Z:  XR = CiR ZR - CiI ZI,  XI = CiR ZI + CiI ZR  (into the P_occ buffers).
+  // X = C^{-1} Z as one real product of 2 N_mu rows and 2 N_mu terms (into the P_occ buffers).
   {
-    const double* cir = aug + 2LL * nmu;             // right half, real parts (stride 2)
-    const double* cii = cir + 1;
-    auto prod = [&](const double* a, const double* b, double* out, double alpha,
-                    double beta) -> int {
-      GemmArgs g;
-      g.M = nmu; g.N = ng; g.K = nmu;
-      g.A = a; g.sam = 4LL * nmu; g.sak = 2;
-      g.B = b; g.sbn = 1; g.sbk = ng;
-      g.C = out; g.ldc = ng; g.alpha = alpha; g.beta = beta;
-      return dgemm(c, g);
-    };
-    if ((st = prod(cir, pr, qr, 1.0, 0.0))) return st;
-    if ((st = prod(cii, pi, qr, -1.0, 1.0))) return st;
-    if ((st = prod(cir, pi, qi, 1.0, 0.0))) return st;
-    if ((st = prod(cii, pr, qi, 1.0, 1.0))) return st;
+    double* ci = (double*)ws_get(c, WS_DINV, sizeof(double) * 4 * nn);
+    if (!ci) return set_error(c, THC_ERR_NOMEM, "thc_isdf_half_complex: inverse");
+    inverse_pairs<<<(int)cdiv(nn, 256), 256, 0, s>>>(aug, nmu, ci);
+    THC_LAUNCHED(c, "inverse_pairs");
+    GemmArgs g;
+    g.M = 2LL * nmu; g.N = ng; g.K = 2 * nmu;
+    g.A = ci; g.sam = 2LL * nmu; g.sak = 1;
+    g.B = prpi; g.sbn = 1; g.sbk = ng;
+    g.C = qrqi; g.ldc = ng;
+    if ((st = dgemm(c, g))) return st;
   }
   // zeta = conj(X), interleaved for cuFFT (in the P buffers), then both transforms.
   double* zc = prpi;
   conj_interleave<<<(int)cdiv(nmg, 256), 256, 0, s>>>(qr, qi, nmg, zc);
   THC_LAUNCHED(c, "conj_interleave");
   double* ivg = spec;
-  double* ivmg = spec + 2 * nmg;
-  {
+  double* left1 = spec + 2 * nmg;
+  double* left2 = prpi;              // after the transform
+  const bool fft_products = fft_tc_fits(c, mesh[0], mesh[1], mesh[2], nmu);
+  if (fft_products) {
+    if ((st = fft_tc(c, mesh[0], mesh[1], mesh[2], nmu, false, zc, ivg))) return st;
+  } else {
     ProfScope prof(c, "fft");
     for (int f0 = 0; f0 < nmu; f0 += kFftChunk) {
       const int nb = std::min(kFftChunk, nmu - f0);
@@ -337,33 +371,37 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
       if ((st = get_plan(c, mesh[0], mesh[1], mesh[2], nb, CUFFT_Z2Z, &plan))) return st;
       cufftDoubleComplex* src = (cufftDoubleComplex*)(zc + 2LL * ng * f0);
       if (cufftExecZ2Z(plan, src, (cufftDoubleComplex*)(ivg + 2LL * ng * f0), CUFFT_FORWARD) !=
-              CUFFT_SUCCESS ||
-          cufftExecZ2Z(plan, src, (cufftDoubleComplex*)(ivmg + 2LL * ng * f0), CUFFT_INVERSE) !=
-              CUFFT_SUCCESS)
+          CUFFT_SUCCESS)
         return set_error(c, THC_ERR_CUFFT, "thc_isdf_half_complex: cufftExecZ2Z failed");
-      c->launches += 2;
+      c->launches++;
     }
   }
+  double* vs = (double*)ws_get(c, WS_DSYM, sizeof(double) * ng);
+  if (!vs) return set_error(c, THC_ERR_NOMEM, "thc_isdf_half_complex: Coulomb kernel");
+  left_spectra<<<dim3((unsigned)cdiv(ng, 256), 16), 256, 0, s>>>(
+      (const double2*)ivg, coul, mesh[0], mesh[1], mesh[2], fft_products, nmu, (double2*)left1,
+      (double2*)left2, vs);
+  THC_LAUNCHED(c, "left_spectra");
   c->zeta_last = nullptr;            // complex vectors: not served by the real accessor
-  // M = sum_G v(G) IVMG_mu(G) IVG_nu(G):  MR = sum v (ar br - ai bi), MI = sum v (ar bi + ai br).
+  // M = sum_G v(G) IVMG_mu(G) IVG_nu(G) over (re, im) pairs: the real and the imaginary part.
   double* mr = Mw;
   double* mi = Mw + nn;
   {
-    auto prod = [&](const double* a, const double* b, double* out, double alpha,
-                    double beta) -> int {
-      GemmArgs g;
-      g.M = nmu; g.N = nmu; g.K = (int)ng;
-      g.A = a; g.sam = 2 * ng; g.sak = 2;
-      g.B = b; g.sbn = 2 * ng; g.sbk = 2;
-      g.dk = coul; g.dk_shift = 0;
-      g.C = out; g.ldc = nmu; g.alpha = alpha; g.beta = beta;
-      return dgemm(c, g);
-    };
     if (ng > 0x7fffffffLL) return set_error(c, THC_ERR_SHAPE, "thc_isdf_half_complex: mesh too large");
-    if ((st = prod(ivmg, ivg, mr, 1.0, 0.0))) return st;
-    if ((st = prod(ivmg + 1, ivg + 1, mr, -1.0, 1.0))) return st;
-    if ((st = prod(ivmg, ivg + 1, mi, 1.0, 0.0))) return st;
-    if ((st = prod(ivmg + 1, ivg, mi, 1.0, 1.0))) return st;
+    constexpr long long kPart = 1LL << 30;           // the GEMM's K is an int
+    for (long long k = 0; k < 2 * ng; k += kPart) {
+      GemmArgs g;
+      g.M = nmu; g.N = nmu; g.K = (int)std::min(kPart, 2 * ng - k);
+      g.A = left1 + k; g.sam = 2 * ng; g.sak = 1;
+      g.B = ivg + k; g.sbn = 2 * ng; g.sbk = 1;
+      g.dk = vs + k / 2; g.dk_shift = 1;
+      g.beta = k ? 1.0 : 0.0;
+      g.C = mr; g.ldc = nmu;
+      if ((st = dgemm(c, g))) return st;
+      g.A = left2 + k;
+      g.C = mi;
+      if ((st = dgemm(c, g))) return st;
+    }
   }
   double* mcx = Mw + 2 * nn;
   interleave<<<(int)cdiv(nn, 256), 256, 0, s>>>(mr, mi, nn, mcx);

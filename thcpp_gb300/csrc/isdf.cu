@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "dense64.cuh"
+#include "fft_tc.cuh"
 #include "isdf.cuh"
 
 namespace thc {
@@ -64,7 +65,7 @@ __global__ void gather_rows(const double* __restrict__ phi, long long ng, int no
 // root = sqrt|dsym|, for a product that takes half the weight on each side.
 __global__ void coulomb_weights(const double* __restrict__ v, int n0, int n1, int n2,
                                 double* dsym, double* danti, double* root, int* n_anti,
-                                int* n_neg)
+                                int* n_neg, bool zyx)
 {
   int nc = n2 / 2 + 1;
   long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -73,6 +74,12 @@ __global__ void coulomb_weights(const double* __restrict__ v, int n0, int n1, in
   int k2 = (int)(e % nc);
   long long r = e / nc;
   int k1 = (int)(r % n1), k0 = (int)(r / n1);
+  if (zyx) {                 // the spectrum's order (fft_tc): kz, ky, kx with kx fastest
+    k0 = (int)(e % n0);
+    r = e / n0;
+    k1 = (int)(r % n1);
+    k2 = (int)(r / n1);
+  }
   int j0 = (n0 - k0) % n0, j1 = (n1 - k1) % n1, j2 = (n2 - k2) % n2;
   double vp = v[((long long)k0 * n1 + k1) * n2 + k2];
   double vn = v[((long long)j0 * n1 + j1) * n2 + j2];
@@ -351,8 +358,9 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
 
   // The Coulomb weights depend on the kernel only: with them first, their counts reach the
   // host with C's factorisation status and cost no wait of their own.
+  const bool fft_products = fft_tc_fits(c, n0, n1, n2, nmu);
   coulomb_weights<<<(int)cdiv(nc, 256), 256, 0, s>>>(coul, n0, n1, n2, dsym, danti, droot, n_anti,
-                                                     n_neg);
+                                                     n_neg, fft_products);
   THC_LAUNCHED(c, "coulomb_weights");
   int h_counts[2] = {0, 0};            // n_anti, n_neg
   gather_rows<<<(int)cdiv((long long)nmu * kw, 256), 256, 0, s>>>(phi, ng, kw, idx, nmu, phimu,
@@ -509,7 +517,9 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
     if ((st = dgemm(c, g))) return st;
   }
   // FFT of every interpolating vector.
-  if ((st = fft_forward(c, n0, n1, n2, nmu, CUFFT_D2Z, zeta, zhat))) return st;
+  if ((st = fft_products ? fft_tc(c, n0, n1, n2, nmu, true, zeta, zhat)
+                         : fft_forward(c, n0, n1, n2, nmu, CUFFT_D2Z, zeta, zhat)))
+    return st;
   const int h_anti = h_counts[0];
   // Re M (lower) = sum_k zh[mu,k] dsym[k/2] zh[nu,k] over interleaved (re, im) pairs.
   double* mre = Mw;
