@@ -241,30 +241,32 @@ struct Args {
   double alpha, beta;
   int square, scaled, added;   // epilogue: the square, alpha != 1, beta != 0 (not with a split)
   int lower;
+  unsigned two8, two16;    // 2^8 and 2^16: factors of integer multiply-adds, opaque (constants
+                           // become shifts on the integer pipe)
   double* part;
   int* error;
   long long spin_limit;
-  long long mtn, ntn, tiles;
+  unsigned mtn, ntn, tiles;  // 32-bit: a 64-bit division is a hundred instructions, per warp
+                             // and tile
 };
 
 constexpr int kGroupM = 16;    // m-tiles swept per n-tile: the CTAs of a wave share B tiles
 
-__device__ __forceinline__ void tile_of(const Args& g, long long t, long long& mt, long long& nt)
+__device__ __forceinline__ void tile_of(const Args& g, unsigned t, unsigned& mt, unsigned& nt)
 {
   if (g.lower) {
     // Row i of 128 x 64 tiles reaches column 2i + 1: it starts at tile i (i + 1).
-    long long i = (long long)((sqrtf(4.f * (float)t + 1.f) - 1.f) * 0.5f);
+    unsigned i = (unsigned)((sqrtf(4.f * (float)t + 1.f) - 1.f) * 0.5f);
     while (i * (i + 1) > t) i--;
     while ((i + 1) * (i + 2) <= t) i++;
     mt = i;
     nt = t - i * (i + 1);
     return;
   }
-  const long long per = (long long)kGroupM * g.ntn, grp = t / per, first = grp * kGroupM;
-  const long long gm = g.mtn - first < kGroupM ? g.mtn - first : kGroupM;
-  const long long r = t - grp * per;
-  mt = first + r % gm;
+  const unsigned per = kGroupM * g.ntn, grp = t / per, first = grp * kGroupM;
+  const unsigned gm = min(g.mtn - first, (unsigned)kGroupM), r = t - grp * per;
   nt = r / gm;
+  mt = first + r - nt * gm;
 }
 
 // 2^E v by ldexp: results that leave FP64's normal range.
@@ -280,27 +282,31 @@ __device__ __noinline__ double wide_double(unsigned hi, unsigned lo, int E, unsi
 // operations of the FP64 pipe, 16,000 clocks a tile.)
 template <bool WIDE>
 __device__ __forceinline__ double to_double(unsigned w0, unsigned w1, unsigned w2, int E,
-                                            unsigned& wide)
+                                            bool& wide)
 {
-  const unsigned neg = (unsigned)((int)w2 >> 31);     // all ones for a negative sum
+  // The magnitude as the one's complement of a negative sum: a unit of 2^-70 2^{eA+eB} less,
+  // far below the expansion's truncation.
+  const unsigned neg = (unsigned)((int)w2 >> 31);
   w0 ^= neg;
   w1 ^= neg;
   w2 ^= neg;
-  asm("add.cc.u32 %0, %0, %3;\n addc.cc.u32 %1, %1, 0;\n addc.u32 %2, %2, 0;\n"
-      : "+r"(w0), "+r"(w1), "+r"(w2) : "r"(neg & 1u));
+  const bool zero = (w0 | w1 | w2) == 0;
   int be = E + 95 + 1022;                             // biased exponent of bit 95, less one
   if (!w2) { w2 = w1; w1 = w0; w0 = 0; be -= 32; }
-  if (!w2) { w2 = w1; w1 = 0; be -= 32; }
-  if (!w2) return 0.0;
+  if (WIDE) {
+    if (zero) return 0.0;
+    if (!w2) { w2 = w1; w1 = 0; be -= 32; }
+  }
   const int n = __clz((int)w2);
   be -= n;
   const unsigned t1 = __funnelshift_l(w1, w2, n), t0 = __funnelshift_l(w0, w1, n);
   if (WIDE && (unsigned)be > 2044u) return wide_double(t1, t0, be - 1022 - 63, neg);
-  wide |= (unsigned)be > 2044u;
+  wide |= !zero && ((unsigned)be > 2044u || !w2);
   unsigned m0 = __funnelshift_r(t0, t1, 11), m1 = (t1 >> 11) + ((unsigned)be << 20);
   asm("add.cc.u32 %0, %0, %2;\n addc.u32 %1, %1, 0;\n"
       : "+r"(m0), "+r"(m1) : "r"((t0 >> 10) & 1u));
-  return __hiloint2double((int)(m1 | (neg & 0x80000000u)), (int)m0);
+  m1 |= neg & 0x80000000u;
+  return zero ? 0.0 : __hiloint2double((int)m1, (int)m0);
 }
 
 // One CTA per SM walks the items (tile, split of K).  Warp 0 is the TMA producer, warp 1
@@ -357,7 +363,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   int* sexp = (int*)((unsigned char*)full + 256);   // 16 warps x 16 column exponents
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long items = g.tiles * g.ksplit;
+  const unsigned items = g.tiles * g.ksplit;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -383,9 +389,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = *tmem_slot;
 
   // First stage and stage count of item t, and its tile.
-  auto item_of = [&](long long t, long long& mt, long long& nt, int& st0, int& nst) {
-    const int z = (int)(t / g.tiles);
-    tile_of(g, t - (long long)z * g.tiles, mt, nt);
+  auto item_of = [&](unsigned t, unsigned& mt, unsigned& nt, int& st0, int& nst) {
+    const unsigned z = g.ksplit > 1 ? t / g.tiles : 0u;
+    tile_of(g, t - z * g.tiles, mt, nt);
     st0 = z * g.kt_per;
     nst = min(g.stages - st0, g.kt_per);
   };
@@ -395,8 +401,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       int git = 0;
       bool ok = true;
-      for (long long t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        long long mt, nt;
+      for (unsigned t = blockIdx.x; t < items && ok; t += gridDim.x) {
+        unsigned mt, nt;
         int st0, nst;
         item_of(t, mt, nt, st0, nst);
         for (int it = 0; it < nst; it++, git++) {
@@ -420,8 +426,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       int git = 0;
       uint32_t pc = 0;               // periods begun
       bool ok = true;
-      for (long long t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        long long mt, nt;
+      for (unsigned t = blockIdx.x; t < items && ok; t += gridDim.x) {
+        unsigned mt, nt;
         int st0, nst;
         item_of(t, mt, nt, st0, nst);
         int in_period = 0;
@@ -480,11 +486,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     double* stg = (double*)(stg_base + (size_t)ew * (32 * 8 * 8));
     uint32_t pc = 0;                         // periods drained
     bool ok = true;
-    for (long long t = blockIdx.x; t < items && ok; t += gridDim.x) {
-      long long mt, nt;
+    for (unsigned t = blockIdx.x; t < items && ok; t += gridDim.x) {
+      unsigned mt, nt;
       int st0, nst;
       item_of(t, mt, nt, st0, nst);
-      const long long m0 = mt * TBM, n0 = nt * kBN;
+      const long long m0 = (long long)mt * TBM, n0 = (long long)nt * kBN;
       if (lane < kEC) {
         const long long na = n0 + col0 + lane;
         seb[lane] = na < g.N ? g.eb[na] : 0;
@@ -506,55 +512,55 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       // P = 256 V_l + V_{l+1} of eight columns, plus kPair, in 32 bits: V plus a constant is
-      // the bits of V + 1.5 2^23, exactly while |V| <= 2^22; beyond that (digits of one sign
-      // nearly throughout) `off` shows it.
-      auto pair8 = [&](uint32_t src, unsigned (&P)[8], unsigned& off) {
+      // the bits of V + 1.5 2^23, exactly while |V| <= 2^22.  That always holds for level 0;
+      // the squares of the others add up to `sq`, which stays below 2^43 unless their digits
+      // have one sign nearly throughout.  (The sum runs on the FMA pipe; the integer pipe is
+      // the one the epilogue fills.)
+      auto pair8 = [&](uint32_t src, unsigned (&P)[8], float& sq, bool level0) {
         float a[8], c[8];
-        tmem_ld8_issue(src, a);
-        tmem_ld8_issue(src + kBN, c);
-        tmem_ld_wait(a);
-        tmem_ld_wait(c);
+        tmem_ld8x2(src, src + kBN, a, c);
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-          const unsigned x = __float_as_uint(__fadd_rn(a[q], 12582912.f));
-          const unsigned y = __float_as_uint(__fadd_rn(c[q], 12582912.f));
-          off |= (x ^ 0x4b000000u) | (y ^ 0x4b000000u);
-          P[q] = x * 256u + y;
+          if (!level0) sq = __fmaf_rn(a[q], a[q], sq);
+          sq = __fmaf_rn(c[q], c[q], sq);
+          P[q] = __float_as_uint(__fadd_rn(a[q], 12582912.f)) * g.two8 +
+                 __float_as_uint(__fadd_rn(c[q], 12582912.f));
         }
       };
+      // Warps past the last column have nothing to collect or store.
+      const bool act = n0 + col0 < g.N;
       for (int st = 0; st < nst; st += kPeriod, pc++) {
         if (!mbar_wait(acc_full, pc & 1u, abort, g.spin_limit)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;\n");
 #pragma unroll
         for (int l = 4; l >= 0; l -= 4) {      // levels 4-7, then 0-3
 #pragma unroll
-          for (int b = 0; b < kEC; b += 8) {
+          for (int b = 0; b < kEC && act; b += 8) {
             const uint32_t src = tmem + lane_base + (uint32_t)(l * kBN + col0 + b);
-            unsigned P[8], Q[8], off = 0;
-            pair8(src + 2 * kBN, P, off);
-            pair8(src, Q, off);
-            if (!__any_sync(0xffffffffu, off >> 23)) {
+            unsigned P[8], Q[8];
+            float sq = 0.f;
+            pair8(src + 2 * kBN, P, sq, false);
+            pair8(src, Q, sq, l == 0);
+            if (!__any_sync(0xffffffffu, !(sq < 0x1p43f))) {
 #pragma unroll
               for (int q = 0; q < 8; q++) {
                 // 2^16 Q + P, 48 bits, at bit 0 (levels 4-7) or bit 32.
-                unsigned lo = Q[q] << 16, hi = Q[q] >> 16;
+                unsigned long long x = P[q];
+                asm("mad.wide.u32 %0, %1, %2, %0;\n" : "+l"(x) : "r"(Q[q]), "r"(g.two16));
+                const unsigned lo = (unsigned)x, hi = (unsigned)(x >> 32);
                 if (l)
-                  asm("add.cc.u32 %3, %3, %5;\n addc.u32 %4, %4, 0;\n add.cc.u32 %0, %0, %3;\n"
-                      " addc.cc.u32 %1, %1, %4;\n addc.u32 %2, %2, 0;\n"
-                      : "+r"(w0[b + q]), "+r"(w1[b + q]), "+r"(w2[b + q]), "+r"(lo), "+r"(hi)
-                      : "r"(P[q]));
+                  asm("add.cc.u32 %0, %0, %3;\n addc.cc.u32 %1, %1, %4;\n addc.u32 %2, %2, 0;\n"
+                      : "+r"(w0[b + q]), "+r"(w1[b + q]), "+r"(w2[b + q]) : "r"(lo), "r"(hi));
                 else
-                  asm("add.cc.u32 %2, %2, %4;\n addc.u32 %3, %3, 0;\n add.cc.u32 %0, %0, %2;\n"
-                      " addc.u32 %1, %1, %3;\n"
-                      : "+r"(w1[b + q]), "+r"(w2[b + q]), "+r"(lo), "+r"(hi) : "r"(P[q]));
+                  asm("add.cc.u32 %0, %0, %2;\n addc.u32 %1, %1, %3;\n"
+                      : "+r"(w1[b + q]), "+r"(w2[b + q]) : "r"(lo), "r"(hi));
               }
             } else {
               // By conversion (16 a clock and SM), level by level.
 #pragma unroll 1
               for (int j = 0; j < 4; j++) {
                 float v[8];
-                tmem_ld8_issue(src + (uint32_t)(j * kBN), v);
-                tmem_ld_wait(v);
+                tmem_ld8(src + (uint32_t)(j * kBN), v);
                 const long long weight = 1LL << (24 - 8 * j);
                 const long long more = j & 1 ? kPair << (j == 1 ? 16 : 0) : 0;
 #pragma unroll
@@ -579,56 +585,78 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       if (!ok) break;
+      if (!act) continue;
       const long long ld = g.ksplit > 1 ? g.N : g.ldc;
-      double* base = g.ksplit > 1 ? g.part + (t / g.tiles) * g.M * g.N : g.C;
+      double* base = g.ksplit > 1 ? g.part + (long long)(t / g.tiles) * g.M * g.N : g.C;
+      // A tile inside the matrix with 16-byte aligned rows needs no checks per store.
+      const bool whole = m0 + TBM <= g.M && n0 + kBN <= g.N && !g.lower && !g.added &&
+                         !(ld & 1) && !((uintptr_t)base & 15);
 #pragma unroll
       for (int b = 0; b < 2; b++) {          // 8 columns at a time through shared memory
-        const int sw = (lane >> 1) & 7;
-        unsigned wide = 0;
+        // Staging: row `lane`, pairs of columns swizzled so that 16-byte accesses spread over
+        // the banks both ways.
+        double2* row = (double2*)stg + lane * 4;
+        const int sw = (lane >> 1) & 3;
+        bool wide = false;
 #pragma unroll
-        for (int q = 0; q < 8; q++)
-          stg[lane * 8 + (q ^ sw)] = to_double<false>(w0[8 * b + q], w1[8 * b + q], w2[8 * b + q],
-                                                      ea + seb[8 * b + q], wide);
+        for (int q = 0; q < 8; q += 2)
+          row[(q >> 1) ^ sw] = make_double2(
+              to_double<false>(w0[8 * b + q], w1[8 * b + q], w2[8 * b + q], ea + seb[8 * b + q],
+                               wide),
+              to_double<false>(w0[8 * b + q + 1], w1[8 * b + q + 1], w2[8 * b + q + 1],
+                               ea + seb[8 * b + q + 1], wide));
         if (__any_sync(0xffffffffu, wide)) {
-          // Rare: a result outside FP64's normal range.
+          // Rare: a result outside FP64's normal range, or below 2^-38 of 2^{eA+eB}.
 #pragma unroll
-          for (int q = 0; q < 8; q++)
-            stg[lane * 8 + (q ^ sw)] = to_double<true>(w0[8 * b + q], w1[8 * b + q], w2[8 * b + q],
-                                                       ea + seb[8 * b + q], wide);
+          for (int q = 0; q < 8; q += 2)
+            row[(q >> 1) ^ sw] = make_double2(
+                to_double<true>(w0[8 * b + q], w1[8 * b + q], w2[8 * b + q], ea + seb[8 * b + q],
+                                wide),
+                to_double<true>(w0[8 * b + q + 1], w1[8 * b + q + 1], w2[8 * b + q + 1],
+                                ea + seb[8 * b + q + 1], wide));
         }
         if (g.square) {                      // (the barriers keep these branches branches: a
           __syncwarp();                      // predicated-off FP64 operation costs its slot)
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            const double v = stg[lane * 8 + (q ^ sw)];
-            stg[lane * 8 + (q ^ sw)] = __dmul_rn(v, v);
+          for (int q = 0; q < 4; q++) {
+            const double2 v = row[q];
+            row[q] = make_double2(__dmul_rn(v.x, v.x), __dmul_rn(v.y, v.y));
           }
         } else if (g.scaled) {
           __syncwarp();
 #pragma unroll
-          for (int q = 0; q < 8; q++) stg[lane * 8 + (q ^ sw)] *= g.alpha;
+          for (int q = 0; q < 4; q++) {
+            const double2 v = row[q];
+            row[q] = make_double2(v.x * g.alpha, v.y * g.alpha);
+          }
         }
         __syncwarp();
         // Eight rows per pass: 4 lanes per row, two adjacent columns per lane.
-        const int c0 = 2 * (lane & 3);
-        const long long n = n0 + col0 + 8 * b + c0;
-        for (int r0 = 0; r0 < 32; r0 += 8) {
-          const int r = r0 + (lane >> 2), x7 = (r >> 1) & 7;
-          const long long mr = m0 + quad * 32 + r;
-          if (mr >= g.M) break;
-          const bool v0 = n < g.N && !(g.lower && n > mr);
-          const bool v1 = n + 1 < g.N && !(g.lower && n + 1 > mr);
-          double x = stg[r * 8 + (c0 ^ x7)], y = stg[r * 8 + ((c0 + 1) ^ x7)];
-          double* dst = base + mr * ld + n;
-          if (g.added) {
-            if (v0) x += g.beta * dst[0];
-            if (v1) y += g.beta * dst[1];
-          }
-          if (v0 && v1 && !((uintptr_t)dst & 15)) {
-            *(double2*)dst = make_double2(x, y);
-          } else {
-            if (v0) dst[0] = x;
-            if (v1) dst[1] = y;
+        const long long n = n0 + col0 + 8 * b + 2 * (lane & 3);
+        const long long r1 = m0 + quad * 32 + (lane >> 2);
+        double* dst = base + r1 * ld + n;
+        const double2* src = (const double2*)stg + (lane >> 2) * 4 + ((lane & 3) ^ ((lane >> 3) & 3));
+        if (whole) {
+#pragma unroll
+          for (int r0 = 0; r0 < 32; r0 += 8) *(double2*)(dst + r0 * ld) = src[r0 * 4];
+        } else {
+          for (int r0 = 0; r0 < 32; r0 += 8) {
+            const long long mr = r1 + r0;
+            if (mr >= g.M) break;
+            const bool v0 = n < g.N && !(g.lower && n > mr);
+            const bool v1 = n + 1 < g.N && !(g.lower && n + 1 > mr);
+            double2 v = src[r0 * 4];
+            double* p = dst + r0 * ld;
+            if (g.added) {
+              if (v0) v.x += g.beta * p[0];
+              if (v1) v.y += g.beta * p[1];
+            }
+            if (v0 && v1 && !((uintptr_t)p & 15)) {
+              *(double2*)p = v;
+            } else {
+              if (v0) p[0] = v.x;
+              if (v1) p[1] = v.y;
+            }
           }
         }
         __syncwarp();   // the staging and the exponents are rewritten
@@ -739,11 +767,16 @@ int digits_product(Ctx* c, const Digits& a, const Digits& b, const GemmArgs& g)
   t.ea = a.e; t.eb = b.e;
   t.C = g.C; t.ldc = g.ldc; t.alpha = g.alpha; t.beta = g.beta;
   t.lower = g.lower_only;
+  t.two8 = 1u << 8;
+  t.two16 = 1u << 16;
   t.error = c->tc64_err;
   t.spin_limit = c->spin_limit;
-  t.mtn = cdiv(g.M, TBM);
-  t.ntn = cdiv(g.N, kBN);
-  t.tiles = g.lower_only ? (t.mtn - 1) * t.mtn + std::min(2 * t.mtn, t.ntn) : t.mtn * t.ntn;
+  t.mtn = (unsigned)cdiv(g.M, TBM);
+  t.ntn = (unsigned)cdiv(g.N, kBN);
+  const long long tiles = g.lower_only
+      ? ((long long)t.mtn - 1) * t.mtn + std::min(2 * t.mtn, t.ntn) : (long long)t.mtn * t.ntn;
+  if (tiles > 1 << 22) return set_error(c, THC_ERR_SHAPE, "dgemm_tc: too many tiles");
+  t.tiles = (unsigned)tiles;
   // Split of K: waves x (k tiles per item + ~3 k tiles' worth of fill and final drain).
   const int kt = t.stages;
   int best = 1;
@@ -751,7 +784,7 @@ int digits_product(Ctx* c, const Digits& a, const Digits& b, const GemmArgs& g)
   for (int z = 1; z <= std::min(kt, 256); z++) {
     const int pk = (int)cdiv(kt, z);
     if ((size_t)z * g.M * g.N * 8 > ((size_t)1 << 30) && z > 1) break;
-    const double w = (double)cdiv(t.tiles * cdiv(kt, pk), sms) * (pk + 3) + (z > 1 ? 2.0 : 0.0);
+    const double w = (double)cdiv(tiles * cdiv(kt, pk), sms) * (pk + 3) + (z > 1 ? 2.0 : 0.0);
     if (z == 1 || w < 0.98 * cost) { cost = w; best = z; }
   }
   t.kt_per = (int)cdiv(kt, best);
@@ -766,7 +799,7 @@ int digits_product(Ctx* c, const Digits& a, const Digits& b, const GemmArgs& g)
   t.added = t.ksplit == 1 && g.beta != 0.0;
   CUtensorMap ma, mb;
   if ((st = digit_map(c, &ma, a, TBM)) || (st = digit_map(c, &mb, b, kBN))) return st;
-  const unsigned grid = (unsigned)std::min<long long>(t.tiles * t.ksplit, sms);
+  const unsigned grid = (unsigned)std::min<long long>(tiles * t.ksplit, sms);
   {
     ProfScope prof(c, "dgemm_tc");
     dgemm_tc_kernel<<<grid, kThreads, kSmem, c->stream>>>(ma, mb, t);
@@ -813,7 +846,9 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
   if (kpan < kp && g.mode == GEMM_SQUARE) return THC_OK;   // the square needs the whole sum
   const size_t abytes = (size_t)mp * kpan * per, bbytes = same ? 0 : (size_t)npan * kpan * per;
   // Coordinates and launch sizes are 32-bit.
-  if (abytes + bbytes > 4 * budget || mp > 0x7fffff00LL || np > 0x7fffff00LL) return THC_OK;
+  if (abytes + bbytes > 4 * budget || mp > 0x7fffff00LL || np > 0x7fffff00LL ||
+      (mp / TBM) * (npan / kBN) > 1 << 22)
+    return THC_OK;
   char* flags = (char*)ws_get(c, WS_T64_E, 256 + sizeof(int) * (mp + npan) +
                                                sizeof(unsigned) * std::max(mp, npan));
   Digits da, db;

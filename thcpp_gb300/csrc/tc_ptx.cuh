@@ -158,23 +158,18 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v)
   for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// The same load in two halves: the registers hold the columns only after tmem_ld_wait, which
-// names them so that no use moves above it.
-__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, float (&v)[8])
+// Eight columns at each of two addresses, in flight together.
+__device__ __forceinline__ void tmem_ld8x2(uint32_t ta, uint32_t tb, float (&a)[8], float (&b)[8])
 {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
-        "=f"(v[7])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait(float (&v)[8])
-{
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
-               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]),
-                 "+f"(v[7])
-               :
-               : "memory");
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]),
+        "=f"(a[7]), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]), "=f"(b[4]), "=f"(b[5]),
+        "=f"(b[6]), "=f"(b[7])
+      : "r"(ta), "r"(tb)
+      : "memory");
 }
 
 inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
