@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -38,11 +39,26 @@ namespace {
 
 constexpr int kQrThreads = 256;
 
+// A candidate pivot: the residual as an integer that orders like it (NaN below everything),
+// because an FP64 comparison holds a quarter of an SM's pipe for 64 clocks, and its point.
 struct QrPiv {
-  double v;
+  long long v;
   int a;
   int pad;
 };
+
+__device__ __forceinline__ long long order_key(double x)
+{
+  const long long b = __double_as_longlong(x);
+  if ((b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL) return LLONG_MIN;
+  return b < 0 ? b ^ 0x7fffffffffffffffLL : b;
+}
+__device__ __forceinline__ double key_value(long long k)
+{
+  if (k == LLONG_MIN) return __longlong_as_double(0x7ff8000000000000LL);
+  return __longlong_as_double(k < 0 ? k ^ 0x7fffffffffffffffLL : k);
+}
+constexpr long long kNone = LLONG_MIN;       // no candidate (or only NaN)
 
 struct QrGeom {
   const double* phi;     // N_o x N_g (transposed: a warp reads consecutive points)
@@ -73,28 +89,28 @@ __global__ void transpose_rows(const double* __restrict__ src, long long n, int 
   }
 }
 
-__device__ __forceinline__ bool piv_better(double v, int a, double w, int b)
+__device__ __forceinline__ bool piv_better(long long v, int a, long long w, int b)
 {
   return v > w || (v == w && a < b);
 }
 
 // Block argmax (largest value, lowest index) of (v, a); the result is valid in thread 0.
-__device__ QrPiv block_argmax(double v, int a)
+__device__ QrPiv block_argmax(long long v, int a)
 {
   __shared__ QrPiv red[kQrThreads / 32];
   for (int o = 16; o; o >>= 1) {
-    double w = __shfl_down_sync(0xffffffffu, v, o);
+    long long w = __shfl_down_sync(0xffffffffu, v, o);
     int b = __shfl_down_sync(0xffffffffu, a, o);
     if (piv_better(w, b, v, a)) { v = w; a = b; }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) red[warp] = QrPiv{v, a, 0};
   __syncthreads();
-  QrPiv r{-INFINITY, 0x7fffffff, 0};
+  QrPiv r{kNone, 0x7fffffff, 0};
   if (warp == 0) {
     if (lane < kQrThreads / 32) r = red[lane];
     for (int o = 16; o; o >>= 1) {
-      double w = __shfl_down_sync(0xffffffffu, r.v, o);
+      long long w = __shfl_down_sync(0xffffffffu, r.v, o);
       int b = __shfl_down_sync(0xffffffffu, r.a, o);
       if (piv_better(w, b, r.v, r.a)) { r.v = w; r.a = b; }
     }
@@ -103,9 +119,10 @@ __device__ QrPiv block_argmax(double v, int a)
 }
 
 // Publishes the block's candidate; the last block to finish reduces all of them into
-// piv[k] / dpiv[k] and re-arms the ticket for the next launch.
+// piv[k] / dpiv[k] and the reciprocal root of the residual rpiv[k], and re-arms the ticket for
+// the next launch.
 __device__ void finish_argmax(QrPiv mine, QrPiv* blk, unsigned* ticket, int* piv,
-                              double* dpiv, int k)
+                              double* dpiv, double* rpiv, int k)
 {
   __shared__ bool last;
   if (threadIdx.x == 0) {
@@ -116,17 +133,19 @@ __device__ void finish_argmax(QrPiv mine, QrPiv* blk, unsigned* ticket, int* piv
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double v = -INFINITY;
+  long long v = kNone;
   int a = 0x7fffffff;
   for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-    double w = __ldcg(&blk[b].v);
+    long long w = __ldcg(&blk[b].v);
     int i = __ldcg(&blk[b].a);
     if (piv_better(w, i, v, a)) { v = w; a = i; }
   }
   QrPiv r = block_argmax(v, a);
   if (threadIdx.x == 0) {
     piv[k] = r.a;
-    dpiv[k] = r.v;
+    const double d = key_value(r.v);
+    dpiv[k] = d;
+    rpiv[k] = d > 0.0 ? 1.0 / sqrt(d) : 0.0;
     *ticket = 0u;
   }
 }
@@ -166,24 +185,29 @@ __device__ __forceinline__ double gram(const QrGeom& g, long long a, const doubl
 
 // d(a) = G(a, a) and the first pivot.
 __global__ void __launch_bounds__(kQrThreads)
-qrcp_init_kernel(QrGeom g, double* d, QrPiv* blk, unsigned* ticket, int* piv, double* dpiv)
+qrcp_init_kernel(QrGeom g, double* d, QrPiv* blk, unsigned* ticket, int* piv, double* dpiv,
+                 double* rpiv)
 {
   const long long a = blockIdx.x * (long long)g.ppb + threadIdx.x;
   const bool own = threadIdx.x < g.ppb && a < g.ng;
-  double v = -INFINITY;
+  long long v = kNone;
   if (own) {
-    v = gram(g, a, g.phi + a, g.occ ? g.occ + a : nullptr, g.ng);
-    d[a] = v;
+    const double x = gram(g, a, g.phi + a, g.occ ? g.occ + a : nullptr, g.ng);
+    d[a] = x;
+    v = order_key(x);
   }
-  QrPiv r = block_argmax(v, own ? (int)a : 0x7fffffff);
-  finish_argmax(r, blk, ticket, piv, dpiv, 0);
+  QrPiv r = block_argmax(v, v != kNone ? (int)a : 0x7fffffff);
+  finish_argmax(r, blk, ticket, piv, dpiv, rpiv, 0);
 }
 
-// Step k: column k of L, the residual update and the next pivot.  L is column-major
+// Step k: column k of L, the residual update and the next pivot.  Bound by the FP64 pipe: N_o + k
+// FMAs a point and little else in FP64 -- the reciprocal root of the pivot's residual is taken
+// once (a root and a division a point were 50 operations next to 160), candidates compare as
+// integers.  L is column-major
 // (L[j * N_g + a]); a picked point has d = -inf and L(a, k) = 0 after its own step.
-__global__ void __launch_bounds__(kQrThreads)
+__global__ void __launch_bounds__(kQrThreads, 3)   // three blocks an SM: registers for the loads
 qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k, int npts,
-                 QrPiv* blk, unsigned* ticket, int* piv, double* dpiv)
+                 QrPiv* blk, unsigned* ticket, int* piv, double* dpiv, double* rpiv)
 {
   extern __shared__ double sh[];
   const int kw = g.cplx ? 2 * g.no : g.no;
@@ -191,7 +215,7 @@ qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k
   double* op = pp + kw;
   double* lp = op + g.nocc;
   const int p = piv[k];
-  const double dp = dpiv[k];
+  const double rp = rpiv[k];           // 0 where the residual is not positive
   const long long ng = g.ng;
   if (p < 0 || p >= ng) {
     // No valid pivot (every candidate residual was NaN): pass the marker on without
@@ -199,6 +223,7 @@ qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k
     if (k + 1 < npts && blockIdx.x == 0 && threadIdx.x == 0) {
       piv[k + 1] = p;
       dpiv[k + 1] = -INFINITY;
+      rpiv[k + 1] = 0.0;
     }
     return;
   }
@@ -210,31 +235,31 @@ qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k
   __syncthreads();
   const long long a = blockIdx.x * (long long)g.ppb + threadIdx.x;
   const bool own = threadIdx.x < g.ppb && a < ng;
-  double best = -INFINITY;
+  long long best = kNone;
   if (own) {
     double dv = d[a];
     double l = 0.0;
     if (a == p) {
-      l = sqrt(fmax(dp, 0.0));
+      l = sqrt(fmax(dpiv[k], 0.0));
       dv = -INFINITY;
-    } else if (dv != -INFINITY && dp > 0.0) {
+    } else if (__double_as_longlong(dv) != (long long)0xfff0000000000000ULL &&
+               __double_as_longlong(rp) != 0) {
       const double gap = gram(g, a, pp, op, 1);
       double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
       const double* la = L + a;
       int j = 0;
-      for (; j + 8 <= k; j += 8) {
-        // Eight loads in flight before the four FMA chains consume them.
-        double x[8];
+      for (; j + 16 <= k; j += 16) {
+        // Sixteen loads in flight before the four FMA chains consume them.
+        double x[16];
 #pragma unroll
-        for (int u = 0; u < 8; u++) x[u] = la[(j + u) * ng];
-        s0 = fma(x[0], lp[j + 0], s0);
-        s1 = fma(x[1], lp[j + 1], s1);
-        s2 = fma(x[2], lp[j + 2], s2);
-        s3 = fma(x[3], lp[j + 3], s3);
-        s0 = fma(x[4], lp[j + 4], s0);
-        s1 = fma(x[5], lp[j + 5], s1);
-        s2 = fma(x[6], lp[j + 6], s2);
-        s3 = fma(x[7], lp[j + 7], s3);
+        for (int u = 0; u < 16; u++) x[u] = la[(j + u) * ng];
+#pragma unroll
+        for (int u = 0; u < 16; u += 4) {
+          s0 = fma(x[u + 0], lp[j + u + 0], s0);
+          s1 = fma(x[u + 1], lp[j + u + 1], s1);
+          s2 = fma(x[u + 2], lp[j + u + 2], s2);
+          s3 = fma(x[u + 3], lp[j + u + 3], s3);
+        }
       }
       for (; j + 4 <= k; j += 4) {
         s0 = fma(la[(j + 0) * ng], lp[j + 0], s0);
@@ -243,16 +268,16 @@ qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k
         s3 = fma(la[(j + 3) * ng], lp[j + 3], s3);
       }
       for (; j < k; j++) s0 = fma(la[j * ng], lp[j], s0);
-      l = (gap - ((s0 + s1) + (s2 + s3))) / sqrt(dp);
+      l = (gap - ((s0 + s1) + (s2 + s3))) * rp;
       dv = fma(-l, l, dv);
     }
     L[(long long)k * ng + a] = l;
     d[a] = dv;
-    best = dv;
+    best = order_key(dv);
   }
   if (k + 1 >= npts) return;
-  QrPiv r = block_argmax(best, own ? (int)a : 0x7fffffff);
-  finish_argmax(r, blk, ticket, piv, dpiv, k + 1);
+  QrPiv r = block_argmax(best, best != kNone ? (int)a : 0x7fffffff);
+  finish_argmax(r, blk, ticket, piv, dpiv, rpiv, k + 1);
 }
 
 }  // namespace
@@ -293,7 +318,7 @@ int qrcp_run(Ctx* c, const double* phi_in, long long ng, int no, const double* o
   const size_t l_bytes = sizeof(double) * (size_t)npts * ng;
   const size_t t_bytes = sizeof(double) * (size_t)(kw + nt) * ng;
   const size_t bytes = l_bytes + t_bytes + sizeof(double) * ng + sizeof(QrPiv) * nblk +
-                       (sizeof(int) + sizeof(double)) * npts + 1024;
+                       (sizeof(int) + 2 * sizeof(double)) * npts + 1024;
   char* base = (char*)ws_get(c, WS_ZT, bytes);
   if (!base) return set_error(c, THC_ERR_NOMEM, "thc_qrcp: workspace allocation failed");
   double* L = (double*)base;
@@ -302,7 +327,8 @@ int qrcp_run(Ctx* c, const double* phi_in, long long ng, int no, const double* o
   double* d = occt + (size_t)nt * ng;
   QrPiv* blk = (QrPiv*)(d + ng);
   double* dpiv = (double*)(blk + nblk);
-  int* piv = (int*)(dpiv + npts);
+  double* rpiv = dpiv + npts;
+  int* piv = (int*)(rpiv + npts);
   unsigned* ticket = (unsigned*)(((uintptr_t)(piv + npts) + 255) & ~(uintptr_t)255);
   QrGeom g;
   g.phi = phit;
@@ -325,7 +351,7 @@ int qrcp_run(Ctx* c, const double* phi_in, long long ng, int no, const double* o
     if (occ)
       transpose_rows<<<dim3((unsigned)cdiv(ng, 32), (unsigned)cdiv(nt, 32)), tb, 0, s>>>(
           occ, ng, nt, occt);
-    qrcp_init_kernel<<<(unsigned)nblk, kQrThreads, 0, s>>>(g, d, blk, ticket, piv, dpiv);
+    qrcp_init_kernel<<<(unsigned)nblk, kQrThreads, 0, s>>>(g, d, blk, ticket, piv, dpiv, rpiv);
   }
   c->launches += occ ? 2 : 1;  // the transposes
   THC_LAUNCHED(c, "qrcp_init");
@@ -333,7 +359,7 @@ int qrcp_run(Ctx* c, const double* phi_in, long long ng, int no, const double* o
     ProfScope ps(c, "qrcp_step");
     for (int k = 0; k < npts; k++) {
       qrcp_step_kernel<<<(unsigned)nblk, kQrThreads, shmem, s>>>(g, L, d, k, npts, blk, ticket,
-                                                                 piv, dpiv);
+                                                                 piv, dpiv, rpiv);
     }
   }
   c->launches += npts - 1;
