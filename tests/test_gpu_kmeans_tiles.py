@@ -48,3 +48,28 @@ def test_kmeans_tile_edges(request, prec, ng, nmu, kind):
         assert st.iterations == ref.iters and st.final_diff == ref.diff
         diff, pct = ctx.kmeans_history(ref.iters)
         assert np.array_equal(pct, ref.pct)
+
+
+@pytest.mark.parametrize("ng,nmu,clump", [
+    (2048, 8, 0.0), (2500, 8, 0.9), (7500, 9, 0.95),     # members around a block's windows
+    (70000, 80, 0.0), (140000, 140, 0.5),                # index ranges over 65,536
+    (150000, 150, 0.98),                                 # a cluster over more than 512 tiles
+    (7168, 8, 0.0), (7169, 8, 0.0),                      # mean members at the rules' two sides
+    (2560, 8, 0.0), (2561, 8, 0.0)])
+def test_kmeans_cluster_stretches(gpu_ctx_fp64, ng, nmu, clump):
+    """Clusters at and over the buffers of the one-kernel sums: members, index range, tiles."""
+    r = np.random.default_rng(ng)
+    g = r.uniform(-1.0, 1.0, size=(ng, 3))
+    near = r.random(ng) < clump
+    g[near] = 0.9 + 0.01 * g[near]
+    init = np.sort(r.choice(np.flatnonzero(~near), nmu, replace=False)).astype(np.int32)
+    g = np.ascontiguousarray(g)
+    rho = r.uniform(0.5, 2.0, size=ng)
+    ref = oracle.kmeans(g, rho, nmu, init, 4, 1e-9)
+    idx, st, status = gpu_ctx_fp64.kmeans(g, rho, nmu, init, 4, 1e-9, raise_on_error=False)
+    assert status == {0: capi.THC_OK, 2: capi.THC_ERR_EMPTY_CLUSTER}[ref.status]
+    if status == 0:
+        assert np.array_equal(idx, ref.idx)
+        assert st.iterations == ref.iters and st.final_diff == ref.diff
+        diff, pct = gpu_ctx_fp64.kmeans_history(ref.iters)
+        assert np.array_equal(pct, ref.pct)

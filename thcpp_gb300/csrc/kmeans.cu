@@ -23,9 +23,10 @@
 //     a candidate replaces the best only if its sqrt is strictly smaller, which keeps the
 //     first index among equal sqrt values exactly as std::min_element does;
 //   * per-cluster sums run in ascending grid order through a stable counting sort of
-//     the labels (block histograms -> per-cluster scans -> stable warp scatter), then
-//     each cluster's members are accumulated in that order by warp_seqsum, which
-//     reproduces the sequential loop's rounding exactly (seqsum.cuh);
+//     the labels (block histograms -> per-cluster scans -> stable warp scatter, or a
+//     bitmap per cluster, km_cluster), then each cluster's members are accumulated in
+//     that order by segment walks, which reproduce the sequential loop's rounding
+//     exactly (segsum.cuh, seqsum.cuh);
 //   * the normed difference that is reported is the sequential sum in index order (again
 //     warp_seqsum); the per-iteration convergence test uses a fixed-order approximation
 //     and falls back to the exact sum whenever the two could decide differently.
@@ -68,6 +69,7 @@ struct KmState {
   double diff;
   double pct;
   double threshold;
+  double thr2_lo, thr2_hi;   // squares between these are compared exactly (within 1.5e-10 of it)
   double abound;        // |a| bound of the FP32 error estimate
   unsigned long long absmax[3];
   int bad_label;
@@ -80,6 +82,7 @@ struct KmState {
   int diff_exact;                        // st->diff came from the sequential sum
   int ticket;                            // blocks of km_sums finished this iteration
   int nwin;                              // windows of the exact sums this iteration
+  int listed;                            // members listed by km_cluster this iteration
 };
 
 // One window of <= kSegWin consecutive terms of one cluster in the sorted term arrays.
@@ -114,6 +117,11 @@ struct KmBufs {
   int nbins_max;
   float* pf;       // [3][ng] FP32 coordinates in the binned order (pf[d][t] of point perm[t])
   float* box;      // [tiles][6] bounding boxes of its 256-point tiles (min x, y, z, max x, y, z)
+  // Sums by cluster (km_cluster; null: by the counting sort): which tiles hold a member, a bit
+  // per tile, nwt words a cluster.  Labels are then in the binned order.
+  unsigned* mask;
+  int nwt;
+  int pad6;
   // Window-parallel exact sums (nwin_max == 0: the one-kernel km_sums path).
   const double* tq;   // [4][ng] rho_i, rho_i x_i, rho_i y_i, rho_i z_i in point order
   double* sv;         // [4][ng] the same terms in sorted (cluster, ascending point) order
@@ -374,6 +382,7 @@ constexpr int kPruneMax = 1024;   // candidate centroids kept in shared memory p
 // and warp this part cannot afford (17 points a thread and 48 centroids took 52 us).  The test
 // itself is FP32 too, its terms raised by 1e-5 to cover its rounding: in FP64 its two roots
 // cost more than the scan (9 of 21 us at N_g 110592, N_mu 256).
+template <bool BY_TILE>
 __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
 {
   KmState* st = b.st;
@@ -462,9 +471,9 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
   __syncthreads();
   bool amb = false;
   unsigned changed = 0;
+  int k1 = 0;                // this point's label
   if (valid) {
     float m1 = INFINITY, m2 = INFINITY;
-    int k1 = 0;
     if (nc <= kPruneMax) {
       for (int j = 0; j < nc; j++) {
         float dx = ccx[j] - g[0], dy = ccy[j] - g[1], dz = ccz[j] - g[2];
@@ -485,8 +494,7 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
     const float a = (float)st->abound * 1.00001f;
     const float e = 1.1920929e-07f * 1.00001f *
                     (2.f * a * (sqrtf(m1) + sqrtf(m2)) + 5.00001f * (m1 + m2));
-    if ((m2 - m1) * 0.99999f > e + 1e-30f) put_label(b, it, i, k1, changed);
-    else amb = true;
+    amb = !((m2 - m1) * 0.99999f > e + 1e-30f);
   }
   // FP64 rescue of the near ties, at once and by the whole warp, one point at a time: the
   // exact first argmin of the sqrt distances (as km_recheck) over the tile's candidates in
@@ -517,7 +525,20 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
       int k2 = __shfl_xor_sync(0xffffffffu, am.k, off);
       am.merge(s2, m2, k2);
     }
-    if (lane == 0) put_label(b, it, ip, am.k, changed);
+    const int k = __shfl_sync(0xffffffffu, am.k, 0);
+    if (lane == p) k1 = k;
+  }
+  if (BY_TILE) {
+    // In the binned order, with a bit for the tile in each of its clusters' masks.
+    if (valid) {
+      b.labels[(size_t)(it & 1) * b.ng + t] = k1;
+      if (it > 0 && b.labels[(size_t)((it + 1) & 1) * b.ng + t] != k1) changed = 1;
+    }
+    const unsigned peers = __match_any_sync(0xffffffffu, valid ? k1 : -1);
+    if (valid && lane == __ffs(peers) - 1)
+      atomicOr(&b.mask[(size_t)k1 * b.nwt + (blockIdx.x >> 5)], 1u << (blockIdx.x & 31));
+  } else if (valid) {
+    put_label(b, it, i, k1, changed);
   }
   flush_changed(st, changed);
 }
@@ -872,23 +893,6 @@ __device__ __forceinline__ double block_max(double v, double* red)
   return red[0];
 }
 
-// Fixed-order block sum (deterministic; not the reference's rounding).
-__device__ __forceinline__ double block_sum(double v, double* red)
-{
-  for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-    red[0] = t;
-  }
-  __syncthreads();
-  return red[0];
-}
-
 // The terms ((a_i - c_i) / scale)^2 of the reference's normed difference in its index order
 // i = 3k + d (centroid k, coordinate d), written to `terms`; returns scale.  Whole block.
 __device__ double normdiff_terms(const KmBufs& b, const double* a, const double* c,
@@ -912,12 +916,39 @@ __device__ double normdiff_terms(const KmBufs& b, const double* a, const double*
   return scale;
 }
 
+// Exponent field of x >= 0, 0x7ff and above for what is not finite or negative.
+__device__ __forceinline__ int biased_exponent(double x)
+{
+  return (int)((unsigned long long)__double_as_longlong(x) >> 52);
+}
+
+// The reference's normed difference of iteration `it` by the whole block.
+__device__ __noinline__ double normdiff_block(const KmBufs& b, int it, double* red, double* res)
+{
+  const double* a = b.cen + (size_t)((it + 1) & 1) * 3 * b.nmu;
+  const double* c = b.cen + (size_t)(it & 1) * 3 * b.nmu;
+  const double scale = normdiff_terms(b, a, c, b.terms, red);
+  if (threadIdx.x < 32) {
+    const double ssum = warp_seqsum(0.0, b.terms, 3 * b.nmu);
+    if (threadIdx.x == 0) res[0] = __dmul_rn(scale, __dsqrt_rn(ssum));
+  }
+  __syncthreads();
+  return res[0];
+}
+
+// This iteration's centroid coordinate of cluster k for threads 0..2: what sums_finish moves.
+__device__ __forceinline__ double old_coordinate(const KmBufs& b, int k, int it)
+{
+  return threadIdx.x < 3 ? b.cen[((size_t)(it & 1) * 3 + threadIdx.x) * b.nmu + k] : 0.0;
+}
+
 // End of an iteration's sums for cluster k (whole block; res[0..3] = w, x, y, z sums): the
 // new centroid, its squared move, and -- in the last block to finish, found by a ticket in
 // the state -- the convergence decision: the normed difference approximated by a
 // fixed-order sum of squared centroid moves (relative deviation from the reference's value
 // below (3 N_mu + 8) u), evaluated exactly when within 1e-10 of the threshold.
-__device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double* red, int& last)
+__device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double* red, int& last,
+                            double old)
 {
   KmState* st = b.st;
   const int nmu = b.nmu;
@@ -927,12 +958,10 @@ __device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double*
     const int d = threadIdx.x;
     double* nc = b.cen + (size_t)((it + 1) & 1) * 3 * nmu;
     float* nc32 = b.cen32 + (size_t)((it + 1) & 1) * 3 * nmu;
-    const double* oc = b.cen + (size_t)(it & 1) * 3 * nmu;
     const double v = __ddiv_rn(res[1 + d], res[0]);
     nc[d * nmu + k] = v;
     nc32[d * nmu + k] = (float)v;
-    red[d] = __dsub_rn(v, oc[d * nmu + k]);
-    __threadfence();
+    red[d] = __dsub_rn(v, old);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -946,46 +975,71 @@ __device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double*
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // ---- last block: the convergence decision and the state update of this iteration ----
-  if (*(volatile int*)&st->empty || *(volatile int*)&st->bad_label) {
+  // ---- last block: the convergence decision and the state update of this iteration, on the
+  //      square of the normed difference: the sum of the moves' squares in integers, a warp's
+  //      relative to its largest (truncated 2^-51 of it each), because an FP64 instruction
+  //      holds its warp 64 clocks and every warp's five sum steps, the root and the division of
+  //      the percentage took 6,000 (3 of ~24 us an iteration at N_mu 256).  The roots and the
+  //      percentages of the log are km_normdiff_exact's.  The block's warps are a power of two.
+  __shared__ int exps[32];
+  const double x0 = threadIdx.x < nmu ? __ldcg(part + threadIdx.x) : 0.0;
+  int em = biased_exponent(x0);
+#pragma unroll 1
+  for (int i = threadIdx.x + blockDim.x; i < nmu; i += blockDim.x)
+    em = max(em, biased_exponent(__ldcg(part + i)));
+  const int bad = *(volatile int*)&st->empty | *(volatile int*)&st->bad_label;
+  const double lo = st->thr2_lo, hi = st->thr2_hi;
+  em = __reduce_max_sync(0xffffffffu, em);
+  long long su = 0;
+  if (em < 0x7ff) {
+    su = seg_units(x0, em);
+#pragma unroll 1
+    for (int i = threadIdx.x + blockDim.x; i < nmu; i += blockDim.x)
+      su += seg_units(__ldcg(part + i), em);
+#pragma unroll 1
+    for (int off = 16; off; off >>= 1) su += __shfl_xor_sync(0xffffffffu, su, off);
+  }
+  if (lane == 0) {
+    red[warp] = __longlong_as_double(su);
+    exps[warp] = em;
+  }
+  __syncthreads();
+  if (bad) {
     if (threadIdx.x == 0) { st->done = 1; st->iter = it + 1; st->ticket = 0; }
     return;
   }
-  double v = 0.0;
-  for (int i = threadIdx.x; i < nmu; i += blockDim.x) v += __ldcg(part + i);
-  const double approx = sqrt(block_sum(v, red));
-  const double thr = st->threshold;
-  const bool exact = fabs(approx - thr) <= 1e-10 * thr;
-  double diff = approx;
-  if (exact) {
-    const double* a = b.cen + (size_t)((it + 1) & 1) * 3 * nmu;
-    const double* c = b.cen + (size_t)(it & 1) * 3 * nmu;
-    double scale = normdiff_terms(b, a, c, b.terms, red);
-    if (warp == 0) {
-      double ssum = warp_seqsum(0.0, b.terms, 3 * nmu);
-      if (lane == 0) res[0] = __dmul_rn(scale, __dsqrt_rn(ssum));
-    }
-    __syncthreads();
-    diff = res[0];
+  if (warp == 0) {
+    const int e = lane < (int)(blockDim.x >> 5) ? exps[lane] : 0;
+    // S 2^(e - 1073); zero below 2^-970, NaN for what is not finite: both are decided exactly.
+    const double unit = e >= 0x7ff ? CUDART_NAN : e > 50 ? __longlong_as_double((long long)(e - 50) << 52) : 0.0;
+    double v = e ? __dmul_rn((double)__double_as_longlong(red[lane]), unit) : 0.0;
+#pragma unroll 1
+    for (int off = (int)(blockDim.x >> 6); off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if (lane == 0) res[3] = v;
   }
+  __syncthreads();
+  const double sum = res[3], thr = st->threshold;
+  const bool exact = (!(sum < lo) && !(sum > hi)) || sum < 1e-280;
+  double diff = 0.0;
+  if (exact) diff = normdiff_block(b, it, red, res);
   if (threadIdx.x == 0) {
     st->diff_exact = exact;
-    st->diff = diff;
-    st->pct = 100.0 * (double)st->changed / (double)b.ng;
-    b.log[it] = diff;
-    b.log[st->max_it + it] = st->pct;
+    // The difference itself under a sign bit, or the sum of squares; the changed labels' count.
+    b.log[it] = exact ? __longlong_as_double(__double_as_longlong(diff) | (1LL << 63)) : sum;
+    b.log[st->max_it + it] = __longlong_as_double((long long)st->changed);
     st->changed = 0;
     st->rechecked_total += st->recheck_n;
     st->recheck_n = 0;
     st->final_buf = (it + 1) & 1;
-    if (diff < thr) {
+    if (exact ? diff < thr : sum < lo) {
       st->converged = 1;
       st->done = 1;
     } else if (it + 1 >= st->max_it) {
       st->done = 1;
-      st->zero_fill = !(diff > thr);
+      st->zero_fill = exact ? !(diff > thr) : 0;
     }
     st->ticket = 0;
+    st->listed = 0;
     st->iter = it + 1;
   }
 }
@@ -1028,6 +1082,7 @@ __global__ void __launch_bounds__(kSumThreads) km_sums(KmBufs b)
   const int tq = warp / kSumWins, tw = warp % kSumWins;   // this warp's window task
   const int k = blockIdx.x;
   const int s = b.start[k], n = b.total[k];
+  const double old = old_coordinate(b, k, it);
   if (threadIdx.x < 4) sm.acc[threadIdx.x] = 0.0;
   for (int base = 0; base < n; base += kSumCap) {
     const int cnt = min(kSumCap, n - base);
@@ -1086,7 +1141,311 @@ __global__ void __launch_bounds__(kSumThreads) km_sums(KmBufs b)
   __syncthreads();
   if (threadIdx.x < 4) res[threadIdx.x] = sm.acc[threadIdx.x];
   __syncthreads();
-  sums_finish(b, k, it, res, red, last);
+  sums_finish(b, k, it, res, red, last, old);
+}
+
+// A whole iteration's sums in one kernel: a block per cluster collects its members from the
+// tiles that hold one, puts their terms in ascending grid order, and sums them as km_sums does.
+// The order comes from a bitmap over the members' index range (a counting sort with one bit per
+// key): a member's place is the number of bits below its own.  With the assign this makes two
+// kernels an iteration instead of five, and no pass over all points beside the assign's: block
+// counts, their scan, the scatter and the window tables took 27 of 45 us at N_g 110592, N_mu 256
+// (now ~20 of 32; at N_g 4320, N_mu 48 ~10 of 18 instead of ~50).
+// What bounds it is the latency of its dozen dependent steps.  A cluster of more members than
+// NWIN windows hold, or over a wider index range than the bitmap's, is put in order through a
+// list in global memory, stretch by stretch of the bitmap, and summed NWIN windows at a time.
+constexpr int kBmWords = 2048;             // bitmap: 65,536 grid indices
+constexpr long long kClusterMax = 896;     // mean members per cluster
+constexpr int kTileList = 256;             // tiles of a cluster (more: every tile is scanned)
+constexpr int kClPer = 4, kClWin = 32 * kClPer;   // terms a lane and a window
+template <int NW, int NWIN>
+struct ClusterSmem {
+  double sv[4][kClWin * NWIN];
+  union {
+    struct {
+      unsigned bits[kBmWords];
+      unsigned short pre[kBmWords];        // members below a word (at most 65,535)
+      int memb[kClWin * NWIN];
+    };
+    SegChunk<NWIN> sc[4];
+  };
+  int tiles[kTileList];
+  double acc[4], red[32];
+  int wtot[32], bad[4];
+  int n, imin, imax, ntl, total, last, off;
+};
+template <int NW, int NWIN>
+__global__ void __launch_bounds__(128 * NW, 1024 / (128 * NW)) km_cluster(KmBufs b)
+{
+  constexpr int T = 128 * NW, CH = kClWin * NWIN;
+  static_assert(CH <= 1024, "seg_units");
+  KmState* st = b.st;
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  ClusterSmem<NW, NWIN>& sm = *reinterpret_cast<ClusterSmem<NW, NWIN>*>(cl_smem);
+  const int done = st->done, it = st->iter;
+  const int k = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // This warp's quantity and first window.
+  const int tq = warp & 3, tw = warp >> 2;
+  unsigned* mk = b.mask + (size_t)k * b.nwt;
+  unsigned word = lane < b.nwt ? mk[lane] : 0u;
+  if (done) return;
+  const int* lab = b.labels + (size_t)(it & 1) * b.ng;
+  const double old = old_coordinate(b, k, it);
+  if (warp == 0) {
+    // The tiles, and the mask cleared for the next iteration.
+    int cnt = 0;
+#pragma unroll 1
+    for (int w0 = 0; w0 < b.nwt; w0 += 32) {
+      const int w = w0 + lane;
+      if (w0) word = w < b.nwt ? mk[w] : 0u;
+      if (word) mk[w] = 0u;
+      const int pc = __popc(word);
+      int x = pc;
+#pragma unroll 1
+      for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+      }
+      int pos = cnt + x - pc;
+#pragma unroll 1
+      for (; word; word &= word - 1, pos++)
+        if (pos < kTileList) sm.tiles[pos] = w * 32 + __ffs(word) - 1;
+      cnt += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) {
+      sm.ntl = cnt;
+      sm.n = 0;
+      sm.imin = 0x7fffffff;
+      sm.imax = -1;
+    }
+  } else {
+#pragma unroll 1
+    for (int w = tid - 32; w < kBmWords; w += T - 32) sm.bits[w] = 0u;
+    if (tid < 36) sm.acc[tid - 32] = 0.0;
+  }
+  __syncthreads();
+  const bool every = sm.ntl > kTileList;
+  const int items = (every ? (int)((b.ng + 255) >> 8) : sm.ntl) << 8;
+  // f(grid index, or -1) for four points of the tiles at a time, their loads in flight together;
+  // all lanes of a warp call it together.
+  auto scan = [&](auto f) {
+#pragma unroll 1
+    for (int e0 = 0; e0 < items; e0 += 4 * T) {
+      int l[4], i[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int e = e0 + q * T + tid;
+        const long long t = e < items
+            ? ((long long)(every ? e >> 8 : sm.tiles[e >> 8]) << 8) + (e & 255) : b.ng;
+        l[q] = t < b.ng ? lab[t] : -1;
+        i[q] = t < b.ng ? b.perm[t] : -1;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (l[q] != k) i[q] = -1;
+      f(i);
+    }
+  };
+  {
+    int mn = 0x7fffffff, mx = -1;
+    scan([&](const int (&i)[4]) {
+      unsigned m[4];
+      int c = 0;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        m[q] = __ballot_sync(0xffffffffu, i[q] >= 0);
+        c += __popc(m[q]);
+      }
+      if (c == 0) return;
+      int s = 0;
+      if (lane == 0) s = atomicAdd(&sm.n, c);
+      s = __shfl_sync(0xffffffffu, s, 0);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (i[q] >= 0) {
+          const int p = s + __popc(m[q] & ((1u << lane) - 1u));
+          if (p < CH) sm.memb[p] = i[q];
+          mn = min(mn, i[q]);
+          mx = max(mx, i[q]);
+        }
+        s += __popc(m[q]);
+      }
+    });
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0 && mx >= 0) {
+      atomicMin(&sm.imin, mn);
+      atomicMax(&sm.imax, mx);
+    }
+  }
+  __syncthreads();
+  const int n = sm.n, imin = sm.imin, imax = sm.imax;
+  // The four terms of grid point i.
+  auto terms = [&](int i, double (&x)[4]) {
+    if (b.tq) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) x[q] = __ldg(b.tq + (size_t)q * b.ng + i);
+    } else {
+      x[0] = b.rho[i];
+      x[1] = __dmul_rn(x[0], b.gx[i]);
+      x[2] = __dmul_rn(x[0], b.gy[i]);
+      x[3] = __dmul_rn(x[0], b.gz[i]);
+    }
+  };
+  // pre[] and total from the bitmap's first `words` words; a barrier on both sides.
+  auto count = [&](int words) {
+    const int per = (words + T - 1) / T, w0 = min(words, tid * per), w1 = min(words, w0 + per);
+    int s = 0;
+#pragma unroll 1
+    for (int w = w0; w < w1; w++) s += __popc(sm.bits[w]);
+    int x = s;
+#pragma unroll 1
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, off);
+      if (lane >= off) x += y;
+    }
+    if (lane == 31) sm.wtot[warp] = x;
+    __syncthreads();
+    int r = __reduce_add_sync(0xffffffffu, lane < warp ? sm.wtot[lane] : 0) + x - s;
+    if (tid == T - 1) sm.total = r + s;
+#pragma unroll 1
+    for (int w = w0; w < w1; w++) {
+      sm.pre[w] = (unsigned short)r;
+      r += __popc(sm.bits[w]);
+    }
+    __syncthreads();
+  };
+  // The running sums over the cc terms in sv: every window's table, then the walk.
+  auto chunk = [&](int cc) {
+    const int nwin = (cc + kClWin - 1) / kClWin;
+    SegChunk<NWIN>& sc = sm.sc[tq];
+    double t[kClPer];
+    auto load = [&](int w) {
+#pragma unroll
+      for (int u = 0; u < kClPer; u++) {
+        const int i = w * kClWin + lane * kClPer + u;
+        t[u] = i < cc ? sm.sv[tq][i] : 0.0;
+      }
+    };
+    int emax = 0;
+#pragma unroll 1
+    for (int w = tw; w < nwin; w += NW) {
+      load(w);
+      emax = max(emax, seg_emax(t));
+    }
+    if (lane == 0) sc.emax[tw] = emax;
+    __syncthreads();
+    const double acc = sm.acc[tq];
+    emax = (int)((unsigned long long)__double_as_longlong(acc) >> 52);
+#pragma unroll
+    for (int v = 0; v < NW; v++) emax = max(emax, sc.emax[v]);
+    const bool ok = emax > 0 && emax < 0x7ff;
+    if (tw == 0 && lane == 0) sc.usable = ok;
+    long long loc[kClPer], incl = 0;
+    if (ok) {
+#pragma unroll 1
+      for (int w = tw + (nwin - 1 - tw) / NW * NW; w >= tw; w -= NW) {   // the first one last
+        load(w);
+        incl = seg_prefix(t, emax, loc);
+        if (lane == 31) sc.units[w] = incl;
+      }
+    }
+    __syncthreads();
+    if (ok && tw < nwin) {
+      long long base = seg_units(acc, emax);
+#pragma unroll 1
+      for (int v = 0; v < tw; v++) base += sc.units[v];
+#pragma unroll 1
+      for (int w = tw;;) {
+        const int ns = seg_table(t, loc, base + incl - loc[kClPer - 1], emax,
+                                 min(kClWin, cc - w * kClWin), sc.tab[w]);
+        if (lane == 0) sc.nseg[w] = ns;
+        if (w + NW >= nwin) break;
+        for (int v = 0; v < NW; v++) base += sc.units[w + v];
+        w += NW;
+        load(w);
+        incl = seg_prefix(t, emax, loc);
+      }
+    }
+    __syncthreads();
+    if (warp == 0) seg_walk4<NWIN>(sm.acc, sm.bad, nwin, sm.sc);
+    __syncthreads();
+    if (tw == 0 && sm.bad[tq]) {
+      const double a = warp_seqsum(acc, sm.sv[tq], cc);
+      if (lane == 0) sm.acc[tq] = a;
+    }
+    __syncthreads();
+  };
+  // The members at hand (the usual case) go to their places at once; else their order goes to
+  // a run of b.member, stretch by stretch of the bitmap, from a scan each.
+  const bool held = n <= CH && (long long)imax - imin < 32LL * kBmWords;
+  const int* list = nullptr;
+  if (held) {
+    double x[4];               // a thread's first member's, under way while the places are found
+    if (tid < n) terms(sm.memb[tid], x);
+#pragma unroll 1
+    for (int m = tid; m < n; m += T) {
+      const int d = sm.memb[m] - imin;
+      atomicOr(&sm.bits[d >> 5], 1u << (d & 31));
+    }
+    __syncthreads();
+    count(n > 0 ? ((imax - imin) >> 5) + 1 : 0);
+#pragma unroll 1
+    for (int m = tid; m < n; m += T) {
+      const int i = sm.memb[m], d = i - imin;
+      if (m >= T) terms(i, x);
+      const int r = sm.pre[d >> 5] + __popc(sm.bits[d >> 5] & ((1u << (d & 31)) - 1u));
+#pragma unroll
+      for (int q = 0; q < 4; q++) sm.sv[q][r] = x[q];
+    }
+    __syncthreads();
+  } else {
+    if (tid == 0) sm.off = atomicAdd(&st->listed, n);
+    __syncthreads();
+    int* run = b.member + sm.off;
+    list = run;
+#pragma unroll 1
+    for (long long lo = imin; lo <= imax; lo += 32LL * kBmWords) {
+      const int words = (int)min((long long)kBmWords, ((imax - lo) >> 5) + 1);
+#pragma unroll 1
+      for (int w = tid; w < words; w += T) sm.bits[w] = 0u;
+      __syncthreads();
+      scan([&](const int (&i)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const long long d = i[q] - lo;
+          if (i[q] >= 0 && d >= 0 && d < 32LL * words)
+            atomicOr(&sm.bits[d >> 5], 1u << (d & 31));
+        }
+      });
+      __syncthreads();
+      count(words);
+#pragma unroll 1
+      for (int w = tid; w < words; w += T) {
+        int r = sm.pre[w];
+#pragma unroll 1
+        for (unsigned x = sm.bits[w]; x; x &= x - 1) run[r++] = (int)(lo + 32 * w + __ffs(x) - 1);
+      }
+      run += sm.total;
+      __syncthreads();
+    }
+  }
+#pragma unroll 1
+  for (int r0 = 0; r0 < n; r0 += CH) {
+    const int cc = min(CH, n - r0);
+    if (!held) {
+#pragma unroll 1
+      for (int m = tid; m < cc; m += T) {
+        double x[4];
+        terms(list[r0 + m], x);
+#pragma unroll
+        for (int q = 0; q < 4; q++) sm.sv[q][m] = x[q];
+      }
+      __syncthreads();
+    }
+    chunk(cc);
+  }
+  sums_finish(b, k, it, sm.acc, sm.red, sm.last, old);
 }
 
 // Window-parallel exact sums, phase 1: one warp per (window, quantity) builds the window's
@@ -1125,6 +1484,7 @@ __global__ void __launch_bounds__(128) km_swalk(KmBufs b)
   const int k = blockIdx.x, q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w0 = b.wbase[k], w1 = b.wbase[k + 1];
   const double* t = b.sv + (size_t)q * b.ng;
+  const double old = old_coordinate(b, k, it);
   double acc = 0.0;
   if (w0 < w1) {
     // The next window's position and table are loaded while the current one is walked.
@@ -1144,17 +1504,30 @@ __global__ void __launch_bounds__(128) km_swalk(KmBufs b)
   }
   if (lane == 0) res[q] = acc;
   __syncthreads();
-  sums_finish(b, k, it, res, red, last);
+  sums_finish(b, k, it, res, red, last, old);
 }
 
-// The reference's normed difference of the last iteration, exactly (one block).
+// The log's roots and percentages (sums_finish leaves squares and counts), and the reference's
+// normed difference of the last iteration, exactly (one block).
 __global__ void __launch_bounds__(1024) km_normdiff_exact(KmBufs b)
 {
   KmState* st = b.st;
-  if (st->diff_exact || st->empty || st->iter < 1) return;
+  if (st->iter < 1) return;
   __shared__ double red[32];
   __shared__ double out;
   const int it = st->iter - 1;
+  double* pct = b.log + st->max_it;
+  for (int i = threadIdx.x; i <= it; i += blockDim.x) {
+    const double v = b.log[i], p = 100.0 * (double)__double_as_longlong(pct[i]) / (double)b.ng;
+    b.log[i] = __double_as_longlong(v) < 0 ? -v : sqrt(v);
+    pct[i] = p;
+    if (i == it) {
+      st->diff = b.log[i];
+      st->pct = p;
+    }
+  }
+  __syncthreads();
+  if (st->diff_exact || st->empty) return;
   const double* a = b.cen + (size_t)((it + 1) & 1) * 3 * b.nmu;
   const double* c = b.cen + (size_t)(it & 1) * 3 * b.nmu;
   const double scale = normdiff_terms(b, a, c, b.terms, red);
@@ -1464,7 +1837,23 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   b.cen = cen; b.cen32 = cen32; b.labels = labels; b.hist = hist; b.total = tot;
   b.start = tot + nmu; b.member = member; b.terms = terms; b.recheck = recheck;
   b.log = logb; b.st = st;
-  if (!fixed) {
+  const bool prune = c->km_prune && nmu >= 8;
+  // Clusters of kClusterMax members and fewer on average are summed a block each, in one
+  // kernel (km_cluster); above, a block's few windows at a time leave the GPU idle where the
+  // counting sort spreads every window over it.  us an iteration at N_g 110592, counting sort
+  // and km_cluster: mean 216 51.7 and 41.1, 432 46.2 and 37.9, 864 49.6 and 45.5, 1024 77.5 and
+  // 83.1, 2304 135 and 149.
+  const bool by_cluster = prune && ng <= kClusterMax * nmu;
+  if (by_cluster) {
+    b.mask = (unsigned*)hist;              // at most the block counts' size
+    b.nwt = (int)cdiv(cdiv(ng, 256), 32);
+  }
+  if (!fixed && by_cluster) {
+    double* tq = (double*)al.get(WS_KM_SV, sizeof(double) * 4 * ng);
+    if (!tq) return set_error(c, THC_ERR_NOMEM, "thc_kmeans: workspace allocation failed");
+    b.tq = tq;
+  }
+  if (!fixed && !by_cluster) {
     // Window-parallel exact sums (the caller-provided fixed scratch keeps the one-kernel
     // sums, whose footprint is smaller).
     const long long nwin_max = ng / kSegWin + nmu + 1;
@@ -1483,6 +1872,12 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   KmState h{};
   h.max_it = max_it;
   h.threshold = threshold;
+  {
+    const double t2 = threshold * threshold;
+    h.thr2_lo = threshold > 0 && t2 < 1e-270 ? 0.0 : t2 * (1.0 - 3e-10);
+    h.thr2_hi = threshold > 0 && t2 < 1e-270 ? 1e-270 : t2 * (1.0 + 3e-10);
+    if (threshold <= 0) h.thr2_lo = h.thr2_hi = -1.0;   // nothing is below it
+  }
   for (int d = 0; d < 3; d++) h.bmin[d] = ~0ULL;
   THC_CUDA(c, cudaMemcpyAsync(st, &h, sizeof(KmState), cudaMemcpyHostToDevice, s));
   THC_CUDA(c, cudaEventRecord(c->ev0, s));
@@ -1494,7 +1889,6 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   // Spatial binning of the grid (once per call): perm lists the points bin by bin.  From 8
   // centroids on, where the tile boxes fit the map's partials (part_s): at N_g 4320, N_mu 48
   // the pruned map takes 25 us against 530, the assign 6 against 52 (FP64).
-  const bool prune = c->km_prune && nmu >= 8;
   if (prune) {
     THC_CUDA(c, cudaMemsetAsync(b.bcount, 0, sizeof(int) * 2 * (size_t)nbins_max, s));
     km_bin_count<<<(int)cdiv(ng, 256), 256, 0, s>>>(grid, b);
@@ -1519,6 +1913,15 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   }
   THC_CUDA(c, cudaFuncSetAttribute(km_sums, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)sizeof(SumSmem)));
+  // 8 warps and 512 terms a block while most clusters fit that, so that more blocks share an SM;
+  // 16 and 1024 above.  us a call at a mean of 216 members (N_mu 2048): 9030 against 11060; at
+  // 432 (N_mu 256): 3770 against 3245.
+  const bool small_clusters = ng <= 320LL * nmu;
+  void (*cluster)(KmBufs) = small_clusters ? km_cluster<2, 4> : km_cluster<4, 8>;
+  const int cluster_threads = small_clusters ? 256 : 512;
+  const int cluster_smem = (int)(small_clusters ? sizeof(ClusterSmem<2, 4>) : sizeof(ClusterSmem<4, 8>));
+  THC_CUDA(c, cudaFuncSetAttribute(cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   cluster_smem));
   int* hflag = (int*)c->pinned;   // [2]: the done flag after a block of iterations
   const int kCheckEvery = 8;
   // One k-means iteration; every kernel reads the iteration index from device state and
@@ -1527,7 +1930,8 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
     // The pruned assign counts the histogram itself (put_label); the scatter clears it.
     if (prune) {
       ProfScope p(prof ? c : nullptr, "km_assign");
-      km_assign_p<<<nassign, kAssignThreads, prune_smem, s>>>(b);
+      if (by_cluster) km_assign_p<true><<<nassign, kAssignThreads, prune_smem, s>>>(b);
+      else km_assign_p<false><<<nassign, kAssignThreads, prune_smem, s>>>(b);
       THC_LAUNCHED(c, "km_assign_p");
     } else if (mixed) {
       {
@@ -1543,6 +1947,11 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
         km_assign64<<<nassign, kAssignThreads, 0, s>>>(b);
       }
       THC_LAUNCHED(c, "km_assign64");
+    }
+    if (by_cluster) {
+      cluster<<<nmu, cluster_threads, cluster_smem, s>>>(b);
+      THC_LAUNCHED(c, "km_cluster");
+      return THC_OK;
     }
     if (!prune) {
       km_hist<<<b.nb, 256, hist_smem, s>>>(b);
@@ -1612,7 +2021,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
     const int nblock = std::min(kCheckEvery, max_it - launched);
     if (gexec && nblock == kCheckEvery) {
       THC_CUDA(c, cudaGraphLaunch(gexec, s));
-      c->launches += (prune ? 5LL : mixed ? 7LL : 6LL) * kCheckEvery;  // kernels per captured iteration
+      c->launches += (by_cluster ? 2LL : prune ? 5LL : mixed ? 7LL : 6LL) * kCheckEvery;  // kernels per captured iteration
     } else {
       for (int k = 0; k < nblock; k++) {
         int rc = iteration(!fixed);

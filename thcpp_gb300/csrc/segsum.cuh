@@ -60,17 +60,12 @@ __device__ __forceinline__ void seg_compose(long long x0, long long x1, long lon
 // x = 0) a step is valid only for t == +0, and it leaves the sum at +0 (c = 0).
 __device__ __forceinline__ void seg_term(double t, int e, long long& c0, long long& c1, bool& bad)
 {
-  if (e == 0) {
-    c0 = c1 = 0;
-    bad = __double_as_longlong(t) != 0;
-    return;
-  }
   const unsigned long long tb = (unsigned long long)__double_as_longlong(t);
   const int et = (int)((tb >> 52) & 0x7ff);
   unsigned long long m = tb & ((1ULL << 52) - 1);
   if (et) m |= 1ULL << 52;
   const int sh = e - max(et, 1);                 // t = m 2^(-sh) grid units
-  bad = sh <= 0;
+  bad = e == 0 ? tb != 0 : sh <= 0;
   const int shc = min(max(sh, 1), 63);
   const unsigned long long kf = m >> shc;
   const unsigned long long rem = m & ((1ULL << shc) - 1);
@@ -78,8 +73,8 @@ __device__ __forceinline__ void seg_term(double t, int e, long long& c0, long lo
   const bool tie = rem == half;
   const long long k = (long long)(kf + (rem > half ? 1 : 0));
   const long long f = (long long)kf;
-  c0 = tie ? f + (f & 1) : k;
-  c1 = tie ? f + ((f + 1) & 1) : k;
+  c0 = e == 0 ? 0 : tie ? f + (f & 1) : k;
+  c1 = e == 0 ? 0 : tie ? f + ((f + 1) & 1) : k;
 }
 
 // Phases 1-3 for one window of cnt <= kSegWin terms: the segment table in sc (sc.nseg = -1
@@ -327,6 +322,220 @@ __device__ __forceinline__ double seg_walk_regs(double acc, const double* tw, in
     }
   }
   return acc;
+}
+
+// ---- The same sum over a chunk of windows, a warp per window of 32 PER terms: what the block
+// of km_cluster calls, with a barrier after each part (its windows share one unit, so that the
+// prediction needs no estimate of the earlier ones).  Few terms a lane, because a block waits on
+// one warp's chain of ~100 dependent instructions a term: eight a lane took 11,500 clocks a
+// window, however few its terms.  An entry holds all that a walk's step needs in one 32-byte
+// record, fetched a step ahead, and the significand map is applied to the FP64 word itself
+// (S -> S + c without a carry leaves the exponent alone): 650 -> 130 clocks a segment.
+// Loops over lanes' offsets stay rolled: the kernel's straight code outgrows the instruction cache.
+struct __align__(16) Seg {
+  double t;             // the segment's first term
+  long long c0, c1;     // the rest of the segment: word + c0 (even significand) or + c1 (odd)
+  unsigned e, mask;     // top word of a running sum in the predicted binade, and the bits that
+                        // count (none: any sum passes); mask's bit 0: the window's last segment
+};
+constexpr int kSegTab = 32;              // entries a window
+
+template <int NWIN>
+struct SegChunk {
+  int emax[NWIN];                        // largest biased exponent; >= 0x7ff: not summable here
+  long long units[NWIN];                 // window sums in units
+  int nseg[NWIN];                        // -1: too many segments
+  int usable;                            // every term finite and non-negative, not all zero
+  Seg tab[NWIN][kSegTab + 1];
+};
+
+// Part 1: a window's largest exponent.  t: the lane's terms (0 past the end).
+template <int PER>
+__device__ __forceinline__ int seg_emax(const double (&t)[PER])
+{
+  int m = 0;
+#pragma unroll
+  for (int u = 0; u < PER; u++) m = max(m, (int)((unsigned long long)__double_as_longlong(t[u]) >> 52));
+  return __reduce_max_sync(0xffffffffu, m);   // a sign bit counts as an exponent over 0x7ff
+}
+
+// x in units of 2^(emax - 1073): at most 2^10 terms and a running sum stay below 2^62 units.
+__device__ __forceinline__ long long seg_units(double x, int emax)
+{
+  const long long xb = __double_as_longlong(x);
+  const int ex = (int)((xb >> 52) & 0x7ff);
+  long long m = xb & ((1LL << 52) - 1);
+  if (ex) m |= 1LL << 52;
+  const int sh = emax + 2 - max(ex, 1);
+  return sh >= 63 ? 0 : (m >> sh);
+}
+
+// Part 2: the lane's inclusive prefix sums in units; returns the lanes' inclusive scan.
+template <int PER>
+__device__ __forceinline__ long long seg_prefix(const double (&t)[PER], int emax,
+                                                long long (&loc)[PER])
+{
+  long long run = 0;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    run += seg_units(t[u], emax);
+    loc[u] = run;
+  }
+  long long incl = run;
+#pragma unroll 1
+  for (int off = 1; off < 32; off <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, incl, off);
+    if ((int)(threadIdx.x & 31) >= off) incl += y;
+  }
+  return incl;
+}
+
+// Part 3: the window's table from the predicted sums base + loc[u] of its cnt terms.  Without
+// branches, and a map kept as c0 and d = c1 - c0: a term's d is 0, or +-1 for an exact half, and
+// composites keep to these three values (x then y: c0 = x0 + y[x0 & 1], and d is x's, or y's
+// with the sign of x0's parity where x has none).
+template <int PER>
+__device__ __forceinline__ int seg_table(const double (&t)[PER], const long long (&loc)[PER],
+                                         long long base, int emax, int cnt, Seg* tab)
+{
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, i0 = lane * PER;
+  auto compose = [](long long x0, int xd, long long& y0, int& yd) {
+    const bool odd = x0 & 1;
+    y0 += x0 + (odd ? yd : 0);
+    yd = xd ? xd : odd ? -yd : yd;
+  };
+  int E[PER];
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const long long P = base + loc[u];
+    E[u] = P > 0 ? (63 - __clzll(P)) + emax - 50 : 0;
+  }
+  const int prev = __shfl_up_sync(full, E[PER - 1], 1);
+  unsigned stm = 0, badm = 0;            // segment starts; bad since the start (in this lane)
+  long long c[PER];                      // composite since the start (in this lane)
+  int d[PER];
+  long long a0 = 0;
+  int ad = 0;
+  bool abad = false;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const bool in = i0 + u < cnt;
+    const bool start = in && (i0 + u == 0 || E[u] != (u ? E[u - 1] : prev));
+    long long c0, c1;
+    bool bad;
+    seg_term(t[u], E[u], c0, c1, bad);
+    int dd = (int)(c1 - c0);
+    compose(a0, ad, c0, dd);
+    a0 = start ? 0 : in ? c0 : a0;
+    ad = start ? 0 : in ? dd : ad;
+    abad = !start && (abad || (in && (bad || E[u] >= 0x7ff)));
+    stm |= (unsigned)start << u;
+    badm |= (unsigned)abad << u;
+    c[u] = a0;
+    d[u] = ad;
+  }
+  // (x then y) = y if y starts a segment, else their composite.  Flags: bit 0 a segment starts,
+  // bit 1 a bad step, the segments' number above.
+  long long s0 = a0;
+  int sd = ad, sf = (stm != 0) | (int)abad << 1 | __popc(stm) << 2;
+#pragma unroll 1
+  for (int off = 1; off < 32; off <<= 1) {
+    const long long x0 = __shfl_up_sync(full, s0, off);
+    const int xm = __shfl_up_sync(full, sf << 2 | (sd & 3), off);
+    const int xf = xm >> 2, xd = (int)((unsigned)xm << 30) >> 30;
+    long long y0 = s0;
+    int yd = sd;
+    compose(x0, xd, y0, yd);
+    const bool on = lane >= off, join = on && !(sf & 1);
+    s0 = join ? y0 : s0;
+    sd = join ? yd : sd;
+    sf = (join ? sf | (xf & 3) : sf) + (on ? xf & ~3 : 0);
+  }
+  long long e0 = __shfl_up_sync(full, s0, 1);
+  int ed = __shfl_up_sync(full, sd, 1), ef = __shfl_up_sync(full, sf, 1);
+  if (lane == 0) { e0 = 0; ed = 0; ef = 0; }
+  const int total = __shfl_sync(full, sf, 31) >> 2;
+  if (total > kSegTab) return -1;
+  unsigned next = __shfl_down_sync(full, stm & 1, 1);
+  if (lane == 31) next = 0;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const unsigned upto = stm & ((2u << u) - 1u);
+    const bool in = i0 + u < cnt, first = stm >> u & 1;
+    Seg* sg = tab + ((ef >> 2) - 1 + __popc(upto));
+    if (first) sg->t = t[u];
+    long long c0 = c[u];
+    int cd = d[u];
+    compose(e0, ed, c0, cd);
+    const bool mine = upto != 0;
+    c0 = mine ? c[u] : c0;
+    cd = mine ? d[u] : cd;
+    const bool bad = (badm >> u & 1) || (!mine && (ef & 2));
+    if (in && (i0 + u == cnt - 1 || (u + 1 < PER ? (stm >> (u + 1) & 1) : next))) {
+      sg->c0 = c0;
+      sg->c1 = c0 + cd;
+      // A one-term segment is its FP64 add: any sum passes.  A bad one: none does.
+      sg->e = bad ? 0xfff00000u : (unsigned)E[u] << 20;
+      sg->mask = (first ? 0u : 0xfff00000u) | (i0 + u == cnt - 1);
+    }
+  }
+  return total;
+}
+
+// Part 4: the exact running sums of four quantities over nwin windows, lane l walking quantity
+// l & 3 (a warp of its own each took twice as long: the FP64 unit serves the whole SM).  A
+// quantity whose tables are missing (ok false) or whose walk fails a check keeps its acc and
+// gets bad[q] set: its terms are to be added one by one.  One warp.
+template <int NWIN>
+__device__ __forceinline__ void seg_walk4(double* acc, int* bad, int nwin, const SegChunk<NWIN>* sc)
+{
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, q = lane & 3;
+  bool ok = sc[q].usable;
+  int left = 0;                          // the quantity's segments
+  if (ok) {
+#pragma unroll 1
+    for (int v = lane >> 2; v < nwin; v += 8) {
+      const int ns = sc[q].nseg[v];
+      ok &= ns >= 0;
+      left += ns;
+    }
+  }
+#pragma unroll 1
+  for (int off = 4; off < 32; off <<= 1) left += __shfl_xor_sync(full, left, off);
+  const unsigned okm = __ballot_sync(full, ok);
+  ok = ((okm >> q) & 0x11111111u) == 0x11111111u;
+  if (!ok) left = 0;
+  const int steps = __reduce_max_sync(full, left);
+  const Seg* p = sc[q].tab[0];
+  const Seg* next = sc[q].tab[1];        // of the next window
+  Seg nx = *p;
+  double a = acc[q];
+  bool good = true;
+#pragma unroll 1
+  for (int j = 0; j < steps; j++, left--) {
+    const Seg s = nx;
+    {                                    // the next entry, while this step's sum is under way
+      const bool over = s.mask & 1;
+      p = left > 1 ? over ? next : p + 1 : p;
+      next += over ? kSegTab + 1 : 0;
+      nx = *p;
+    }
+    const bool on = left > 0;            // past its last segment a quantity adds +0
+    const double t = on ? s.t : 0.0;
+    const long long c0 = on ? s.c0 : 0, c1 = on ? s.c1 : 0;
+    const unsigned mask = on ? s.mask & 0xfff00000u : 0u;
+    const long long ab = __double_as_longlong(__dadd_rn(a, t));
+    const long long rb = ab + ((ab & 1) ? c1 : c0);
+    good &= ((((unsigned)(ab >> 32) ^ s.e) | ((unsigned)(rb >> 32) ^ s.e)) & mask) == 0;
+    a = __longlong_as_double(rb);
+  }
+  ok &= good;
+  if (lane < 4) {
+    if (ok) acc[q] = a;
+    bad[q] = !ok;
+  }
 }
 
 // acc + t[0] + ... + t[n-1] evaluated left to right in FP64 round-to-nearest by one full
