@@ -117,6 +117,7 @@ struct KmBufs {
   int nbins_max;
   float* pf;       // [3][ng] FP32 coordinates in the binned order (pf[d][t] of point perm[t])
   float* box;      // [tiles][6] bounding boxes of its 256-point tiles (min x, y, z, max x, y, z)
+  float* wbox;     // [ceil(ng / 32)][6] the same of 32 points; shares recheck's memory
   // Sums by cluster (km_cluster; null: by the counting sort): which tiles hold a member, a bit
   // per tile, nwt words a cluster.  Labels are then in the binned order.
   unsigned* mask;
@@ -364,6 +365,7 @@ __device__ __forceinline__ void flush_changed(KmState* st, unsigned changed)
 }
 
 constexpr int kPruneMax = 1024;   // candidate centroids kept in shared memory per tile
+constexpr int kWarpMax = 64;      // and per warp
 
 // Assign with exact spatial pruning, for both precisions: FP32 filters, FP64 decides.
 //
@@ -375,28 +377,29 @@ constexpr int kPruneMax = 1024;   // candidate centroids kept in shared memory p
 // sqrt.  Of the kept centroids, in ascending index order, each thread takes the nearest in FP32
 // with the gap to the second: with u = 2^-24,
 //   |d2_32 - d2_64| <= u (2 |d| |a| + 5 d2) + O(u^2),   a_i = |c_i| + |g_i|,
-// so a gap above E(m1) + E(m2), E(m) = 2u (2 sqrt(m) |a| + 5 m) (a factor 2 for the O(u^2)
+// so a gap above 2 E(m2), E(m) = 2u (2 sqrt(m) |a| + 5 m) (a factor 2 for the O(u^2)
 // terms), proves that every other centroid is strictly farther in FP64, hence also after sqrt.
 // Other points are resolved at once in FP64 by their whole warp, one at a time, with the
 // reference's semantics.  The labels are those of an FP64 scan, whose 64 clocks an operation
 // and warp this part cannot afford (17 points a thread and 48 centroids took 52 us).  The test
 // itself is FP32 too, its terms raised by 1e-5 to cover its rounding: in FP64 its two roots
-// cost more than the scan (9 of 21 us at N_g 110592, N_mu 256).
+// cost more than the scan (9 of 21 us at N_g 110592, N_mu 256).  A second test with the box of
+// a warp's 32 points leaves it a third of the tile's candidates (N_g 442368, N_mu 2048: 50-180
+// to 7-45; the call 8.98 -> 8.58 ms).
 template <bool BY_TILE>
 __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
 {
   KmState* st = b.st;
-  if (st->done) return;
-  int it = st->iter;
+  // All of the state at once: a load behind another costs a memory latency, as does each below.
+  const int done = st->done, it = st->iter;
+  const float slack = (float)st->slack32, a = (float)st->abound * 1.00001f;
+  if (done) return;
   const float* cx = b.cen32 + (size_t)(it & 1) * 3 * b.nmu;
   const float* cy = cx + b.nmu;
   const float* cz = cy + b.nmu;
-  extern __shared__ unsigned char sm[];
-  int* cand = (int*)sm;
-  float* ccx = (float*)(sm + sizeof(int) * kPruneMax);
-  float* ccy = ccx + kPruneMax;
-  float* ccz = ccy + kPruneMax;
-  unsigned* kept = (unsigned*)(ccz + kPruneMax);        // 32 centroids a word
+  extern __shared__ __align__(16) unsigned char sm[];
+  float4* cand = (float4*)sm;                           // x, y, z and the index's bits
+  unsigned* kept = (unsigned*)(cand + kPruneMax);       // 32 centroids a word
   constexpr int kW = kAssignThreads / 32;
   __shared__ float uw[kW];
   __shared__ int wsum[kW];
@@ -404,12 +407,20 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
   bool valid = t < b.ng;
   long long i = valid ? b.perm[t] : 0;
   float g[3] = {0, 0, 0};
-  if (valid) { g[0] = b.pf[t]; g[1] = b.pf[b.ng + t]; g[2] = b.pf[2 * b.ng + t]; }
+  int before = 0;            // the label of the iteration before
+  if (valid) {
+    g[0] = b.pf[t]; g[1] = b.pf[b.ng + t]; g[2] = b.pf[2 * b.ng + t];
+    if (BY_TILE && it > 0) before = b.labels[(size_t)((it + 1) & 1) * b.ng + t];
+  }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  float lo[3], hi[3];
+  float lo[3], hi[3], wlo[3], whi[3];
+  const long long wrow = min(t, b.ng - 1) >> 5;
+#pragma unroll
   for (int d = 0; d < 3; d++) {
     lo[d] = b.box[(size_t)blockIdx.x * 6 + d];
     hi[d] = b.box[(size_t)blockIdx.x * 6 + 3 + d];
+    wlo[d] = b.wbox[wrow * 6 + d];
+    whi[d] = b.wbox[wrow * 6 + 3 + d];
   }
   // Warp w owns the words w nwords / kW .. of 32 consecutive centroids each, so that the
   // compaction keeps the index order with one exchange of counts.
@@ -433,7 +444,7 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
   __syncthreads();
   float U = uw[0];
   for (int w = 1; w < kW; w++) U = fminf(U, uw[w]);
-  const float cut = U * (1.0f + 1e-4f) + (float)st->slack32;
+  const float cut = U * (1.0f + 1e-4f) + slack;
   int count = 0;
 #pragma unroll 4
   for (int w = w0; w < w1; w++) {
@@ -464,24 +475,69 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
       const unsigned bal = kept[w];
       if (bal >> lane & 1) {
         const int k = w * 32 + lane, q = slot + __popc(bal & ((1u << lane) - 1u));
-        cand[q] = k; ccx[q] = cx[k]; ccy[q] = cy[k]; ccz[q] = cz[k];
+        cand[q] = make_float4(cx[k], cy[k], cz[k], __int_as_float(k));
       }
       slot += __popc(bal);
     }
   __syncthreads();
+  // The same test for the warp's 32 points, a candidate a lane, into a list of the warp's own.
+  __shared__ __align__(16) float4 wcand[kW][kWarpMax];
+  const float4* list = cand;
+  int nw = nc;
+  bool alone = false;
+  if (nc <= kPruneMax) {
+    auto bounds = [&](int j, float& ub) {
+      const float4 c = cand[j];
+      const float c3[3] = {c.x, c.y, c.z};
+      float lb = 0.f;
+      ub = 0.f;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const float p = c3[d] - wlo[d], q = c3[d] - whi[d], v = fmaxf(0.f, fmaxf(-p, q));
+        ub += fmaxf(p * p, q * q);
+        lb += v * v;
+      }
+      return lb;
+    };
+    float ub, wu = INFINITY;
+#pragma unroll 1
+    for (int j = lane; j < nc; j += 32) {
+      bounds(j, ub);
+      wu = fminf(wu, ub);
+    }
+    wu = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(wu)));
+    const float wcut = wu * (1.0f + 1e-4f) + slack;
+    nw = 0;
+#pragma unroll 1
+    for (int j0 = 0; j0 < nc; j0 += 32) {
+      const int j = j0 + lane;
+      const unsigned bal = __ballot_sync(0xffffffffu, j < nc && bounds(j, ub) <= wcut);
+      const int q = nw + __popc(bal & ((1u << lane) - 1u));
+      if ((bal >> lane & 1) && q < kWarpMax) wcand[wid][q] = cand[j];
+      nw += __popc(bal);
+    }
+    __syncwarp();
+    alone = nw == 1 && wcut < INFINITY;
+    if (nw <= kWarpMax) list = wcand[wid];
+    else nw = nc;
+  }
   bool amb = false;
   unsigned changed = 0;
   int k1 = 0;                // this point's label
   if (valid) {
     float m1 = INFINITY, m2 = INFINITY;
     if (nc <= kPruneMax) {
-      for (int j = 0; j < nc; j++) {
-        float dx = ccx[j] - g[0], dy = ccy[j] - g[1], dz = ccz[j] - g[2];
-        float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
-        if (d2 < m1) { m2 = m1; m1 = d2; k1 = j; }
-        else if (d2 < m2) { m2 = d2; }
+      // Without branches, one 16-byte load a candidate: 35 clocks each, 55 with the points of
+      // a warp on either side of a branch.
+#pragma unroll 4
+      for (int j = 0; j < nw; j++) {
+        const float4 c = list[j];
+        const float dx = c.x - g[0], dy = c.y - g[1], dz = c.z - g[2];
+        const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
+        m2 = fminf(m2, fmaxf(m1, d2));
+        k1 = d2 < m1 ? __float_as_int(c.w) : k1;
+        m1 = fminf(m1, d2);
       }
-      k1 = nc ? cand[k1] : 0;
     } else {
       for (int k = 0; k < b.nmu; k++) {
         float dx = cx[k] - g[0], dy = cy[k] - g[1], dz = cz[k] - g[2];
@@ -490,11 +546,13 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
         else if (d2 < m2) { m2 = d2; }
       }
     }
-    // 2u (2 |a| (sqrt m1 + sqrt m2) + 5 (m1 + m2)), every factor rounded up.
-    const float a = (float)st->abound * 1.00001f;
-    const float e = 1.1920929e-07f * 1.00001f *
-                    (2.f * a * (sqrtf(m1) + sqrtf(m2)) + 5.00001f * (m1 + m2));
-    amb = !((m2 - m1) * 0.99999f > e + 1e-30f);
+    // 2u (2 |a| (sqrt m1 + sqrt m2) + 5 (m1 + m2)), every factor rounded up and sqrt m2 for
+    // both roots (near ties, decided here, have them alike); on squares, without the root.  No
+    // tie where the boxes leave one centroid.
+    const float gap = (m2 - m1) * 0.99999f - 1.1920929e-07f * 5.0001f * (m1 + m2) - 1e-30f;
+    const float rt = 1.1920929e-07f * 4.0001f * a;
+    amb = !(gap > 0.f && gap * gap * 0.9999f > rt * rt * m2 * 1.0001f + 1e-36f) &&
+          !(alone && m1 < INFINITY);
   }
   // FP64 rescue of the near ties, at once and by the whole warp, one point at a time: the
   // exact first argmin of the sqrt distances (as km_recheck) over the tile's candidates in
@@ -513,7 +571,7 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
     am.init();
     if (nc <= kPruneMax) {
       for (int j = lane; j < nc; j += 32) {
-        const int k = cand[j];
+        const int k = __float_as_int(cand[j].w);
         am.push(d2_exact(px[k], py[k], pz[k], gx, gy, gz), k);
       }
     } else {
@@ -532,7 +590,7 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
     // In the binned order, with a bit for the tile in each of its clusters' masks.
     if (valid) {
       b.labels[(size_t)(it & 1) * b.ng + t] = k1;
-      if (it > 0 && b.labels[(size_t)((it + 1) & 1) * b.ng + t] != k1) changed = 1;
+      changed = it > 0 && before != k1;
     }
     const unsigned peers = __match_any_sync(0xffffffffu, valid ? k1 : -1);
     if (valid && lane == __ffs(peers) - 1)
@@ -1544,8 +1602,8 @@ __global__ void __launch_bounds__(1024) km_normdiff_exact(KmBufs b)
   }
 }
 
-// Bounding box of each 256-point tile of the binned order, from the FP32 coordinates (for
-// the pruned assign and map_to_grid; once per call).
+// Bounding boxes of each 256-point tile and each warp's 32 points of the binned order, from
+// the FP32 coordinates (for the pruned assign and map_to_grid; once per call).
 __global__ void km_tile_boxes(KmBufs b)
 {
   __shared__ float red[6][8];
@@ -1561,6 +1619,10 @@ __global__ void km_tile_boxes(KmBufs b)
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     }
     if (lane == 0) { red[d][wid] = mn; red[3 + d][wid] = mx; }
+    if (lane == 0 && valid) {
+      b.wbox[(t >> 5) * 6 + d] = mn;
+      b.wbox[(t >> 5) * 6 + 3 + d] = mx;
+    }
   }
   __syncthreads();
   if (threadIdx.x < 6) {
@@ -1815,7 +1877,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   int* tot = (int*)al.get(WS_KM_TOTAL, sizeof(int) * 2 * nmu);
   int* member = (int*)al.get(WS_KM_MEMBER, sizeof(int) * ng);
   double* terms = (double*)al.get(WS_KM_TERMS, sizeof(double) * 4 * nmu);
-  int* recheck = (int*)al.get(WS_KM_RECHECK, sizeof(int) * ng);
+  int* recheck = (int*)al.get(WS_KM_RECHECK, sizeof(int) * std::max(ng, 8LL));
   KmState* st = (KmState*)al.get(WS_KM_STATE, sizeof(KmState) + 64);
   double* logb = (double*)al.get(WS_KM_LOG, sizeof(double) * 2 * max_it);
   int nch = (int)cdiv(ng, kMapChunk);
@@ -1836,6 +1898,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   b.box = (float*)part_s;   // 6 floats per tile: at most 12 N_mu N_g / 1024 bytes from N_mu 8 on
   b.cen = cen; b.cen32 = cen32; b.labels = labels; b.hist = hist; b.total = tot;
   b.start = tot + nmu; b.member = member; b.terms = terms; b.recheck = recheck;
+  b.wbox = (float*)recheck;   // the pruned assign queues nothing
   b.log = logb; b.st = st;
   const bool prune = c->km_prune && nmu >= 8;
   // Clusters of kClusterMax members and fewer on average are summed a block each, in one
@@ -1901,7 +1964,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
     THC_LAUNCHED(c, "km_tile_boxes");
   }
   // Candidates (index and FP32 coordinates) and a bit per centroid.
-  const size_t prune_smem = (size_t)kPruneMax * (sizeof(int) + 3 * sizeof(float)) +
+  const size_t prune_smem = (size_t)kPruneMax * sizeof(float4) +
                             sizeof(unsigned) * (size_t)cdiv(nmu, 32);
   THC_CUDA(c, cudaMemsetAsync(hist, 0, sizeof(int) * (size_t)nmu * b.nb, s));
   const bool mixed = c->precision == THC_PREC_MIXED;
