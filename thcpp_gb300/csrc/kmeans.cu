@@ -364,6 +364,17 @@ __device__ __forceinline__ void flush_changed(KmState* st, unsigned changed)
   if ((threadIdx.x & 31) == 0 && changed) atomicAdd(&st->changed, (unsigned long long)changed);
 }
 
+// Programmatic dependent launch: a kernel of the iteration is set up while the one before it
+// runs out, and waits here, before its first load, until that one's writes are visible.  Every
+// block waits, also one with nothing to do, so that the order holds along the whole chain.  us a
+// call: 670 -> 650 at N_g 4320, N_mu 48, 3160 -> 3110 at 110592, 256.  Letting the next kernel's
+// blocks in before the last of this one's are done puts two km_cluster blocks on an SM where
+// others have none: 3160-3190.
+__device__ __forceinline__ void wait_for_previous()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 constexpr int kPruneMax = 1024;   // candidate centroids kept in shared memory per tile
 constexpr int kWarpMax = 64;      // and per warp
 
@@ -389,6 +400,7 @@ constexpr int kWarpMax = 64;      // and per warp
 template <bool BY_TILE>
 __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
 {
+  wait_for_previous();
   KmState* st = b.st;
   // All of the state at once: a load behind another costs a memory latency, as does each below.
   const int done = st->done, it = st->iter;
@@ -1240,6 +1252,7 @@ __global__ void __launch_bounds__(128 * NW, 1024 / (128 * NW)) km_cluster(KmBufs
   KmState* st = b.st;
   extern __shared__ __align__(16) unsigned char cl_smem[];
   ClusterSmem<NW, NWIN>& sm = *reinterpret_cast<ClusterSmem<NW, NWIN>*>(cl_smem);
+  wait_for_previous();
   const int done = st->done, it = st->iter;
   const int k = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // This warp's quantity and first window.
@@ -1814,6 +1827,23 @@ __global__ void km_sort(int* idx, int n, int npow2, int* dups)
 
 }  // namespace
 
+// A launch that may overlap the end of the kernel before it on the stream (wait_for_previous).
+static cudaError_t launch_chained(void (*kernel)(KmBufs), int grid, int threads, size_t smem,
+                                  cudaStream_t s, const KmBufs& b)
+{
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &a;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, b);
+}
+
 int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng, int nmu,
                const int* init_in, int max_it, double threshold, int* out_idx,
                thc_kmeans_stats* stats, KmAlloc* fixed)
@@ -1993,7 +2023,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
     // The pruned assign counts the histogram itself (put_label); the scatter clears it.
     if (prune) {
       ProfScope p(prof ? c : nullptr, "km_assign");
-      if (by_cluster) km_assign_p<true><<<nassign, kAssignThreads, prune_smem, s>>>(b);
+      if (by_cluster) THC_CUDA(c, launch_chained(km_assign_p<true>, nassign, kAssignThreads, prune_smem, s, b));
       else km_assign_p<false><<<nassign, kAssignThreads, prune_smem, s>>>(b);
       THC_LAUNCHED(c, "km_assign_p");
     } else if (mixed) {
@@ -2012,7 +2042,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
       THC_LAUNCHED(c, "km_assign64");
     }
     if (by_cluster) {
-      cluster<<<nmu, cluster_threads, cluster_smem, s>>>(b);
+      THC_CUDA(c, launch_chained(cluster, nmu, cluster_threads, cluster_smem, s, b));
       THC_LAUNCHED(c, "km_cluster");
       return THC_OK;
     }
