@@ -94,95 +94,94 @@ struct GjStatus {
   double max_abs2;
 };
 
-// Step k, part 1 (one block): pivot p = argmax_{r >= k} |A[r][k]|^2 (lowest row on ties),
-// swap rows k and p, scale row k by 1 / A[k][k], and save column k (after the swap) in f.
-__global__ void __launch_bounds__(1024) gj_pivot(double* a, int n, int k, double* f,
-                                                 GjStatus* gs)
+// Step k of the elimination, in one kernel: the pivot p = argmax_{r >= k} |A[r][k]|^2 (lowest row
+// on ties), rows k and p swapped, row k scaled by 1 / A[k][k], and A[r][c] -= A[r][k] A[k][c] for
+// every other row and the columns c > k (those up to k are not read again).  From one buffer into
+// the other, so that every block can find the pivot by itself and the swap is a choice of rows;
+// with a pivot kernel of one block and an elimination in place the 144 steps at N_mu 144 took 2.4
+// ms, now 0.5 (0.9 without the chained launches).  What bounds a step is the chain of column,
+// pivot, reciprocal and row; R rows a thread are as few as keep the blocks resident at once.
+constexpr int kGjCols = 64, kGjThreads = 256;   // 64 columns, 4 rows at a time
+template <int R>
+__global__ void __launch_bounds__(kGjThreads) gj_step(const double2* __restrict__ a, double2* o,
+                                                      int n, int k, GjStatus* gs)
 {
-  __shared__ double bv[32];
-  __shared__ int bi[32];
+  __shared__ long long bv[kGjThreads / 32];
+  __shared__ int bi[kGjThreads / 32];
   __shared__ double piv[2];
-  const long long w = 2LL * n;                        // complex row length
-  if (gs->singular) return;
-  double best = -1.0;
+  wait_for_previous();
+  const unsigned full = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long w = 2LL * n;                        // row length
+  const int over = gs->singular;
+  // Integer comparisons: an FP64 one holds its warp as long as an FP64 sum.  NaN never wins.
+  long long best = -1;
   int arg = n;
-  for (int r = k + threadIdx.x; r < n; r += blockDim.x) {
-    const double re = a[2 * (r * w + k)], im = a[2 * (r * w + k) + 1];
-    const double v = re * re + im * im;
-    if (v > best) { best = v; arg = r; }
+  for (int r = k + tid; r < n; r += kGjThreads) {
+    const double2 z = a[r * w + k];
+    const double v = z.x * z.x + z.y * z.y;
+    const long long b = v >= 0.0 ? __double_as_longlong(v) : -1;
+    if (b > best) { best = b; arg = r; }
   }
-  for (int off = 16; off; off >>= 1) {
-    const double v2 = __shfl_xor_sync(0xffffffffu, best, off);
-    const int i2 = __shfl_xor_sync(0xffffffffu, arg, off);
-    if (v2 > best || (v2 == best && i2 < arg)) { best = v2; arg = i2; }
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto warp_best = [&]() {
+    const int hi = __reduce_max_sync(full, (int)(best >> 32));
+    bool in = (int)(best >> 32) == hi;
+    const unsigned lo = __reduce_max_sync(full, in ? (unsigned)best : 0u);
+    in = in && (unsigned)best == lo;
+    arg = __reduce_min_sync(full, in ? arg : n);
+    best = (long long)hi << 32 | lo;
+  };
+  warp_best();
   if (lane == 0) { bv[warp] = best; bi[warp] = arg; }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 1; q < (int)(blockDim.x >> 5); q++)
-      if (bv[q] > bv[0] || (bv[q] == bv[0] && bi[q] < bi[0])) { bv[0] = bv[q]; bi[0] = bi[q]; }
-    if (!(bv[0] > 0.0) || bi[0] >= n) {
-      gs->singular = k + 1;
-    } else {
-      gs->min_abs2 = k ? fmin(gs->min_abs2, bv[0]) : bv[0];
-      gs->max_abs2 = k ? fmax(gs->max_abs2, bv[0]) : bv[0];
-    }
-  }
-  __syncthreads();
-  if (gs->singular) return;
-  const int p = bi[0];
-  if (p != k)
-    for (long long c = threadIdx.x; c < 2 * w; c += blockDim.x) {
-      const double t = a[2 * k * w + c];
-      a[2 * k * w + c] = a[2 * p * w + c];
-      a[2 * p * w + c] = t;
-    }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    // 1 / (x + i y) = (x - i y) / (x^2 + y^2)
-    const double x = a[2 * (k * w + k)], y = a[2 * (k * w + k) + 1];
-    const double d = x * x + y * y;
-    piv[0] = x / d;
-    piv[1] = -y / d;
-  }
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    f[2 * r] = a[2 * (r * w + k)];
-    f[2 * r + 1] = a[2 * (r * w + k) + 1];
-  }
-  __syncthreads();
-  const double ir = piv[0], ii = piv[1];
-  // Row k: every column from k on (the left part below k is already zero; the right part,
-  // permuted by the row swaps, is dense in general).
-  for (long long c = k + threadIdx.x; c < w; c += blockDim.x) {
-    const double x = a[2 * (k * w + c)], y = a[2 * (k * w + c) + 1];
-    a[2 * (k * w + c)] = x * ir - y * ii;
-    a[2 * (k * w + c) + 1] = x * ii + y * ir;
-  }
-}
-
-// Step k, part 2: A[r][c] -= f[r] A[k][c] for every row r != k and column c >= k (the
-// left part before k is zero), and column k becomes e_k.
-__global__ void gj_eliminate(double* a, int n, int k, const double* __restrict__ f,
-                             const GjStatus* gs)
-{
-  if (gs->singular) return;
-  const long long w = 2LL * n;
-  const long long ncols = w - k;
-  long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= (long long)n * ncols) return;
-  const int r = (int)(e / ncols);
-  const long long c = k + e % ncols;
-  if (r == k) return;
-  if (c == k) {
-    a[2 * (r * w + k)] = 0.0;
-    a[2 * (r * w + k) + 1] = 0.0;
+  best = lane < kGjThreads / 32 ? bv[lane] : -1;
+  arg = lane < kGjThreads / 32 ? bi[lane] : n;
+  warp_best();
+  if (over) return;
+  const int p = arg;
+  if (best <= 0 || p >= n) {
+    if (blockIdx.x + blockIdx.y == 0 && tid == 0) gs->singular = k + 1;
     return;
   }
-  const double fr = f[2 * r], fi = f[2 * r + 1];
-  const double xr = a[2 * (k * w + c)], xi = a[2 * (k * w + c) + 1];
-  a[2 * (r * w + c)] = __fma_rn(-fr, xr, __fma_rn(fi, xi, a[2 * (r * w + c)]));
-  a[2 * (r * w + c) + 1] = __fma_rn(-fr, xi, __fma_rn(-fi, xr, a[2 * (r * w + c) + 1]));
+  const long long c = k + 1 + (long long)blockIdx.x * kGjCols + (tid & (kGjCols - 1));
+  const int r0 = (int)blockIdx.y * 4 * R + tid / kGjCols;
+  const bool in = c < w;
+  double2 x = {0.0, 0.0}, y[R], f[R];
+  if (in) x = a[p * w + c];
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const int r = r0 + 4 * q, m = r == p ? k : r;
+    y[q] = f[q] = {0.0, 0.0};
+    if (in && r < n && r != k) {
+      y[q] = a[m * w + c];
+      f[q] = a[m * w + k];
+    }
+  }
+  if (warp == 0) {
+    // 1 / (x + i y) = (x - i y) / (x^2 + y^2), a lane each.
+    const double2 z = a[p * w + k];
+    const double d = z.x * z.x + z.y * z.y, v = (lane ? -z.y : z.x) / d;
+    if (lane < 2) piv[lane] = v;
+    if (blockIdx.x + blockIdx.y == 0 && lane == 0) {
+      const double b = __longlong_as_double(best);
+      gs->min_abs2 = k ? fmin(gs->min_abs2, b) : b;
+      gs->max_abs2 = k ? fmax(gs->max_abs2, b) : b;
+    }
+  }
+  __syncthreads();
+  if (!in) return;
+  const double2 xs = {x.x * piv[0] - x.y * piv[1], x.x * piv[1] + x.y * piv[0]};
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const int r = r0 + 4 * q;
+    if (r >= n) continue;
+    double2 z = xs;
+    if (r != k) {
+      z.x = __fma_rn(-f[q].x, xs.x, __fma_rn(f[q].y, xs.y, y[q].x));
+      z.y = __fma_rn(-f[q].x, xs.y, __fma_rn(-f[q].y, xs.x, y[q].y));
+    }
+    o[r * w + c] = z;
+  }
 }
 
 // zeta (interleaved complex, row mu = zeta_mu on the grid) = conj(XR + i XI).
@@ -281,7 +280,7 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   double* qrqi = (double*)ws_get(c, WS_ZETA, sizeof(double) * 2 * nmg);   // P_occ, then X
   double* spec = (double*)ws_get(c, WS_ZHAT, sizeof(double) * 4 * nmg);   // IVG, IVMG
   double* aug = (double*)ws_get(c, WS_C, sizeof(double) * 4 * nn);        // [C | I]
-  double* fcol = (double*)ws_get(c, WS_CINV, sizeof(double) * 2 * nmu + 64);
+  double* aug2 = (double*)ws_get(c, WS_CINV, sizeof(double) * 4 * nn);
   double* Mw = (double*)ws_get(c, WS_M, sizeof(double) * 4 * nn);
   char* scr = (char*)ws_get(c, WS_SCRATCH, 4096);
   const bool orb_host = out_orb && !is_device_ptr(out_orb);
@@ -289,7 +288,7 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   double* stage = nullptr;
   if (orb_host || occ_host)
     stage = (double*)ws_get(c, WS_ORB, sizeof(double) * 2 * nmu * (no + nocc));
-  if (!rows || !prpi || !qrqi || !spec || !aug || !fcol || !Mw || !scr ||
+  if (!rows || !prpi || !qrqi || !spec || !aug || !aug2 || !Mw || !scr ||
       ((orb_host || occ_host) && !stage))
     return set_error(c, THC_ERR_NOMEM, "thc_isdf_half_complex: workspace allocation failed");
   double* pmu = rows;
@@ -333,13 +332,18 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   // C^{-1} by Gauss-Jordan elimination on [C | I].
   build_augmented<<<(int)cdiv(2 * nn, 256), 256, 0, s>>>(pr, pi, ng, idx, nmu, aug);
   THC_LAUNCHED(c, "build_augmented");
+  // The fewest rows a thread whose blocks the 152 SMs hold at once, eight each.
+  int gr = 1;
+  while (gr < 8 && cdiv(nmu, 4 * gr) * cdiv(2 * nmu, kGjCols) > 152 * 8) gr *= 2;
+  auto step = gr == 1 ? gj_step<1> : gr == 2 ? gj_step<2> : gr == 4 ? gj_step<4> : gj_step<8>;
   for (int k = 0; k < nmu; k++) {
-    gj_pivot<<<1, 1024, 0, s>>>(aug, nmu, k, fcol, gs);
-    const long long items = (long long)nmu * (2LL * nmu - k);
-    gj_eliminate<<<(unsigned)cdiv(items, 256), 256, 0, s>>>(aug, nmu, k, fcol, gs);
+    const dim3 grid((unsigned)cdiv(2LL * nmu - k - 1, kGjCols), (unsigned)cdiv(nmu, 4 * gr));
+    THC_CUDA(c, launch_chained(step, grid, kGjThreads, 0, s, (const double2*)aug, (double2*)aug2,
+                               nmu, k, gs));
+    std::swap(aug, aug2);
   }
-  c->launches += 2LL * nmu;
-  THC_LAUNCHED(c, "gj_eliminate");
+  c->launches += nmu;
+  THC_LAUNCHED(c, "gj_step");
   // X = C^{-1} Z as one real product of 2 N_mu rows and 2 N_mu terms (into the P_occ buffers).
   {
     double* ci = (double*)ws_get(c, WS_DINV, sizeof(double) * 4 * nn);

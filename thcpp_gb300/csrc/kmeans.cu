@@ -364,17 +364,6 @@ __device__ __forceinline__ void flush_changed(KmState* st, unsigned changed)
   if ((threadIdx.x & 31) == 0 && changed) atomicAdd(&st->changed, (unsigned long long)changed);
 }
 
-// Programmatic dependent launch: a kernel of the iteration is set up while the one before it
-// runs out, and waits here, before its first load, until that one's writes are visible.  Every
-// block waits, also one with nothing to do, so that the order holds along the whole chain.  us a
-// call: 670 -> 650 at N_g 4320, N_mu 48, 3160 -> 3110 at 110592, 256.  Letting the next kernel's
-// blocks in before the last of this one's are done puts two km_cluster blocks on an SM where
-// others have none: 3160-3190.
-__device__ __forceinline__ void wait_for_previous()
-{
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 constexpr int kPruneMax = 1024;   // candidate centroids kept in shared memory per tile
 constexpr int kWarpMax = 64;      // and per warp
 
@@ -1827,23 +1816,6 @@ __global__ void km_sort(int* idx, int n, int npow2, int* dups)
 
 }  // namespace
 
-// A launch that may overlap the end of the kernel before it on the stream (wait_for_previous).
-static cudaError_t launch_chained(void (*kernel)(KmBufs), int grid, int threads, size_t smem,
-                                  cudaStream_t s, const KmBufs& b)
-{
-  cudaLaunchAttribute a{};
-  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  a.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &a;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, b);
-}
-
 int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng, int nmu,
                const int* init_in, int max_it, double threshold, int* out_idx,
                thc_kmeans_stats* stats, KmAlloc* fixed)
@@ -2017,6 +1989,10 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
                                    cluster_smem));
   int* hflag = (int*)c->pinned;   // [2]: the done flag after a block of iterations
   const int kCheckEvery = 8;
+  // The two kernels of the summed-by-cluster form are chained (launch_chained), us a call: 670 ->
+  // 650 at N_g 4320, N_mu 48, 3160 -> 3110 at 110592, 256.  Letting the next kernel's blocks in
+  // before the last of this one's are done puts two km_cluster blocks on an SM where others
+  // have none: 3160-3190.
   // One k-means iteration; every kernel reads the iteration index from device state and
   // returns at once after convergence, so the same launch sequence serves any iteration.
   auto iteration = [&](bool prof) -> int {
