@@ -103,7 +103,7 @@ struct GjStatus {
 // pivot, reciprocal and row; R rows a thread are as few as keep the blocks resident at once.
 constexpr int kGjCols = 64, kGjThreads = 256;   // 64 columns, 4 rows at a time
 template <int R>
-__global__ void __launch_bounds__(kGjThreads) gj_step(const double2* __restrict__ a, double2* o,
+__global__ void __launch_bounds__(kGjThreads) gj_step(const double2* a, double2* o,
                                                       int n, int k, GjStatus* gs)
 {
   __shared__ long long bv[kGjThreads / 32];
