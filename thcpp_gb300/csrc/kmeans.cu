@@ -1047,7 +1047,11 @@ __device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double*
   for (int i = threadIdx.x + blockDim.x; i < nmu; i += blockDim.x)
     em = max(em, biased_exponent(__ldcg(part + i)));
   const int bad = *(volatile int*)&st->empty | *(volatile int*)&st->bad_label;
-  const double lo = st->thr2_lo, hi = st->thr2_hi;
+  // Everything the decision reads, at once.
+  const double lo = st->thr2_lo, hi = st->thr2_hi, thr = st->threshold;
+  const unsigned long long changed = __ldcg(&st->changed);
+  const int rechecks = __ldcg(&st->recheck_n), max_it = st->max_it;
+  const long long rechecked = st->rechecked_total;
   em = __reduce_max_sync(0xffffffffu, em);
   long long su = 0;
   if (em < 0x7ff) {
@@ -1077,7 +1081,7 @@ __device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double*
     if (lane == 0) res[3] = v;
   }
   __syncthreads();
-  const double sum = res[3], thr = st->threshold;
+  const double sum = res[3];
   const bool exact = (!(sum < lo) && !(sum > hi)) || sum < 1e-280;
   double diff = 0.0;
   if (exact) diff = normdiff_block(b, it, red, res);
@@ -1085,15 +1089,15 @@ __device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double*
     st->diff_exact = exact;
     // The difference itself under a sign bit, or the sum of squares; the changed labels' count.
     b.log[it] = exact ? __longlong_as_double(__double_as_longlong(diff) | (1LL << 63)) : sum;
-    b.log[st->max_it + it] = __longlong_as_double((long long)st->changed);
+    b.log[max_it + it] = __longlong_as_double((long long)changed);
     st->changed = 0;
-    st->rechecked_total += st->recheck_n;
+    st->rechecked_total = rechecked + rechecks;
     st->recheck_n = 0;
     st->final_buf = (it + 1) & 1;
     if (exact ? diff < thr : sum < lo) {
       st->converged = 1;
       st->done = 1;
-    } else if (it + 1 >= st->max_it) {
+    } else if (it + 1 >= max_it) {
       st->done = 1;
       st->zero_fill = exact ? !(diff > thr) : 0;
     }

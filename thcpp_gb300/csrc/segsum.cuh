@@ -484,7 +484,7 @@ __device__ __forceinline__ int seg_table(const double (&t)[PER], const long long
 }
 
 // Part 4: the exact running sums of four quantities over nwin windows, lane l walking quantity
-// l & 3 (a warp of its own each took twice as long: the FP64 unit serves the whole SM).  A
+// l & 3 (a warp of its own each measured twice as long).  A
 // quantity whose tables are missing (ok false) or whose walk fails a check keeps its acc and
 // gets bad[q] set: its terms are to be added one by one.  One warp.
 template <int NWIN>
