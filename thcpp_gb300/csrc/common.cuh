@@ -189,33 +189,6 @@ int check_launch(Ctx* c, const char* what);
 
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-#if defined(__CUDACC__)
-// Programmatic dependent launch, for chains of short kernels (a launch boundary costs ~1.3 us):
-// a kernel is set up while the one before it on the stream runs out, and waits, before its first
-// load, until that one's writes are visible.  Every block of a chained kernel calls
-// wait_for_previous, also one with nothing to do, so that the order holds along the chain.
-__device__ __forceinline__ void wait_for_previous()
-{
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
-                                  cudaStream_t s, A... args)
-{
-  cudaLaunchAttribute a{};
-  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  a.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = &a;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-#endif
-
 // Residency of a caller pointer.
 bool is_device_ptr(const void* p);
 

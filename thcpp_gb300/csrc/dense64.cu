@@ -107,7 +107,6 @@ __global__ void __launch_bounds__(256) dgemm_kernel(GemmArgs g)
 // Sum split-K partials in split order, then apply the epilogue.
 __global__ void dgemm_reduce(GemmArgs g)
 {
-  wait_for_previous();
   long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (e >= g.M * g.N) return;
   long long m = e / g.N, n = e % g.N;
@@ -164,7 +163,6 @@ constexpr int CS = NB + 2;                   // shared row length: 16-byte rows,
 __global__ void __launch_bounds__(256) chol_diag(double* A, long long ld, int n, int k0,
                                                  const double* thr_p, CholStatus* cs, double* dinv)
 {
-  wait_for_previous();
   if (cs->flag) return;
   const double thr = thr_p ? *thr_p : 0.0;
   __shared__ __align__(16) double a[NB][CS];
@@ -298,7 +296,6 @@ constexpr int IW = 4;                        // columns a block: one warp to eac
 __global__ void __launch_bounds__(32 * IW) chol_diag_inv(const double* A, long long ld, int n,
                                                          int k0, const CholStatus* cs, double* dinv)
 {
-  wait_for_previous();
   if (cs->flag) return;
   __shared__ double a[NB][NB + 1];
   __shared__ double rr[NB];
@@ -343,9 +340,9 @@ __global__ void __launch_bounds__(32 * IW) chol_diag_inv(const double* A, long l
 // launch).  Two threads an entry sum k below and above 32, the order of that GEMM's split.
 template <int R>
 __global__ void __launch_bounds__(128 * R) chol_panel(double* P, long long ld, int rows,
-                                                      const double* dinv, const int* flag)
+                                                      const double* __restrict__ dinv,
+                                                      const int* flag)
 {
-  wait_for_previous();
   if (*flag) return;
   __shared__ __align__(16) double v[NB][CS];
   __shared__ __align__(16) double x[R][NB];
@@ -384,10 +381,9 @@ __global__ void __launch_bounds__(128 * R) chol_panel(double* P, long long ld, i
 // takes two FMAs a clock and 192 rows are 1.2e6 of them.  (That GEMM and the sum of its
 // partials were two launches of 12 and 4 us at 192 rows.)
 constexpr int RM = 8, RN = 16;
-__global__ void __launch_bounds__(256) chol_rank64(const double* L, double* C,
+__global__ void __launch_bounds__(256) chol_rank64(const double* __restrict__ L, double* C,
                                                    long long ld, int rows, const int* flag)
 {
-  wait_for_previous();
   // Tile t: row block i of 8 reaches column block i / 2 of 16; 2 q (q + 1) / 2 tiles lie
   // before row blocks 2q and 2q + 1, which have q + 1 each.
   const int t = blockIdx.x;
@@ -570,7 +566,7 @@ int dgemm(Ctx* c, const GemmArgs& g_in)
 
 int dgemm_reduce_partials(Ctx* c, const GemmArgs& g)
 {
-  THC_CUDA(c, launch_chained(dgemm_reduce, (int)cdiv(g.M * g.N, 256), 256, 0, c->stream, g));
+  dgemm_reduce<<<(unsigned)cdiv(g.M * g.N, 256), 256, 0, c->stream>>>(g);
   THC_LAUNCHED(c, "dgemm_reduce");
   return THC_OK;
 }
@@ -583,14 +579,12 @@ static int rank64_update(Ctx* c, const GemmArgs& g)
   choose_tile(t);
   if (t.ksplit != 2 || g.K != NB) return dgemm(c, g);
   const long long q = cdiv(g.M, 2 * RM);
-  THC_CUDA(c, launch_chained(chol_rank64, (int)(q * (q + 1)), 256, 0, c->stream, g.A, g.C, g.ldc,
-                             (int)g.M, g.skip_flag));
+  chol_rank64<<<(unsigned)(q * (q + 1)), 256, 0, c->stream>>>(g.A, g.C, g.ldc, (int)g.M,
+                                                             g.skip_flag);
   THC_LAUNCHED(c, "chol_rank64");
   return THC_OK;
 }
 
-// The kernels are chained launches, 18 of them in a row at n 256 (0.49 -> 0.45 ms with the
-// inverse's reductions), but for a panel behind another stream's event.
 // Blocked Cholesky whose panel solve is a GEMM with the inverted diagonal block; the
 // inverted diagonal blocks are kept in dinv (nblk x 64 x 64) for the triangular inverse.
 int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholStatus* cs,
@@ -609,9 +603,9 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
   for (int k0 = 0; k0 < n; k0 += NB) {
     int nb = std::min(NB, n - k0);
     double* di = dinv + (long long)(k0 / NB) * NB * NB;
-    THC_CUDA(c, launch_chained(chol_diag, 1, 256, 0, s, A, ld, n, k0, thr, cs, di));
+    chol_diag<<<1, 256, 0, s>>>(A, ld, n, k0, thr, cs, di);
     THC_LAUNCHED(c, "chol_diag");
-    THC_CUDA(c, launch_chained(chol_diag_inv, NB / IW, 32 * IW, 0, s, A, ld, n, k0, cs, di));
+    chol_diag_inv<<<NB / IW, 32 * IW, 0, s>>>(A, ld, n, k0, cs, di);
     THC_LAUNCHED(c, "chol_diag_inv");
     int rest = n - k0 - nb;
     if (rest <= 0) break;
@@ -623,10 +617,8 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
       double* panel = A + (long long)(k0 + nb) * ld + k0;
       // Rows a CTA: two while their blocks find an SM at once, else four, which share the copy
       // of the inverse block.
-      const int rows = rest <= 608 ? 2 : 4, grid = (int)cdiv(rest, rows);
-      auto kernel = rows == 2 ? chol_panel<2> : chol_panel<4>;
-      if (la) kernel<<<grid, 128 * rows, 0, s>>>(panel, ld, rest, di, &cs->flag);   // after an event
-      else THC_CUDA(c, launch_chained(kernel, grid, 128 * rows, 0, s, panel, ld, rest, di, &cs->flag));
+      if (rest <= 608) chol_panel<2><<<(unsigned)cdiv(rest, 2), 256, 0, s>>>(panel, ld, rest, di, &cs->flag);
+      else chol_panel<4><<<(unsigned)cdiv(rest, 4), 512, 0, s>>>(panel, ld, rest, di, &cs->flag);
       THC_LAUNCHED(c, "chol_panel");
     }
     const double* l21 = A + (long long)(k0 + nb) * ld + k0;
@@ -723,8 +715,8 @@ int chol_inverse(Ctx* c, const double* L, long long ld, int n, const double* din
   g.M = n; g.N = n; g.K = n;                            // Cinv = X^T X
   g.A = X; g.sam = 1; g.sak = ld;
   g.B = X; g.sbn = 1; g.sbk = ld;
-  g.a_zero_below = g.b_zero_below = 1;                  // X lower triangular
   g.C = Cinv; g.ldc = n;
+  g.a_zero_below = g.b_zero_below = 1;                  // X lower triangular
   g.skip_flag = cs ? &cs->flag : nullptr;
   return dgemm(c, g);
 }

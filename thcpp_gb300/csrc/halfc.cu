@@ -99,17 +99,16 @@ struct GjStatus {
 // every other row and the columns c > k (those up to k are not read again).  From one buffer into
 // the other, so that every block can find the pivot by itself and the swap is a choice of rows;
 // with a pivot kernel of one block and an elimination in place the 144 steps at N_mu 144 took 2.4
-// ms, now 0.5 (0.9 without the chained launches).  What bounds a step is the chain of column,
+// ms, now 0.9.  What bounds a step is the chain of column,
 // pivot, reciprocal and row; R rows a thread are as few as keep the blocks resident at once.
 constexpr int kGjCols = 64, kGjThreads = 256;   // 64 columns, 4 rows at a time
 template <int R>
-__global__ void __launch_bounds__(kGjThreads) gj_step(const double2* a, double2* o,
+__global__ void __launch_bounds__(kGjThreads) gj_step(const double2* __restrict__ a, double2* o,
                                                       int n, int k, GjStatus* gs)
 {
   __shared__ long long bv[kGjThreads / 32];
   __shared__ int bi[kGjThreads / 32];
   __shared__ double piv[2];
-  wait_for_previous();
   const unsigned full = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long w = 2LL * n;                        // row length
@@ -338,8 +337,7 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   auto step = gr == 1 ? gj_step<1> : gr == 2 ? gj_step<2> : gr == 4 ? gj_step<4> : gj_step<8>;
   for (int k = 0; k < nmu; k++) {
     const dim3 grid((unsigned)cdiv(2LL * nmu - k - 1, kGjCols), (unsigned)cdiv(nmu, 4 * gr));
-    THC_CUDA(c, launch_chained(step, grid, kGjThreads, 0, s, (const double2*)aug, (double2*)aug2,
-                               nmu, k, gs));
+    step<<<grid, kGjThreads, 0, s>>>((const double2*)aug, (double2*)aug2, nmu, k, gs);
     std::swap(aug, aug2);
   }
   c->launches += nmu;

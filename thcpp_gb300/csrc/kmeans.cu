@@ -389,7 +389,6 @@ constexpr int kWarpMax = 64;      // and per warp
 template <bool BY_TILE>
 __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
 {
-  wait_for_previous();
   KmState* st = b.st;
   // All of the state at once: a load behind another costs a memory latency, as does each below.
   const int done = st->done, it = st->iter;
@@ -588,6 +587,10 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
     if (lane == p) k1 = k;
   }
   if (BY_TILE) {
+    if ((unsigned)k1 >= (unsigned)b.nmu) {   // reported, not used as an index
+      st->bad_label = 1;
+      k1 = 0;
+    }
     // In the binned order, with a bit for the tile in each of its clusters' masks.
     if (valid) {
       b.labels[(size_t)(it & 1) * b.ng + t] = k1;
@@ -1245,7 +1248,6 @@ __global__ void __launch_bounds__(128 * NW, 1024 / (128 * NW)) km_cluster(KmBufs
   KmState* st = b.st;
   extern __shared__ __align__(16) unsigned char cl_smem[];
   ClusterSmem<NW, NWIN>& sm = *reinterpret_cast<ClusterSmem<NW, NWIN>*>(cl_smem);
-  wait_for_previous();
   const int done = st->done, it = st->iter;
   const int k = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // This warp's quantity and first window.
@@ -1305,8 +1307,13 @@ __global__ void __launch_bounds__(128 * NW, 1024 / (128 * NW)) km_cluster(KmBufs
         i[q] = t < b.ng ? b.perm[t] : -1;
       }
 #pragma unroll
-      for (int q = 0; q < 4; q++)
+      for (int q = 0; q < 4; q++) {
         if (l[q] != k) i[q] = -1;
+        else if ((unsigned)i[q] >= (unsigned)b.ng) {   // reported, not used as an index
+          st->bad_label = 1;
+          i[q] = -1;
+        }
+      }
       f(i);
     }
   };
@@ -1343,7 +1350,8 @@ __global__ void __launch_bounds__(128 * NW, 1024 / (128 * NW)) km_cluster(KmBufs
     }
   }
   __syncthreads();
-  const int n = sm.n, imin = sm.imin, imax = sm.imax;
+  int n = sm.n;
+  const int imin = sm.imin, imax = sm.imax;
   // The four terms of grid point i.
   auto terms = [&](int i, double (&x)[4]) {
     if (b.tq) {
@@ -1466,7 +1474,12 @@ __global__ void __launch_bounds__(128 * NW, 1024 / (128 * NW)) km_cluster(KmBufs
   } else {
     if (tid == 0) sm.off = atomicAdd(&st->listed, n);
     __syncthreads();
+    if ((long long)sm.off + n > b.ng) {                // as above
+      if (tid == 0) st->bad_label = 1;
+      n = 0;
+    }
     int* run = b.member + sm.off;
+    int left = n;                                      // entries of the run not written yet
     list = run;
 #pragma unroll 1
     for (long long lo = imin; lo <= imax; lo += 32LL * kBmWords) {
@@ -1488,10 +1501,16 @@ __global__ void __launch_bounds__(128 * NW, 1024 / (128 * NW)) km_cluster(KmBufs
       for (int w = tid; w < words; w += T) {
         int r = sm.pre[w];
 #pragma unroll 1
-        for (unsigned x = sm.bits[w]; x; x &= x - 1) run[r++] = (int)(lo + 32 * w + __ffs(x) - 1);
+        for (unsigned x = sm.bits[w]; x && r < left; x &= x - 1)
+          run[r++] = (int)(lo + 32 * w + __ffs(x) - 1);
       }
       run += sm.total;
+      left -= sm.total;
       __syncthreads();
+    }
+    if (left != 0) {                                   // the scans disagree: as above
+      if (tid == 0) st->bad_label = 1;
+      n = 0;
     }
   }
 #pragma unroll 1
@@ -1993,17 +2012,13 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
                                    cluster_smem));
   int* hflag = (int*)c->pinned;   // [2]: the done flag after a block of iterations
   const int kCheckEvery = 8;
-  // The two kernels of the summed-by-cluster form are chained (launch_chained), us a call: 670 ->
-  // 650 at N_g 4320, N_mu 48, 3160 -> 3110 at 110592, 256.  Letting the next kernel's blocks in
-  // before the last of this one's are done puts two km_cluster blocks on an SM where others
-  // have none: 3160-3190.
   // One k-means iteration; every kernel reads the iteration index from device state and
   // returns at once after convergence, so the same launch sequence serves any iteration.
   auto iteration = [&](bool prof) -> int {
     // The pruned assign counts the histogram itself (put_label); the scatter clears it.
     if (prune) {
       ProfScope p(prof ? c : nullptr, "km_assign");
-      if (by_cluster) THC_CUDA(c, launch_chained(km_assign_p<true>, nassign, kAssignThreads, prune_smem, s, b));
+      if (by_cluster) km_assign_p<true><<<nassign, kAssignThreads, prune_smem, s>>>(b);
       else km_assign_p<false><<<nassign, kAssignThreads, prune_smem, s>>>(b);
       THC_LAUNCHED(c, "km_assign_p");
     } else if (mixed) {
@@ -2022,7 +2037,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
       THC_LAUNCHED(c, "km_assign64");
     }
     if (by_cluster) {
-      THC_CUDA(c, launch_chained(cluster, nmu, cluster_threads, cluster_smem, s, b));
+      cluster<<<nmu, cluster_threads, cluster_smem, s>>>(b);
       THC_LAUNCHED(c, "km_cluster");
       return THC_OK;
     }
