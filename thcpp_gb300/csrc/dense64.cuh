@@ -74,8 +74,9 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
               double* dinv);
 // Cinv = (L L^T)^{-1} via X = L^{-1}; X (n x ld) and T (64 x n) are scratch.
 // With Cinv == nullptr only X = L^{-1} is formed.
+// tensor: X^T X may take the tensor-core route (other roundings than the FMA kernel's).
 int chol_inverse(Ctx* c, const double* L, long long ld, int n, const double* dinv, double* X,
-                 double* T, double* Cinv, const CholStatus* cs);
+                 double* T, double* Cinv, const CholStatus* cs, bool tensor = false);
 // Iterative refinement of a shifted solve, in closed form.  With L L^T = C + sI and
 // X = L^{-1} (n x n, ld n), k steps zeta_{j+1} = zeta_j + (C + sI)^{-1} (Z^T - C zeta_j)
 // from zeta_0 = (C + sI)^{-1} Z^T give zeta_k = X^T P X Z^T, P = sum_{j<=k} (s X X^T)^j

@@ -490,7 +490,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   // C^{-1} and zeta^T = C^{-1} Z^T.  With a shift and refinement steps, C^{-1} becomes
   // X^T P X (X = L^{-1}, P the refinement polynomial; refine_polynomial).
   const bool refining = shifted && c->refine > 0;
-  if ((st = chol_inverse(c, Lc, nmu, nmu, dinv, Xinv, Tinv, refining ? nullptr : Cinv, cs)))
+  if ((st = chol_inverse(c, Lc, nmu, nmu, dinv, Xinv, Tinv, refining ? nullptr : Cinv, cs, true)))
     return st;
   if (refining) {
     double hs = 0.0;
