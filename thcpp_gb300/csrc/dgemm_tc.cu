@@ -11,18 +11,18 @@
 //     C[m,n] = 2^{eA[m]+eB[n]-14} sum_{l<=7} 2^{-8l} V_l,   V_l = sum_{i+j=l} sum_k S_i T_j.
 // The tensor cores sum V_l in FP32, exactly for l <= 4: over the 192 k between two drains
 // |V_l| <= 5 192 2^14 < 2^24.  Levels 5 to 7 (weight <= 2^-40) could pass 2^24 only with
-// digits of one sign throughout, and then round by less than 2^-55 of the sum.  A drain adds the sums to integers in registers (two 64-bit words per element),
-// which hold the sum over any K without rounding, so C is the correctly rounded value of the
-// truncated expansion: about 2^-57 sqrt(K) off relative to 2^{eA+eB}, where a chain of FP64
-// FMAs over terms of that size is 2^-54 sqrt(K) and more.
+// digits of one sign throughout, and then round by less than 2^-55 of the sum.  A drain adds the
+// sums to 96-bit integers in registers, which hold the sum over any K without rounding, so C is
+// the correctly rounded value of the truncated expansion: about 2^-57 sqrt(K) off relative to
+// 2^{eA+eB}, where a chain of FP64 FMAs over terms of that size is 2^-54 sqrt(K) and more.
 //
 // Measured against the FMA kernel of dense64.cu, cut and product together (random operands;
 // errors relative to |a||b| of an entry's row and column, root mean square):
 //     M x N x K                     FMA              tensor cores
 //     256 x 110592 x 256            11.8 ms 3.4e-17  0.54 ms 3.7e-18   (27 TFLOP/s)
-//     256 x 110592 x 32, squared    1.54 ms 3.5e-17  0.22 ms 9.9e-18
-//     256 x 256 x 115200, lower     15.9 ms 2.6e-16  0.48 ms 9.5e-18
-//     1024 x 1024 x 215040, lower    340 ms 7.2e-16  6.7 ms 4.8e-18   (68 TFLOP/s)
+//     256 x 110592 x 32, squared    1.54 ms 3.5e-17  0.21 ms 9.9e-18
+//     256 x 256 x 115200, lower     15.9 ms 2.6e-16  0.47 ms 9.5e-18
+//     1024 x 1024 x 215040, lower    340 ms 7.2e-16  6.6 ms 4.8e-18   (69 TFLOP/s)
 // What bounds the product is shared memory: the eleven MMAs of 16 k read 112 KB and the copies
 // write 43 KB, 1211 clocks at 128 B, against 1088 of tensor work; without the drains 1350
 // clocks are measured, with them 1580.
@@ -95,9 +95,10 @@ __device__ __forceinline__ unsigned max8(const CutSrc& a, int k, const double (&
 template <bool SC>
 __device__ __forceinline__ void scale8(const CutSrc& a, int k, double (&v)[8])
 {
-  if (!SC) return;
+  if constexpr (SC) {
 #pragma unroll
-  for (int j = 0; j < 8; j++) v[j] *= scale_at(a, k + j);
+    for (int j = 0; j < 8; j++) v[j] *= scale_at(a, k + j);
+  }
 }
 
 // Short rows (K <= kFusedK, k contiguous or nearly): lpr lanes per row, eight columns per
