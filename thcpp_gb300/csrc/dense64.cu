@@ -12,6 +12,7 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "common.cuh"
 #include "dense64.cuh"
@@ -760,6 +761,50 @@ int refine_polynomial(Ctx* c, const double* X, int n, double s, int k, double* G
     if ((r = dgemm(c, g))) return r;
     cur = dst;
   }
+  return THC_OK;
+}
+
+namespace {
+
+__global__ void __launch_bounds__(1024) balance_exponents_k(const double* a, long long stride,
+                                                            int n, int* k, int* range)
+{
+  __shared__ int lo[32], hi[32];
+  int mn = INT_MAX, mx = INT_MIN;
+  for (int i = threadIdx.x; i < n; i += 1024) {
+    const double v = a[i * stride];
+    const int E = (__double2hiint(v) >> 20) & 0x7ff;
+    const bool use = E != 0x7ff && v != 0.0;
+    const int e = use ? (max(E, 1) - 1023) >> 1 : 0;
+    k[i] = e;
+    if (use) {
+      mn = min(mn, e);
+      mx = max(mx, e);
+    }
+  }
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) {
+    lo[threadIdx.x >> 5] = mn;
+    hi[threadIdx.x >> 5] = mx;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    mn = __reduce_min_sync(0xffffffffu, lo[threadIdx.x]);
+    mx = __reduce_max_sync(0xffffffffu, hi[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      range[0] = mn <= mx ? mn : 0;
+      range[1] = mn <= mx ? mx : 0;
+    }
+  }
+}
+
+}  // namespace
+
+int balance_exponents(Ctx* c, const double* a, long long stride, int n, int* k, int* range)
+{
+  balance_exponents_k<<<1, 1024, 0, c->stream>>>(a, stride, n, k, range);
+  THC_LAUNCHED(c, "balance_exponents");
   return THC_OK;
 }
 

@@ -23,6 +23,8 @@ struct GemmArgs {
   int dk_shift = 0;
   const double* dkr = nullptr;       // sqrt(dk), where A == B and no dk is negative: lets the
                                      // tensor-core route cut one operand for both sides
+  const int* kexp = nullptr;         // powers of two along k (K of them) that balance the operands'
+                                     // rows before they are cut: A(m, k) 2^kexp, B(n, k) 2^-kexp
   double alpha = 1.0, beta = 0.0;
   int mode = GEMM_STORE;
   int lower_only = 0;
@@ -84,6 +86,18 @@ int chol_inverse(Ctx* c, const double* L, long long ld, int n, const double* din
 // Xt = P X by Horner's rule in FP64 (k + 1 GEMMs of n^3); G and T are n x n scratch.
 int refine_polynomial(Ctx* c, const double* X, int n, double s, int k, double* G, double* T,
                       double* Xt);
+// The solve zeta = C^{-1} Z on the tensor cores.  C^{-1} scales as 1/d along k and Z as d,
+// d = sqrt(diag C): a row cut relative to its largest entry holds the entries of the other points
+// in few bits, and the error of zeta grows with d's range, from 10 on (two fragments of different
+// amplitude, N_g 43200, N_mu 140: M 3.8 times the FMA kernel's error at a range of 1.5e4, 87
+// times at 1.7e5).  So both operands are balanced by powers of two, 2^k_i = d_i to a factor of
+// two (GemmArgs::kexp, exact); over 42 such systems the error then is the FMA kernel's within 5 %
+// up to a range of 3e4, at 7e4 the smallest points' part of it is twice that.  Beyond
+// 2^kBalancedBinades the FMA kernel takes the product, and C^{-1} = X^T X.
+constexpr int kBalancedBinades = 13;
+// k_i = floor(log2 sqrt|a_i|) of n values a_i, `stride` doubles apart (0 where a_i is 0 or not
+// finite), and the smallest and the largest k_i of the others in range[0..1].
+int balance_exponents(Ctx* c, const double* a, long long stride, int n, int* k, int* range);
 int set_identity(Ctx* c, double* A, long long ld, int n);
 int add_diag_shift(Ctx* c, double* A, long long ld, int n, double rel, double* shift_out);
 int diag_mean(Ctx* c, const double* A, long long ld, int n, double* out);

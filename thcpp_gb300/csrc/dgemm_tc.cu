@@ -82,29 +82,53 @@ __device__ __forceinline__ double scale_at(const CutSrc& a, int k)
   return k < a.K ? __ldg(a.scale + ((a.k0 + k) >> a.shift)) : 0.0;
 }
 
+__device__ __forceinline__ int shift_at(const CutSrc& a, int k)
+{
+  return k < a.K ? a.ksign * __ldg(a.kexp + a.k0 + k) : 0;
+}
+
+// The row maximum's contribution of x at column k.
+template <CutScale SC>
+__device__ __forceinline__ unsigned field_at(const CutSrc& a, int k, double x)
+{
+  if constexpr (SC == CUT_SCALED) return (unsigned)field_of(x, scale_at(a, k));
+  if constexpr (SC == CUT_SHIFTED) return field_shifted(x, shift_at(a, k));
+  return abs_hi(x);
+}
+
 // The maximum's contribution of eight columns.
-template <bool SC>
+template <CutScale SC>
 __device__ __forceinline__ unsigned max8(const CutSrc& a, int k, const double (&v)[8], unsigned mx)
 {
 #pragma unroll
-  for (int j = 0; j < 8; j++)
-    mx = max(mx, SC ? (unsigned)field_of(v[j], scale_at(a, k + j)) : abs_hi(v[j]));
+  for (int j = 0; j < 8; j++) mx = max(mx, field_at<SC>(a, k + j, v[j]));
   return mx;
 }
 
-template <bool SC>
+template <CutScale SC>
 __device__ __forceinline__ void scale8(const CutSrc& a, int k, double (&v)[8])
 {
-  if constexpr (SC) {
+  if constexpr (SC == CUT_SCALED) {
 #pragma unroll
     for (int j = 0; j < 8; j++) v[j] *= scale_at(a, k + j);
   }
 }
 
+// Columns k .. k + 7 of row r, scaled already, as digits relative to 2^e.
+template <CutScale SC>
+__device__ __forceinline__ void cut8(const CutSrc& a, const Digits& o, long long r, int k, int e,
+                                     const double (&v)[8])
+{
+  if constexpr (SC == CUT_SHIFTED)
+    store8(o, r, k, 1022 + e, v, [&](int j) { return shift_at(a, k + j); });
+  else
+    store8(o, r, k, 1022 + e, v);
+}
+
 // Short rows (K <= kFusedK, k contiguous or nearly): lpr lanes per row, eight columns per
 // lane and step, the row read twice (the second time from L1/L2).
 constexpr int kFusedK = 4096;
-template <bool SC>
+template <CutScale SC>
 __global__ void __launch_bounds__(256) cut_rows(CutSrc a, Digits o, int lpr, int* flag)
 {
   const int lane = threadIdx.x & 31, sub = lane & (lpr - 1);
@@ -134,14 +158,14 @@ __global__ void __launch_bounds__(256) cut_rows(CutSrc a, Digits o, int lpr, int
 #pragma unroll
       for (int j = 0; j < 8; j++) v[j] = 0.0;
     }
-    store8(o, r, k, 1022 + e, v);
+    cut8<SC>(a, o, r, k, e, v);
   }
 }
 
 // Long rows (the Coulomb product's K = 2 N_c): row maxima by column chunks, then the digits,
 // each with the whole GPU on a few rows.
 constexpr int kMaxChunk = 4096;
-template <bool SC>
+template <CutScale SC>
 __global__ void __launch_bounds__(256) cut_rowmax(CutSrc a, int nch, unsigned* rowmax)
 {
   const long long r = blockIdx.x / nch;
@@ -156,7 +180,7 @@ __global__ void __launch_bounds__(256) cut_rowmax(CutSrc a, int nch, unsigned* r
   if ((threadIdx.x & 31) == 0 && mx) atomicMax(&rowmax[r], mx);
 }
 
-template <bool SC>
+template <CutScale SC>
 __global__ void __launch_bounds__(256) cut_long(CutSrc a, Digits o, int nch,
                                                 const unsigned* __restrict__ rowmax, int* flag)
 {
@@ -175,14 +199,14 @@ __global__ void __launch_bounds__(256) cut_long(CutSrc a, Digits o, int nch,
     load8(a, r, k, v);
     scale8<SC>(a, k, v);
   }
-  store8(o, r, k, 1022 + e, v);
+  cut8<SC>(a, o, r, k, e, v);
 }
 
 // Row-contiguous operands (sr == 1: Z^T, N_mu x N_g, as the B of the zeta product): a block
 // owns 64 rows; the maximum's pass reads coalesced along the rows, the second pass turns
 // 32 k x 64 rows at a time through shared memory.
 constexpr int kTR = 64;
-template <bool SC>
+template <CutScale SC>
 __global__ void __launch_bounds__(256) cut_cols(CutSrc a, Digits o, int* flag)
 {
   __shared__ unsigned smx[4][kTR];
@@ -197,7 +221,7 @@ __global__ void __launch_bounds__(256) cut_cols(CutSrc a, Digits o, int* flag)
 #pragma unroll 8
     for (int k = w; k < a.K; k += 4) {
       const double x = __ldg(col + k * a.sk);
-      mx = max(mx, SC ? (unsigned)field_of(x, scale_at(a, k)) : abs_hi(x));
+      mx = max(mx, field_at<SC>(a, k, x));
     }
   smx[w][rr] = mx;
   __syncthreads();
@@ -217,7 +241,7 @@ __global__ void __launch_bounds__(256) cut_cols(CutSrc a, Digits o, int* flag)
       double x = 0.0;
       if (live && k < a.K) {
         x = __ldg(col + k * a.sk);
-        if (SC) x *= scale_at(a, k);
+        if (SC == CUT_SCALED) x *= scale_at(a, k);
       }
       t[w + 4 * q][rr] = x;
     }
@@ -225,7 +249,7 @@ __global__ void __launch_bounds__(256) cut_cols(CutSrc a, Digits o, int* flag)
     double v[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) v[j] = t[oc + j][orow];
-    store8(o, r0 + orow, kt + oc, 1022 + se[orow], v);
+    cut8<SC>(a, o, r0 + orow, kt + oc, se[orow], v);
   }
 }
 
@@ -721,7 +745,7 @@ int digit_map(Ctx* c, CUtensorMap* map, const Digits& d, int box_rows)
   return THC_OK;
 }
 
-template <bool SC>
+template <CutScale SC>
 int cut_operand_t(Ctx* c, const CutSrc& a, const Digits& d, unsigned* rowmax, int* flag)
 {
   cudaStream_t s = c->stream;
@@ -752,8 +776,9 @@ int cut_operand_t(Ctx* c, const CutSrc& a, const Digits& d, unsigned* rowmax, in
 int digits_cut(Ctx* c, const CutSrc& a, const Digits& d, unsigned* rowmax, int* flag)
 {
   ProfScope prof(c, "slice64");
-  return a.scale ? cut_operand_t<true>(c, a, d, rowmax, flag)
-                 : cut_operand_t<false>(c, a, d, rowmax, flag);
+  return a.scale  ? cut_operand_t<CUT_SCALED>(c, a, d, rowmax, flag)
+         : a.kexp ? cut_operand_t<CUT_SHIFTED>(c, a, d, rowmax, flag)
+                  : cut_operand_t<CUT_PLAIN>(c, a, d, rowmax, flag);
 }
 
 int digits_product(Ctx* c, const Digits& a, const Digits& b, const GemmArgs& g)
@@ -817,7 +842,7 @@ int digits_product(Ctx* c, const Digits& a, const Digits& b, const GemmArgs& g)
 
 bool dgemm_tc_fits(const Ctx* c, const GemmArgs& g)
 {
-  if (!c->gemm_tc || g.fma_only || g.skip_flag || g.a_zero_below || g.b_zero_below ||
+  if (!c->gemm_tc || g.fma_only || (g.kexp && g.dk) || g.skip_flag || g.a_zero_below || g.b_zero_below ||
       g.lower_offset || g.no_split || g.ksplit > 1 || g.part || (g.lower_only && g.M != g.N))
     return false;
   return 2.0 * (double)g.M * (double)g.N * (double)g.K >= kDgemmTcFlops && g.K >= 8;
@@ -830,7 +855,7 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
   const double* dkr = g.dkr;
   // One buffer of digits serves both operands of a symmetric product.
   const bool same = g.A == g.B && g.sam == g.sbn && g.sak == g.sbk && g.M == g.N &&
-                    (!g.dk || dkr);
+                    (!g.dk || dkr) && !g.kexp;
   // Panels: of N while A's digits and a panel of B's fit the budget, else of K (C accumulated
   // in FP64 over the panels).
   const size_t per = kNS * sizeof(__nv_bfloat16);
@@ -873,7 +898,7 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
     THC_CUDA(c, cudaMemsetAsync(nonfin, 0, sizeof(int), c->stream));
     {
       CutSrc a{g.A, g.M, g.sam, g.sak, k0, K, same ? dkr : g.dk, g.dk_shift,
-               vec(g.A, g.sam, g.sak)};
+               vec(g.A, g.sam, g.sak), g.kexp, 1};
       if ((st = digits_cut(c, a, da, rowmax, nonfin))) return st;
     }
     for (long long n0 = 0; n0 < g.N; n0 += npan) {
@@ -887,7 +912,7 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
       } else {
         db.rows_pad = oz_pad_mn(p.N);
         db.e = eb_own;
-        CutSrc b{p.B, p.N, g.sbn, g.sbk, k0, K, nullptr, 0, vec(p.B, g.sbn, g.sbk)};
+        CutSrc b{p.B, p.N, g.sbn, g.sbk, k0, K, nullptr, 0, vec(p.B, g.sbn, g.sbk), g.kexp, -1};
         if ((st = digits_cut(c, b, db, rowmax, nonfin))) return st;
       }
       if ((st = digits_product(c, da, db, p))) return st;

@@ -27,11 +27,27 @@ __device__ __forceinline__ int field_of(double x, double s)
   return (ex == 0x7ff || es == 0x7ff) ? kNonFinite : ex + es;
 }
 
-// e from the maximum of abs_hi (plain rows) or of field_of (scaled rows).
-template <bool SC>
+// The exponent field of x 2^h, biased: 0 for x = 0 only.
+constexpr int kShiftBias = 4096;         // |h| < 2^11
+__device__ __forceinline__ unsigned field_shifted(double x, int h)
+{
+  const unsigned a = abs_hi(x), E = a >> 20;
+  if (E == 0x7ff) return kNonFinite;
+  if ((a | (unsigned)__double2loint(x)) == 0) return 0;
+  return (unsigned)((int)max(E, 1u) + h + kShiftBias);
+}
+
+// What multiplies an operand along k: nothing, doubles (CutSrc::scale), or powers of two
+// (CutSrc::kexp).
+enum CutScale { CUT_PLAIN, CUT_SCALED, CUT_SHIFTED };
+
+// e from the maximum of abs_hi (plain rows), of field_of (scaled rows) or of field_shifted.
+template <CutScale SC>
 __device__ __forceinline__ int row_exponent(unsigned mx)
 {
-  if (SC) return (int)mx - 2044 > 1024 ? kNonFinite : max((int)mx - 2044, -1021);
+  if (SC == CUT_SHIFTED)
+    return mx == (unsigned)kNonFinite ? kNonFinite : mx ? (int)mx - kShiftBias - 1022 : -1021;
+  if (SC == CUT_SCALED) return (int)mx - 2044 > 1024 ? kNonFinite : max((int)mx - 2044, -1021);
   const int E = (int)(mx >> 20);
   return E == 0x7ff ? kNonFinite : max(E, 1) - 1022;
 }
@@ -76,13 +92,14 @@ struct Digits {
   long long rows_pad = 0, kpad = 0;
 };
 
-// Cuts columns k .. k + 7 of row r: one 16-byte store per digit.
+// Cuts columns k .. k + 7 of row r, column k + j times 2^h[j]: one 16-byte store per digit.
+template <class H>
 __device__ __forceinline__ void store8(const Digits& o, long long r, long long k, int base,
-                                       const double (&v)[8])
+                                       const double (&v)[8], H h)
 {
   unsigned lo[8], hi[8];
 #pragma unroll
-  for (int j = 0; j < 8; j++) cut(v[j], base, lo[j], hi[j]);
+  for (int j = 0; j < 8; j++) cut(v[j], base - h(j), lo[j], hi[j]);
   __nv_bfloat16* p = o.s + (k >> 5) * (kNS * o.rows_pad * 32) + r * 32 + (k & 31);
   const long long step = o.rows_pad * 32;
   unsigned w[4];
@@ -105,14 +122,22 @@ __device__ __forceinline__ void store8(const Digits& o, long long r, long long k
   }
 }
 
+__device__ __forceinline__ void store8(const Digits& o, long long r, long long k, int base,
+                                       const double (&v)[8])
+{
+  store8(o, r, k, base, v, [](int) { return 0; });
+}
+
 // Where an operand's element (row r, index k) lies and what multiplies it.
 struct CutSrc {
   const double* x;
   long long rows, sr, sk;    // x[r sr + k sk]
   int k0, K;                 // the panel's first k and its length
-  const double* scale;       // SC: indexed (k0 + k) >> shift
+  const double* scale;       // CUT_SCALED: indexed (k0 + k) >> shift
   int shift;
   bool vec;                  // sk == 1, rows 16-byte aligned
+  const int* kexp = nullptr; // CUT_SHIFTED: x 2^{ksign kexp[k0 + k]}
+  int ksign = 1;
 };
 
 // Digits of one operand's panel (k0, K) into d; flag (device) is set if a row is not finite.

@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) cut_slab(SlabSrc a, Digits o, int* flag)
   __syncthreads();
   if (threadIdx.x < kTR) {
     for (int q = 1; q < 4; q++) mx = max(mx, smx[q][rr]);
-    const int e = row_exponent<false>(mx);
+    const int e = row_exponent<CUT_PLAIN>(mx);
     se[rr] = e;
     o.e[r] = e;
     if (e == kNonFinite) atomicExch(flag, 1);

@@ -331,6 +331,14 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   // C^{-1} by Gauss-Jordan elimination on [C | I].
   build_augmented<<<(int)cdiv(2 * nn, 256), 256, 0, s>>>(pr, pi, ng, idx, nmu, aug);
   THC_LAUNCHED(c, "build_augmented");
+  int* bal = (int*)ws_get(c, WS_EQUIL, sizeof(int) * 2 * nmu);
+  if (!bal) return set_error(c, THC_ERR_NOMEM, "thc_isdf_half_complex: workspace allocation failed");
+  int* bal_range = bad + 1;
+  if ((st = balance_exponents(c, aug, 4LL * nmu + 2, nmu, bal, bal_range))) return st;
+  THC_CUDA(c, cudaMemcpyAsync(bal + nmu, bal, sizeof(int) * nmu, cudaMemcpyDeviceToDevice, s));
+  int* h_range = (int*)c->pinned;
+  THC_CUDA(c, cudaMemcpyAsync(h_range, bal_range, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  THC_CUDA(c, cudaEventRecord(c->ev_fork, s));
   // The fewest rows a thread whose blocks the 152 SMs hold at once, eight each.
   int gr = 1;
   while (gr < 8 && cdiv(nmu, 4 * gr) * cdiv(2 * nmu, kGjCols) > 152 * 8) gr *= 2;
@@ -352,6 +360,9 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
     g.M = 2LL * nmu; g.N = ng; g.K = 2 * nmu;
     g.A = ci; g.sam = 2LL * nmu; g.sak = 1;
     g.B = prpi; g.sbn = 1; g.sbk = ng;
+    g.kexp = bal;
+    THC_CUDA(c, cudaEventSynchronize(c->ev_fork));   // long past, behind the elimination's launches
+    g.fma_only = h_range[1] - h_range[0] > kBalancedBinades;
     g.C = qrqi; g.ldc = ng;
     if ((st = dgemm(c, g))) return st;
   }

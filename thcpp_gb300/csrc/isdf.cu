@@ -339,6 +339,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   int* bad = (int*)(scr + 512);
   int* n_anti = bad + 1;
   int* n_neg = bad + 2;
+  int* bal_range = bad + 3;
   double* droot = dsym + nc;
   // Orbital outputs: written in place on the device, else staged for the host copy.
   double* orb_dev = nullptr;
@@ -362,7 +363,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   coulomb_weights<<<(int)cdiv(nc, 256), 256, 0, s>>>(coul, n0, n1, n2, dsym, danti, droot, n_anti,
                                                      n_neg, fft_products);
   THC_LAUNCHED(c, "coulomb_weights");
-  int h_counts[2] = {0, 0};            // n_anti, n_neg
+  int h_counts[4] = {0, 0, 0, 0};      // n_anti, n_neg, the smallest and largest exponent of C's
   gather_rows<<<(int)cdiv((long long)nmu * kw, 256), 256, 0, s>>>(phi, ng, kw, idx, nmu, phimu,
                                                                   cplx ? nullptr : orb_dev, bad);
   THC_LAUNCHED(c, "gather_rows");
@@ -451,6 +452,9 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
     hadamard_k<<<(int)cdiv((long long)nmu * ng, 256), 256, 0, s>>>(zt, ng, zeta, ng, nmu, ng);
     THC_LAUNCHED(c, "hadamard");
   }
+  int* bal = (int*)ws_get(c, WS_EQUIL, sizeof(int) * nmu);
+  if (!bal) return set_error(c, THC_ERR_NOMEM, "thc_isdf: workspace allocation failed");
+  if ((st = balance_exponents(c, C, nmu + 1, nmu, bal, bal_range))) return st;
   // Cholesky of C with breakdown detection, then the shift policy.
   double* Lc = C + nn;
   if ((st = diag_mean(c, C, nmu, nmu, dmean))) return st;
@@ -490,7 +494,8 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   // C^{-1} and zeta^T = C^{-1} Z^T.  With a shift and refinement steps, C^{-1} becomes
   // X^T P X (X = L^{-1}, P the refinement polynomial; refine_polynomial).
   const bool refining = shifted && c->refine > 0;
-  if ((st = chol_inverse(c, Lc, nmu, nmu, dinv, Xinv, Tinv, refining ? nullptr : Cinv, cs, true)))
+  const bool graded = h_counts[3] - h_counts[2] > kBalancedBinades;   // dense64.cuh
+  if ((st = chol_inverse(c, Lc, nmu, nmu, dinv, Xinv, Tinv, refining ? nullptr : Cinv, cs, !graded)))
     return st;
   if (refining) {
     double hs = 0.0;
@@ -513,6 +518,8 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
     g.M = nmu; g.N = ng; g.K = nmu;
     g.A = Cinv; g.sam = nmu; g.sak = 1;
     g.B = zt; g.sbn = 1; g.sbk = ng;
+    g.kexp = bal;
+    g.fma_only = graded;
     g.C = zeta; g.ldc = ng;
     if ((st = dgemm(c, g))) return st;
   }
