@@ -70,3 +70,15 @@ def test_singular_c_without_shift(gpu_ctx_fp64, gpu_ctx_mixed, prec):
     assert "Cholesky of C failed" in ctx.lib.thc_ctx_last_error(ctx.h).decode()
     r = ctx.isdf(s.phi, idx, s.mesh, s.coulG)
     assert r["status"] == capi.THC_OK and r["stats"].rank_deficient == 1
+
+
+@pytest.mark.parametrize("bad", [-1, 1000])
+def test_index_outside_the_grid(gpu_ctx_fp64, bad):
+    """An interpolating index that is no grid point is reported, and never used as an address."""
+    r = np.random.default_rng(1)
+    phi = r.standard_normal((1000, 6)) + 1j * r.standard_normal((1000, 6))
+    idx = np.array([3, 500, bad, 800], dtype=np.int32)
+    with pytest.raises(capi.ThcError, match="interpolating index out of range") as e:
+        gpu_ctx_fp64.isdf_half_complex(phi, np.ascontiguousarray(phi[:, :3]), idx, (10, 10, 10),
+                                       np.ones(1000))
+    assert e.value.status == capi.THC_ERR_ARG

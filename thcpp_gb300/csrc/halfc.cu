@@ -78,8 +78,10 @@ __global__ void build_augmented(const double* __restrict__ zr, const double* __r
   double re = 0.0, im = 0.0;
   if (c < n) {
     const long long g = idx[c];
-    re = zr[(long long)r * ng + g];
-    im = zi[(long long)r * ng + g];
+    if (g >= 0 && g < ng) {                            // gather_pairs has reported the others
+      re = zr[(long long)r * ng + g];
+      im = zi[(long long)r * ng + g];
+    }
   } else {
     re = (c - n == r) ? 1.0 : 0.0;
   }
