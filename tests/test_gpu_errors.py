@@ -41,6 +41,43 @@ def test_device_wait_timeout_is_reported_and_context_stays_usable(gpu_ctx_mixed)
     assert _rel(_cplx(r["M"]), ref["M"]) < 1e-6
 
 
+def _noise(mesh, norb, nmu, cplx=False):
+    r = np.random.default_rng(norb + nmu)
+    ng = int(np.prod(mesh))
+    phi = r.standard_normal((ng, norb))
+    if cplx:
+        phi = phi + 1j * r.standard_normal((ng, norb))
+    idx = np.sort(r.choice(ng, nmu, replace=False)).astype(np.int32)
+    return phi, idx, np.ones(ng)
+
+
+# The products on the tensor cores: from C's on (2 N_mu^2 N_o >= 4e7, the one whose result the
+# call judges half-way), from Z's on, and with the transforms (N_g N_mu >= 1e6) as products too.
+@pytest.mark.parametrize("kind,mesh,norb,nmu", [
+    ("real", (16, 16, 20), 64, 640), ("real", (16, 16, 18), 24, 96), ("real", (20, 24, 25), 24, 96),
+    ("half", (16, 16, 20), 64, 640), ("complex", (16, 16, 20), 40, 640),
+    ("half_complex", (20, 24, 25), 24, 96)])
+def test_fp64_device_wait_timeout(gpu_ctx_fp64, kind, mesh, norb, nmu):
+    ctx = gpu_ctx_fp64
+    phi, idx, v = _noise(mesh, norb, nmu, "complex" in kind)
+    occ = np.ascontiguousarray(phi[:, :norb // 2])
+    call = {"real": lambda: ctx.isdf(phi, idx, mesh, v),
+            "half": lambda: ctx.isdf_half(phi, occ, idx, mesh, v),
+            "complex": lambda: ctx.isdf_complex(phi, idx, mesh, v),
+            "half_complex": lambda: ctx.isdf_half_complex(phi, occ, idx, mesh, v)}[kind]
+    before = call()["M"].copy()
+    # Stale workspace: another call's C, Z and zeta, which the next one must not take for its own.
+    ctx.isdf(*_noise(mesh, 8, 30)[:2], mesh, v)
+    ctx.set_option("spin_limit", 0)
+    try:
+        with pytest.raises(capi.ThcError, match="timed out") as e:
+            call()
+        assert e.value.status == capi.THC_ERR_TIMEOUT
+    finally:
+        ctx.set_option("spin_limit", 1 << 24)
+    assert np.array_equal(call()["M"], before)
+
+
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 def test_m_not_positive_definite(gpu_ctx_fp64, gpu_ctx_mixed, prec):
     """A negative Coulomb kernel makes M negative definite: THC_ERR_NOT_PD with the failed

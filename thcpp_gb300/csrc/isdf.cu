@@ -364,6 +364,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
                                                      n_neg, fft_products);
   THC_LAUNCHED(c, "coulomb_weights");
   int h_counts[4] = {0, 0, 0, 0};      // n_anti, n_neg, the smallest and largest exponent of C's
+  int herr = 0;                        // a product of C or Z gave up waiting
   gather_rows<<<(int)cdiv((long long)nmu * kw, 256), 256, 0, s>>>(phi, ng, kw, idx, nmu, phimu,
                                                                   cplx ? nullptr : orb_dev, bad);
   THC_LAUNCHED(c, "gather_rows");
@@ -478,8 +479,11 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   if ((st = factor(shift_rel > 0.0 ? shift_rel : 0.0))) return st;
   shifted = shift_rel > 0.0;
   THC_CUDA(c, cudaMemcpyAsync(h_counts, n_anti, sizeof(h_counts), cudaMemcpyDeviceToHost, s));
+  THC_CUDA(c, cudaMemcpyAsync(&herr, c->tc64_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hcs, cs, sizeof(CholStatus), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaStreamSynchronize(s));
+  // Before C is judged: without its product C is whatever the workspace held.
+  if (herr) return set_error(c, THC_ERR_TIMEOUT, "thc_isdf: tensor-core GEMM wait timed out");
   if (hcs.flag) {
     chol_c_info = hcs.info;
     if (shift_rel < 0.0 && !shifted) {
@@ -581,7 +585,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   if (out_L && !half)
     THC_CUDA(c, cudaMemcpyAsync(out_L, Lout, sizeof(double) * 2 * nn, cudaMemcpyDefault, s));
   CholStatus hm{};
-  int hbad = 0, herr = 0;
+  int hbad = 0;
   THC_CUDA(c, cudaMemcpyAsync(&herr, c->tc64_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hm, csm, sizeof(CholStatus), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
