@@ -101,7 +101,10 @@ int thc_ctx_set_stream(thc_ctx* ctx, void* cuda_stream);
 /* Named numeric options: "slices_p", "slices_z", "slices_m" (sliced-GEMM depths of the
  * P, zeta and Coulomb products, 2..6); "gemm_tc" (1 = tcgen05 tensor-core kernels, the
  * default; 0 = warp-level mma.sync kernel, and FP64 FMAs for the FP64 products); "km_prune" (1 = spatially pruned k-means
- * assignment, the default; 0 = exhaustive scan -- both exact); "graphs" (1 = replay the
+ * assignment, the default; 0 = exhaustive scan -- both exact); "digits_mb" (FP64 products and
+ * transforms on the tensor cores: most workspace for their digits in MiB, default 3072; larger
+ * products run in panels, 0 leaves them to the FP64 FMAs and cuFFT, as does a workspace that
+ * cannot be allocated); "graphs" (1 = replay the
  * k-means iteration block as a CUDA graph, the default); "tc_bk" (k-step per
  * pipeline stage of the tensor-core kernel: 32, the default, or 16; setting it turns the
  * autotuner off); "tc_bn" (tile width of the tensor-core kernel: 128, the default, or 64

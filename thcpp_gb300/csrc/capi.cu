@@ -39,6 +39,15 @@ void* ws_get(Ctx* c, Slot s, size_t bytes)
     cudaGetLastError();
     if (cudaMallocAsync(&p, bytes, c->stream) != cudaSuccess) {
       cudaGetLastError();
+      // The digits of the FP64 tensor-core products are optional: what asks for anything else than
+      // they and what is used with them holds no pointer to them.
+      if (s != WS_T64_A && s != WS_T64_B && s != WS_T64_E && s != WS_DPART && s != WS_FFTWORK)
+        for (Slot t : {WS_T64_A, WS_T64_B})
+          if (c->ws[t]) {
+            cudaFreeAsync(c->ws[t], c->stream);
+            c->ws[t] = nullptr;
+            c->ws_bytes[t] = 0;
+          }
       // The pool keeps freed memory reserved (release threshold = max), possibly in pieces
       // too small for this request: return what no allocation uses and try once more.
       // The whole device first: trimming may then release nothing that a kernel of another
@@ -322,6 +331,11 @@ int thc_ctx_set_option(thc_ctx* h, const char* key, double value)
   }
   if (!strcmp(key, "overlap")) {
     h->c.overlap = value != 0.0;
+    return THC_OK;
+  }
+  if (!strcmp(key, "digits_mb")) {
+    if (value < 0 || value > 1 << 20) return THC_ERR_ARG;
+    h->c.digit_bytes = (size_t)(value * 1048576.0);
     return THC_OK;
   }
   if (!strcmp(key, "spin_limit")) {

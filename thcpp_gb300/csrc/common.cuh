@@ -110,6 +110,9 @@ struct Ctx {
   int slices_m = 5;
   // 1: tcgen05 GEMMs; 0: mma.sync sliced GEMM (mixed path) and FP64 FMAs (dgemm).
   int gemm_tc = 1;
+  // Most bytes of digits a product of dgemm's tensor-core route holds at a time (larger ones run
+  // in panels); a quarter of it for a chunk of fft_tc's.  0: neither.
+  size_t digit_bytes = (size_t)3 << 30;
   int* tc64_err = nullptr;   // device flag: a bounded wait of dgemm's tensor-core route gave up
   int km_prune = 1;     // 1: spatially pruned k-means assign, 0: exhaustive
   int use_graphs = 1;   // capture the k-means iteration block in a CUDA graph

@@ -60,7 +60,6 @@ int dgemm(Ctx* c, const GemmArgs& g);
 // against 36; 130 x 130 x 1000, 3.4e7: 52 against 46; 130 x 200 x 1000 row-contiguous, 5.2e7:
 // 80 against 85; 256 x 4096 x 32, 6.7e7: 73 against 31).
 constexpr double kDgemmTcFlops = 4e7;
-constexpr size_t kDgemmTcBytes = (size_t)3 << 30;   // digit buffers: larger products run in panels
 bool dgemm_tc_fits(const Ctx* c, const GemmArgs& g);
 // Runs g on the tensor cores; *done = false (and THC_OK) when it does not take it (no room
 // for the digits), and the caller runs the FMA kernel.

@@ -857,9 +857,10 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
   const bool same = g.A == g.B && g.sam == g.sbn && g.sak == g.sbk && g.M == g.N &&
                     (!g.dk || dkr) && !g.kexp;
   // Panels: of N while A's digits and a panel of B's fit the budget, else of K (C accumulated
-  // in FP64 over the panels).
+  // in FP64 over the panels).  A product whose smallest panels (128 columns of B, 512 k) pass the
+  // budget is not taken.
   const size_t per = kNS * sizeof(__nv_bfloat16);
-  const size_t budget = kDgemmTcBytes;
+  const size_t budget = c->digit_bytes;
   long long npan = np;
   int kpan = (int)kp;
   if (!same && !g.lower_only && (size_t)(mp + np) * kp * per > budget &&
@@ -872,7 +873,7 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
   if (kpan < kp && g.mode == GEMM_SQUARE) return THC_OK;   // the square needs the whole sum
   const size_t abytes = (size_t)mp * kpan * per, bbytes = same ? 0 : (size_t)npan * kpan * per;
   // Coordinates and launch sizes are 32-bit.
-  if (abytes + bbytes > 4 * budget || mp > 0x7fffff00LL || np > 0x7fffff00LL ||
+  if (abytes + bbytes > budget || mp > 0x7fffff00LL || np > 0x7fffff00LL ||
       (mp / TBM) * (npan / kBN) > 1 << 22)
     return THC_OK;
   char* flags = (char*)ws_get(c, WS_T64_E, 256 + sizeof(int) * (mp + npan) +

@@ -375,10 +375,11 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   double* ivg = spec;
   double* left1 = spec + 2 * nmg;
   double* left2 = prpi;              // after the transform
-  const bool fft_products = fft_tc_fits(c, mesh[0], mesh[1], mesh[2], nmu);
-  if (fft_products) {
-    if ((st = fft_tc(c, mesh[0], mesh[1], mesh[2], nmu, false, zc, ivg))) return st;
-  } else {
+  bool fft_products = false;
+  if (fft_tc_fits(c, mesh[0], mesh[1], mesh[2], nmu) &&
+      (st = fft_tc(c, mesh[0], mesh[1], mesh[2], nmu, false, zc, ivg, &fft_products)))
+    return st;
+  if (!fft_products) {
     ProfScope prof(c, "fft");
     for (int f0 = 0; f0 < nmu; f0 += kFftChunk) {
       const int nb = std::min(kFftChunk, nmu - f0);

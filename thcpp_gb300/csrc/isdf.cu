@@ -359,10 +359,14 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
 
   // The Coulomb weights depend on the kernel only: with them first, their counts reach the
   // host with C's factorisation status and cost no wait of their own.
+  auto weights = [&](bool zyx) -> int {
+    coulomb_weights<<<(int)cdiv(nc, 256), 256, 0, s>>>(coul, n0, n1, n2, dsym, danti, droot,
+                                                       n_anti, n_neg, zyx);
+    THC_LAUNCHED(c, "coulomb_weights");
+    return THC_OK;
+  };
   const bool fft_products = fft_tc_fits(c, n0, n1, n2, nmu);
-  coulomb_weights<<<(int)cdiv(nc, 256), 256, 0, s>>>(coul, n0, n1, n2, dsym, danti, droot, n_anti,
-                                                     n_neg, fft_products);
-  THC_LAUNCHED(c, "coulomb_weights");
+  if ((st = weights(fft_products))) return st;
   int h_counts[4] = {0, 0, 0, 0};      // n_anti, n_neg, the smallest and largest exponent of C's
   int herr = 0;                        // a product of C or Z gave up waiting
   gather_rows<<<(int)cdiv((long long)nmu * kw, 256), 256, 0, s>>>(phi, ng, kw, idx, nmu, phimu,
@@ -528,9 +532,12 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
     if ((st = dgemm(c, g))) return st;
   }
   // FFT of every interpolating vector.
-  if ((st = fft_products ? fft_tc(c, n0, n1, n2, nmu, true, zeta, zhat)
-                         : fft_forward(c, n0, n1, n2, nmu, CUFFT_D2Z, zeta, zhat)))
-    return st;
+  bool transformed = false;
+  if (fft_products) {
+    if ((st = fft_tc(c, n0, n1, n2, nmu, true, zeta, zhat, &transformed))) return st;
+    if (!transformed && (st = weights(false))) return st;    // the order of cuFFT's spectra
+  }
+  if (!transformed && (st = fft_forward(c, n0, n1, n2, nmu, CUFFT_D2Z, zeta, zhat))) return st;
   const int h_anti = h_counts[0];
   // Re M (lower) = sum_k zh[mu,k] dsym[k/2] zh[nu,k] over interleaved (re, im) pairs.
   double* mre = Mw;
