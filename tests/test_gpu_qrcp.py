@@ -89,3 +89,50 @@ def test_qrcp_complex(gpu_ctx_fp64, name, npts):
     assert np.max(np.abs(r["diag"] - ref["diag"])) <= 1e-10 * ref["diag"][0]
     assert np.array_equal(r["order"], ref["order"])
     assert np.array_equal(r["idx"], ref["idx"])
+
+
+def _fma(a, b, c):
+    from fractions import Fraction
+    return float(Fraction(a) * Fraction(b) + Fraction(c))
+
+
+def _sequential(phi, fused):
+    """Three steps of the pivoted form for two orbitals.  fused: G - sum with G = g g unrounded
+    (a compiler's choice)."""
+    x = [[float(v) for v in row] for row in phi]
+    n = len(x)
+
+    def dot(a, b):
+        return _fma(a[1], b[1], a[0] * b[0])
+
+    d, low, order, diag = [dot(a, a) * dot(a, a) for a in x], [], [], []
+    for k in range(3):
+        p = max(range(n), key=lambda a: (d[a], -a))
+        root = float(np.sqrt(d[p]))
+        order.append(p)
+        diag.append(root)
+        col = []
+        for a in range(n):
+            s, g = 0.0, dot(x[a], x[p])
+            for lk in low:
+                s = _fma(lk[a], lk[p], s)
+            col.append((_fma(g, g, -s) if fused else g * g - s) / root)
+            d[a] = -np.inf if a in order else _fma(-col[a], col[a], d[a])
+        low.append(col)
+    return order, diag
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -230, 2.0 ** 230])
+def test_qrcp_rounding(gpu_ctx_fp64, scale):
+    """Every rounding as in the sequential form: a column of L is a correctly rounded quotient by
+    the root of the pivot's residual (also where it leaves the range in which the quotient comes
+    from the reciprocal)."""
+    same = {False: 0, True: 0}
+    for seed in range(24):
+        phi = np.random.default_rng(seed).standard_normal((300, 2)) * scale
+        phi[5] = 0.0
+        got = gpu_ctx_fp64.qrcp(phi, 3)
+        for fused in same:
+            order, diag = _sequential(phi, fused)
+            same[fused] += list(got["order"]) == order and list(got["diag"]) == diag
+    assert max(same.values()) == 24

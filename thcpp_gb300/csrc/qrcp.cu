@@ -119,8 +119,8 @@ __device__ QrPiv block_argmax(long long v, int a)
 }
 
 // Publishes the block's candidate; the last block to finish reduces all of them into
-// piv[k] / dpiv[k] and the reciprocal root of the residual rpiv[k], and re-arms the ticket for
-// the next launch.
+// piv[k] / dpiv[k] and the reciprocal root of the residual and the root, rpiv[2 k] and [2 k + 1],
+// and re-arms the ticket for the next launch.
 __device__ void finish_argmax(QrPiv mine, QrPiv* blk, unsigned* ticket, int* piv,
                               double* dpiv, double* rpiv, int k)
 {
@@ -145,7 +145,9 @@ __device__ void finish_argmax(QrPiv mine, QrPiv* blk, unsigned* ticket, int* piv
     piv[k] = r.a;
     const double d = key_value(r.v);
     dpiv[k] = d;
-    rpiv[k] = d > 0.0 ? 1.0 / sqrt(d) : 0.0;
+    const double root = sqrt(d);
+    rpiv[2 * k] = d > 0.0 ? 1.0 / root : 0.0;
+    rpiv[2 * k + 1] = root;
     *ticket = 0u;
   }
 }
@@ -200,10 +202,23 @@ qrcp_init_kernel(QrGeom g, double* d, QrPiv* blk, unsigned* ticket, int* piv, do
   finish_argmax(r, blk, ticket, piv, dpiv, rpiv, 0);
 }
 
+// x / b, correctly rounded, from r = RN(1 / b): the quotient x r, its exact remainder and one
+// correction (Markstein 1990, IBM J. Res. Dev. 34, 111), two operations where a division is a
+// dozen.  x r alone doubles the rounding (the picked residuals then were off by 6.4e-15 of
+// 64-bit ones instead of 6.2e-15).  Exponents near the ends of the range take the division.
+__device__ __forceinline__ double quotient(double x, double b, double r)
+{
+  const double q = x * r;
+  const int ex = (__double2hiint(x) >> 20) & 0x7ff, eq = (__double2hiint(q) >> 20) & 0x7ff;
+  if ((unsigned)(ex - 128) < 1792u && (unsigned)(eq - 128) < 1792u)
+    return fma(fma(-q, b, x), r, q);
+  return x == 0.0 ? q : x / b;
+}
+
 // Step k: column k of L, the residual update and the next pivot.  Bound by the FP64 pipe: N_o + k
-// FMAs a point and little else in FP64 -- the reciprocal root of the pivot's residual is taken
-// once (a root and a division a point were 50 operations next to 160), candidates compare as
-// integers.  L is column-major
+// FMAs a point and little else in FP64 -- the root of the pivot's residual and its reciprocal are
+// taken once (a root and a division a point were 50 operations next to 160), candidates compare
+// as integers.  L is column-major
 // (L[j * N_g + a]); a picked point has d = -inf and L(a, k) = 0 after its own step.
 __global__ void __launch_bounds__(kQrThreads, 3)   // three blocks an SM: registers for the loads
 qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k, int npts,
@@ -215,7 +230,7 @@ qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k
   double* op = pp + kw;
   double* lp = op + g.nocc;
   const int p = piv[k];
-  const double rp = rpiv[k];           // 0 where the residual is not positive
+  const double rp = rpiv[2 * k], root = rpiv[2 * k + 1];   // rp 0 where the residual is not positive
   const long long ng = g.ng;
   if (p < 0 || p >= ng) {
     // No valid pivot (every candidate residual was NaN): pass the marker on without
@@ -223,7 +238,7 @@ qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k
     if (k + 1 < npts && blockIdx.x == 0 && threadIdx.x == 0) {
       piv[k + 1] = p;
       dpiv[k + 1] = -INFINITY;
-      rpiv[k + 1] = 0.0;
+      rpiv[2 * k + 2] = rpiv[2 * k + 3] = 0.0;
     }
     return;
   }
@@ -268,7 +283,7 @@ qrcp_step_kernel(QrGeom g, double* __restrict__ L, double* __restrict__ d, int k
         s3 = fma(la[(j + 3) * ng], lp[j + 3], s3);
       }
       for (; j < k; j++) s0 = fma(la[j * ng], lp[j], s0);
-      l = (gap - ((s0 + s1) + (s2 + s3))) * rp;
+      l = quotient(gap - ((s0 + s1) + (s2 + s3)), root, rp);
       dv = fma(-l, l, dv);
     }
     L[(long long)k * ng + a] = l;
@@ -318,7 +333,7 @@ int qrcp_run(Ctx* c, const double* phi_in, long long ng, int no, const double* o
   const size_t l_bytes = sizeof(double) * (size_t)npts * ng;
   const size_t t_bytes = sizeof(double) * (size_t)(kw + nt) * ng;
   const size_t bytes = l_bytes + t_bytes + sizeof(double) * ng + sizeof(QrPiv) * nblk +
-                       (sizeof(int) + 2 * sizeof(double)) * npts + 1024;
+                       (sizeof(int) + 3 * sizeof(double)) * npts + 1024;
   char* base = (char*)ws_get(c, WS_ZT, bytes);
   if (!base) return set_error(c, THC_ERR_NOMEM, "thc_qrcp: workspace allocation failed");
   double* L = (double*)base;
@@ -328,7 +343,7 @@ int qrcp_run(Ctx* c, const double* phi_in, long long ng, int no, const double* o
   QrPiv* blk = (QrPiv*)(d + ng);
   double* dpiv = (double*)(blk + nblk);
   double* rpiv = dpiv + npts;
-  int* piv = (int*)(rpiv + npts);
+  int* piv = (int*)(rpiv + 2 * npts);
   unsigned* ticket = (unsigned*)(((uintptr_t)(piv + npts) + 255) & ~(uintptr_t)255);
   QrGeom g;
   g.phi = phit;
