@@ -247,7 +247,8 @@ __global__ void km_finish_prep(KmState* st, long long ng, int nbins_max)
     a2 += 4.0 * m * m;
   }
   st->abound = sqrt(a2);
-  st->slack32 = 1e-4 * a2;
+  // The last term is far above the rounding of squares that leave FP32's normal range.
+  st->slack32 = 1e-4 * a2 + 1e-37;
   // Spatial bins of ~128 points: cubic cells over the bounding box.
   double ext[3], vol = 1.0;
   for (int d = 0; d < 3; d++) {
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign32(KmBufs b)
   double a = st->abound;
   double e1 = 2.0 * u * (2.0 * sqrt((double)m1) * a + 5.0 * (double)m1);
   double e2 = 2.0 * u * (2.0 * sqrt((double)m2) * a + 5.0 * (double)m2);
-  if ((double)m2 - (double)m1 > e1 + e2 + 1e-300) {
+  if ((double)m2 - (double)m1 > e1 + e2 + 1e-37) {   // and squares below FP32's normal range
     b.labels[(size_t)(it & 1) * b.ng + i] = k1;
   } else {
     int slot = atomicAdd(&st->recheck_n, 1);
