@@ -78,6 +78,7 @@ struct KmState {
   int nbin[3];
   int nbins;
   double blo[3], binv[3];                // bin origin and inverse bin width
+  double org[3];                         // what the FP32 coordinates are relative to
   double slack32;                        // absolute slack of the FP32 candidate bound
   int diff_exact;                        // st->diff came from the sequential sum
   int ticket;                            // blocks of km_sums finished this iteration
@@ -238,12 +239,20 @@ __global__ void km_prep(const double* __restrict__ grid, const double* __restric
   }
 }
 
-__global__ void km_finish_prep(KmState* st, long long ng, int nbins_max)
+// relative: the pruned kernels' FP32 coordinates are taken from the lower corner of the grid's
+// bounding box, so that their rounding follows the cell's size and not its place (a cell 1e4 of
+// its edges from the origin kept every centroid of every tile: 230 ms a call at N_g 262144, N_mu
+// 2048).  The difference from the corner is rounded once in FP64, 2^-53 of itself.
+__global__ void km_finish_prep(KmState* st, long long ng, int nbins_max, bool relative)
 {
   // |a| <= |c| + |g| per component; centroids stay inside the grid's bounding box.
   double a2 = 0.0;
   for (int d = 0; d < 3; d++) {
     double m = __longlong_as_double((long long)st->absmax[d]);
+    const double lo = dunkey(st->bmin[d]), span = dunkey(st->bmax[d]) - lo;
+    const bool use = relative && isfinite(span);
+    st->org[d] = use ? lo : 0.0;
+    if (use) m = span;
     a2 += 4.0 * m * m;
   }
   st->abound = sqrt(a2);
@@ -295,6 +304,9 @@ __global__ void km_bin_count(const double* __restrict__ grid, KmBufs b)
   }
   b.pbin[i] = bin;
   atomicAdd(&b.bcount[bin], 1);
+  if (i < b.nmu)
+    for (int d = 0; d < 3; d++)
+      b.cen32[d * b.nmu + i] = (float)(b.cen[d * b.nmu + i] - st->org[d]);
 }
 
 // Single block: counts -> exclusive offsets (bcount[0..nbins)), cursors zeroed after.
@@ -342,9 +354,10 @@ __global__ void km_bin_scatter(KmBufs b)
   b.perm[pos] = (int)i;
   // The binned order's own copy of the FP32 coordinates: the pruned kernels read them
   // coalesced instead of through perm (a dependent gather).
-  b.pf[pos] = b.fx[i];
-  b.pf[b.ng + pos] = b.fy[i];
-  b.pf[2 * b.ng + pos] = b.fz[i];
+  const double* org = b.st->org;
+  b.pf[pos] = (float)(b.gx[i] - org[0]);
+  b.pf[b.ng + pos] = (float)(b.gy[i] - org[1]);
+  b.pf[2 * b.ng + pos] = (float)(b.gz[i] - org[2]);
 }
 
 // A final label of the pruned assign kernels, with the counting sort's histogram entry
@@ -1021,9 +1034,10 @@ __device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double*
     const int d = threadIdx.x;
     double* nc = b.cen + (size_t)((it + 1) & 1) * 3 * nmu;
     float* nc32 = b.cen32 + (size_t)((it + 1) & 1) * 3 * nmu;
+    const double org = st->org[d];
     const double v = __ddiv_rn(res[1 + d], res[0]);
     nc[d * nmu + k] = v;
-    nc32[d * nmu + k] = (float)v;
+    nc32[d * nmu + k] = (float)(v - org);
     red[d] = __dsub_rn(v, old);
   }
   __syncthreads();
@@ -1973,7 +1987,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   int nprep = (int)cdiv(std::max<long long>(ng, nmu), 256);
   km_prep<<<nprep, 256, 0, s>>>(grid, rho, init, b);
   THC_LAUNCHED(c, "km_prep");
-  km_finish_prep<<<1, 1, 0, s>>>(st, ng, nbins_max);
+  km_finish_prep<<<1, 1, 0, s>>>(st, ng, nbins_max, prune);
   THC_LAUNCHED(c, "km_finish_prep");
   // Spatial binning of the grid (once per call): perm lists the points bin by bin.  From 8
   // centroids on, where the tile boxes fit the map's partials (part_s): at N_g 4320, N_mu 48
