@@ -70,7 +70,6 @@ enum Slot : int {
   WS_T64_A,         // digits of dgemm's tensor-core route
   WS_T64_B,
   WS_T64_E,         // its row exponents and maxima
-  WS_T64_ERR,       // its error flag
   WS_NSLOTS
 };
 
@@ -95,8 +94,8 @@ struct Ctx {
   std::map<std::pair<int, int>, Dft> dft;
   // 4 KB pinned host scratch for asynchronous device-to-host flags.  Users (never live at
   // the same time within one call): bytes [0, 32) the k-means done flags of two blocks in
-  // flight (kmeans.cu) or the CholStatus of C (mixed.cu); bytes [kPinnedCounts, +8) the
-  // Coulomb kernel's two counts (mixed.cu).
+  // flight (kmeans.cu), the CholStatus of C (mixed.cu) or an exponent range (halfc.cu); bytes
+  // [kPinnedCounts, +8) the Coulomb kernel's two counts (mixed.cu).
   void* pinned = nullptr;
   static constexpr size_t kPinnedCounts = 64;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -113,7 +112,9 @@ struct Ctx {
   // Most bytes of digits a product of dgemm's tensor-core route holds at a time (larger ones run
   // in panels); a quarter of it for a chunk of fft_tc's.  0: neither.
   size_t digit_bytes = (size_t)3 << 30;
-  int* tc64_err = nullptr;   // device flag: a bounded wait of dgemm's tensor-core route gave up
+  // Device flag: a bounded wait of dgemm's tensor-core route gave up.  Every entry point whose
+  // products may take that route points it to a zeroed word first and reads it at its end.
+  int* tc64_err = nullptr;
   int km_prune = 1;     // 1: spatially pruned k-means assign, 0: exhaustive
   int use_graphs = 1;   // capture the k-means iteration block in a CUDA graph
   // k-step per pipeline stage of the tensor-core GEMM: 32 (2-3 stages of all slices, the

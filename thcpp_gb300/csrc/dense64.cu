@@ -589,7 +589,7 @@ static int rank64_update(Ctx* c, const GemmArgs& g)
 // Blocked Cholesky whose panel solve is a GEMM with the inverted diagonal block; the
 // inverted diagonal blocks are kept in dinv (nblk x 64 x 64) for the triangular inverse.
 int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholStatus* cs,
-              double* dinv)
+              double* dinv, bool last)
 {
   ProfScope prof(c, "potrf_inv");
   cudaStream_t s = c->stream;
@@ -606,9 +606,11 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
     double* di = dinv + (long long)(k0 / NB) * NB * NB;
     chol_diag<<<1, 256, 0, s>>>(A, ld, n, k0, thr, cs, di);
     THC_LAUNCHED(c, "chol_diag");
-    chol_diag_inv<<<NB / IW, 32 * IW, 0, s>>>(A, ld, n, k0, cs, di);
-    THC_LAUNCHED(c, "chol_diag_inv");
     int rest = n - k0 - nb;
+    if (rest > 0 || last) {
+      chol_diag_inv<<<NB / IW, 32 * IW, 0, s>>>(A, ld, n, k0, cs, di);
+      THC_LAUNCHED(c, "chol_diag_inv");
+    }
     if (rest <= 0) break;
     if (trail_pending) {     // the panel rows below were updated on the second stream
       THC_CUDA(c, cudaStreamWaitEvent(s, c->ev_trail, 0));
@@ -767,16 +769,21 @@ int refine_polynomial(Ctx* c, const double* X, int n, double s, int k, double* G
 namespace {
 
 __global__ void __launch_bounds__(1024) balance_exponents_k(const double* a, long long stride,
-                                                            int n, int* k, int* range)
+                                                            int n, int* k, int* range,
+                                                            double* scalars, bool twice)
 {
   __shared__ int lo[32], hi[32];
+  __shared__ double red[32];
   int mn = INT_MAX, mx = INT_MIN;
+  double s = 0.0;                        // summed as diag_mean_k does
   for (int i = threadIdx.x; i < n; i += 1024) {
     const double v = a[i * stride];
+    s += v;
     const int E = (__double2hiint(v) >> 20) & 0x7ff;
     const bool use = E != 0x7ff && v != 0.0;
     const int e = use ? (max(E, 1) - 1023) >> 1 : 0;
     k[i] = e;
+    if (twice) k[n + i] = e;
     if (use) {
       mn = min(mn, e);
       mx = max(mx, e);
@@ -784,9 +791,11 @@ __global__ void __launch_bounds__(1024) balance_exponents_k(const double* a, lon
   }
   mn = __reduce_min_sync(0xffffffffu, mn);
   mx = __reduce_max_sync(0xffffffffu, mx);
+  for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
   if ((threadIdx.x & 31) == 0) {
     lo[threadIdx.x >> 5] = mn;
     hi[threadIdx.x >> 5] = mx;
+    red[threadIdx.x >> 5] = s;
   }
   __syncthreads();
   if (threadIdx.x < 32) {
@@ -795,15 +804,23 @@ __global__ void __launch_bounds__(1024) balance_exponents_k(const double* a, lon
     if (threadIdx.x == 0) {
       range[0] = mn <= mx ? mn : 0;
       range[1] = mn <= mx ? mx : 0;
+      if (scalars) {
+        double t = 0.0;
+        for (int w = 0; w < 32; w++) t += red[w];
+        scalars[0] = t / n;
+        scalars[1] = 1e-13 * scalars[0];
+        scalars[2] = scalars[3] = 0.0;
+      }
     }
   }
 }
 
 }  // namespace
 
-int balance_exponents(Ctx* c, const double* a, long long stride, int n, int* k, int* range)
+int balance_exponents(Ctx* c, const double* a, long long stride, int n, int* k, int* range,
+                      double* scalars, bool twice)
 {
-  balance_exponents_k<<<1, 1024, 0, c->stream>>>(a, stride, n, k, range);
+  balance_exponents_k<<<1, 1024, 0, c->stream>>>(a, stride, n, k, range, scalars, twice);
   THC_LAUNCHED(c, "balance_exponents");
   return THC_OK;
 }

@@ -64,15 +64,12 @@ bool dgemm_tc_fits(const Ctx* c, const GemmArgs& g);
 // Runs g on the tensor cores; *done = false (and THC_OK) when it does not take it (no room
 // for the digits), and the caller runs the FMA kernel.
 int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done);
-// Clears the device flag that a bounded wait of the kernel sets (c->tc64_err).  Every entry
-// point whose products may take this route calls it first and reads the flag at its end.
-int dgemm_tc_begin(Ctx* c);
 // Split-K partials summed in split order, then the epilogue, into C.
 int dgemm_reduce_partials(Ctx* c, const GemmArgs& g);
 // Cholesky with GEMM panels; dinv receives the inverted NB x NB diagonal blocks
-// (NB = 64: ceil(n/64) x 64 x 64 doubles).
+// (NB = 64: ceil(n/64) x 64 x 64 doubles), the last one's only with `last` (chol_inverse's).
 int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholStatus* cs,
-              double* dinv);
+              double* dinv, bool last = true);
 // Cinv = (L L^T)^{-1} via X = L^{-1}; X (n x ld) and T (64 x n) are scratch.
 // With Cinv == nullptr only X = L^{-1} is formed.
 // tensor: X^T X may take the tensor-core route (other roundings than the FMA kernel's).
@@ -96,7 +93,10 @@ int refine_polynomial(Ctx* c, const double* X, int n, double s, int k, double* G
 constexpr int kBalancedBinades = 13;
 // k_i = floor(log2 sqrt|a_i|) of n values a_i, `stride` doubles apart (0 where a_i is 0 or not
 // finite), and the smallest and the largest k_i of the others in range[0..1].
-int balance_exponents(Ctx* c, const double* a, long long stride, int n, int* k, int* range);
+// scalars (optional): the mean of the a_i, the pivot threshold 1e-13 of it, and two zeros.
+// twice: the k_i once more behind (real and imaginary parts).
+int balance_exponents(Ctx* c, const double* a, long long stride, int n, int* k, int* range,
+                      double* scalars = nullptr, bool twice = false);
 int set_identity(Ctx* c, double* A, long long ld, int n);
 int add_diag_shift(Ctx* c, double* A, long long ld, int n, double rel, double* shift_out);
 int diag_mean(Ctx* c, const double* A, long long ld, int n, double* out);

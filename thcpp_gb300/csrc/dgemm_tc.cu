@@ -925,15 +925,4 @@ int dgemm_tc(Ctx* c, const GemmArgs& g, bool* done)
   return THC_OK;
 }
 
-int dgemm_tc_begin(Ctx* c)
-{
-  if (!c->tc64_err) {
-    char* p = (char*)ws_get(c, WS_T64_ERR, 256);
-    if (!p) return set_error(c, THC_ERR_NOMEM, "workspace allocation failed");
-    c->tc64_err = (int*)p;
-  }
-  THC_CUDA(c, cudaMemsetAsync(c->tc64_err, 0, sizeof(int), c->stream));
-  return THC_OK;
-}
-
 }  // namespace thc

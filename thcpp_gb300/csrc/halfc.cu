@@ -302,7 +302,7 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   double* orb_dev = out_orb ? (orb_host ? stage : out_orb) : nullptr;
   double* occ_dev = out_orb_occ ? (occ_host ? stage + 2LL * nmu * no : out_orb_occ) : nullptr;
   THC_CUDA(c, cudaMemsetAsync(scr, 0, 1024, s));
-  if ((st = dgemm_tc_begin(c))) return st;
+  c->tc64_err = bad + 1;
   THC_CUDA(c, cudaEventRecord(c->ev0, s));
   gather_pairs<<<(int)cdiv((long long)nmu * no, 256), 256, 0, s>>>(phi, ng, no, idx, nmu, pmu,
                                                                   pmu_rot, orb_dev, bad);
@@ -335,11 +335,9 @@ int isdf_half_complex_run(Ctx* c, const double* phi_in, long long ng, int no,
   THC_LAUNCHED(c, "build_augmented");
   int* bal = (int*)ws_get(c, WS_EQUIL, sizeof(int) * 2 * nmu);
   if (!bal) return set_error(c, THC_ERR_NOMEM, "thc_isdf_half_complex: workspace allocation failed");
-  int* bal_range = bad + 1;
-  if ((st = balance_exponents(c, aug, 4LL * nmu + 2, nmu, bal, bal_range))) return st;
-  THC_CUDA(c, cudaMemcpyAsync(bal + nmu, bal, sizeof(int) * nmu, cudaMemcpyDeviceToDevice, s));
-  int* h_range = (int*)c->pinned;
-  THC_CUDA(c, cudaMemcpyAsync(h_range, bal_range, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  volatile int* h_range = (int*)c->pinned;     // written by the kernel, read after the event
+  if ((st = balance_exponents(c, aug, 4LL * nmu + 2, nmu, bal, (int*)h_range, nullptr, true)))
+    return st;
   THC_CUDA(c, cudaEventRecord(c->ev_fork, s));
   // The fewest rows a thread whose blocks the 152 SMs hold at once, eight each.
   int gr = 1;

@@ -133,10 +133,6 @@ __global__ void copy_lower_to_full(const double* __restrict__ src, int n, double
   dst[e] = r >= c ? src[e] : src[(long long)c * n + r];
 }
 
-__global__ void set_scalar(double* p, double v) { *p = v; }
-
-__global__ void scale_scalar(const double* src, double f, double* dst) { *dst = f * *src; }
-
 // Complex orbitals stored as (re, im) pairs, K = 2 N_o real columns per point:
 // out[a, 2i] = Im phi_i(a), out[a, 2i + 1] = -Re phi_i(a), so that a real product of
 // the pair layout with this one is Im P = Im(Phi_mu^H Phi).
@@ -354,7 +350,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   if (out_orb) orb_dev = orb_host ? orb_stage : out_orb;
   if (half && out_orb_occ) occ_dev = occ_host ? orb_stage + 2 * (long long)nmu * no : out_orb_occ;
   THC_CUDA(c, cudaMemsetAsync(scr + 512, 0, 64, s));
-  if ((st = dgemm_tc_begin(c))) return st;
+  c->tc64_err = bad + 5;
   THC_CUDA(c, cudaEventRecord(c->ev0, s));
 
   // The Coulomb weights depend on the kernel only: with them first, their counts reach the
@@ -367,8 +363,9 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   };
   const bool fft_products = fft_tc_fits(c, n0, n1, n2, nmu);
   if ((st = weights(fft_products))) return st;
-  int h_counts[4] = {0, 0, 0, 0};      // n_anti, n_neg, the smallest and largest exponent of C's
-  int herr = 0;                        // a product of C or Z gave up waiting
+  // n_anti, n_neg, the smallest and largest exponent of C's diagonal, and whether a product gave
+  // up waiting.
+  int h_counts[5] = {};
   gather_rows<<<(int)cdiv((long long)nmu * kw, 256), 256, 0, s>>>(phi, ng, kw, idx, nmu, phimu,
                                                                   cplx ? nullptr : orb_dev, bad);
   THC_LAUNCHED(c, "gather_rows");
@@ -459,14 +456,10 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   }
   int* bal = (int*)ws_get(c, WS_EQUIL, sizeof(int) * nmu);
   if (!bal) return set_error(c, THC_ERR_NOMEM, "thc_isdf: workspace allocation failed");
-  if ((st = balance_exponents(c, C, nmu + 1, nmu, bal, bal_range))) return st;
+  // Also diag C's mean, the pivot threshold, the shift (0 so far) and M's threshold 0.
+  if ((st = balance_exponents(c, C, nmu + 1, nmu, bal, bal_range, dmean))) return st;
   // Cholesky of C with breakdown detection, then the shift policy.
   double* Lc = C + nn;
-  if ((st = diag_mean(c, C, nmu, nmu, dmean))) return st;
-  scale_scalar<<<1, 1, 0, s>>>(dmean, 1e-13, thr);
-  THC_LAUNCHED(c, "scale_scalar");
-  set_scalar<<<1, 1, 0, s>>>(shift_dev, 0.0);
-  THC_LAUNCHED(c, "set_scalar");
   int chol_c_info = 0;
   bool shifted = false;
   auto factor = [&](double rel) -> int {
@@ -483,11 +476,10 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   if ((st = factor(shift_rel > 0.0 ? shift_rel : 0.0))) return st;
   shifted = shift_rel > 0.0;
   THC_CUDA(c, cudaMemcpyAsync(h_counts, n_anti, sizeof(h_counts), cudaMemcpyDeviceToHost, s));
-  THC_CUDA(c, cudaMemcpyAsync(&herr, c->tc64_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hcs, cs, sizeof(CholStatus), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaStreamSynchronize(s));
   // Before C is judged: without its product C is whatever the workspace held.
-  if (herr) return set_error(c, THC_ERR_TIMEOUT, "thc_isdf: tensor-core GEMM wait timed out");
+  if (h_counts[4]) return set_error(c, THC_ERR_TIMEOUT, "thc_isdf: tensor-core GEMM wait timed out");
   if (hcs.flag) {
     chol_c_info = hcs.info;
     if (shift_rel < 0.0 && !shifted) {
@@ -570,15 +562,13 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   // Cholesky of M (the half-rotated M is returned as it is).
   init_chol_status<<<1, 1, 0, s>>>(csm);
   THC_LAUNCHED(c, "init_chol_status");
-  set_scalar<<<1, 1, 0, s>>>(zero, 0.0);
-  THC_LAUNCHED(c, "set_scalar");
   double* Lout = Lw;
   if (half) {
     // no factor
   } else if (h_anti == 0) {
     copy_lower_to_full<<<nb2, 256, 0, s>>>(mre, nmu, xim);
     THC_LAUNCHED(c, "copy_lower_to_full");
-    if ((st = potrf_inv(c, xim, nmu, nmu, zero, csm, dinv))) return st;
+    if ((st = potrf_inv(c, xim, nmu, nmu, zero, csm, dinv, false))) return st;
     export_l_real<<<nb2, 256, 0, s>>>(xim, nmu, Lout);
     THC_LAUNCHED(c, "export_l_real");
   } else {
@@ -592,7 +582,7 @@ int isdf_run(Ctx* c, const double* phi_in, long long ng, int no, const int* idx_
   if (out_L && !half)
     THC_CUDA(c, cudaMemcpyAsync(out_L, Lout, sizeof(double) * 2 * nn, cudaMemcpyDefault, s));
   CholStatus hm{};
-  int hbad = 0;
+  int hbad = 0, herr = 0;
   THC_CUDA(c, cudaMemcpyAsync(&herr, c->tc64_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hm, csm, sizeof(CholStatus), cudaMemcpyDeviceToHost, s));
   THC_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s));

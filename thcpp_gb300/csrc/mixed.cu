@@ -579,7 +579,7 @@ int isdf_run_mixed(Ctx* c, const double* phi_in, long long ng, int no, const int
   if (h_anti == 0) {
     copy_lower_to_full_m<<<nb2, 256, 0, s>>>(mre, nmu, xim);
     THC_LAUNCHED(c, "copy_lower_to_full");
-    if ((st = potrf_inv(c, xim, nmu, nmu, zero, csm, dinv))) return st;
+    if ((st = potrf_inv(c, xim, nmu, nmu, zero, csm, dinv, false))) return st;
     export_l_real_m<<<nb2, 256, 0, s>>>(xim, nmu, Lout);
     THC_LAUNCHED(c, "export_l_real");
   } else {
