@@ -118,7 +118,9 @@ int thc_ctx_set_stream(thc_ctx* ctx, void* cuda_stream);
  * 0 = stop and clear); "refine" (steps of iterative refinement of zeta after a shifted
  * solve of C, 0..8, default 0); "equilibrate" (mixed path: solve on C scaled to a unit-range
  * diagonal by powers of two, default 1); "overlap" (mixed path: factor C on a second stream
- * beside the P product, default 0); "spin_limit" (polls before a bounded device wait gives
+ * beside the P product, default 0); "one_stream" (1 = every launch on the context's own stream:
+ * the Cholesky's look-ahead, N_mu >= 512, without a second one, with the same results; the
+ * workers of thc_factorize_batched have it; default 0); "spin_limit" (polls before a bounded device wait gives
  * up with THC_ERR_TIMEOUT, default 2^24); "tc_hi" (drain period of the tensor-core kernel's
  * level >= 3 accumulator in 16-k steps, a power of two 1..32, default 8); "qrcp_all_pairs"
  * (half-rotated QRCP: 1 = every (occupied, orbital) pair instead of the reference's

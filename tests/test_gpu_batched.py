@@ -52,3 +52,33 @@ def test_batched_reports_per_system_errors():
     assert per[0] == capi.THC_OK
     assert per[1] == capi.THC_ERR_EMPTY_CLUSTER
     assert st == capi.THC_ERR_EMPTY_CLUSTER
+
+
+@pytest.mark.parametrize("prec", [capi.THC_PREC_FP64, capi.THC_PREC_MIXED])
+def test_batched_look_ahead(prec):
+    """N_mu 600: the Cholesky looks ahead (from 512 on), in a batch on the worker's one stream with
+    the same results to the last bit."""
+    import torch
+    r = np.random.default_rng(3)
+    mesh, norb, nmu = (16, 18, 20), 40, 600
+    ng = int(np.prod(mesh))
+    grid = np.stack(np.meshgrid(*[np.arange(float(m)) for m in mesh], indexing="ij"), -1).reshape(-1, 3)
+    dev = torch.device("cuda", 0)
+    cu = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+    systems = []
+    for _ in range(2):
+        phi = r.standard_normal((ng, norb))
+        systems.append(dict(
+            grid=cu(grid), rho=cu((phi ** 2).sum(1)), ng=ng, nmu=nmu, max_it=4, threshold=1e-9,
+            init_idx=np.sort(r.choice(ng, nmu, replace=False)).astype(np.int32), phi=cu(phi),
+            norb=norb, mesh=np.array(mesh, np.int32), coulG=cu(np.ones(ng)), shift_rel=-1.0,
+            out_idx=np.zeros(nmu, np.int32), out_orbitals=np.zeros((norb, nmu, 2)),
+            out_M=np.zeros((nmu, nmu, 2)), out_L=np.zeros((nmu, nmu, 2))))
+    torch.cuda.synchronize()
+    status, done = capi.factorize_batched(systems, precision=prec, nstreams=2)
+    assert status == capi.THC_OK
+    with capi.Context(0, prec) as ctx:
+        for s in systems:
+            got = ctx.isdf(s["phi"], s["out_idx"], mesh, s["coulG"])
+            assert got["status"] == capi.THC_OK
+            assert np.array_equal(got["M"], s["out_M"]) and np.array_equal(got["L"], s["out_L"])

@@ -333,6 +333,10 @@ int thc_ctx_set_option(thc_ctx* h, const char* key, double value)
     h->c.overlap = value != 0.0;
     return THC_OK;
   }
+  if (!strcmp(key, "one_stream")) {
+    h->c.one_stream = value != 0.0;
+    return THC_OK;
+  }
   if (!strcmp(key, "digits_mb")) {
     if (value < 0 || value > 1 << 20) return THC_ERR_ARG;
     h->c.digit_bytes = (size_t)(value * 1048576.0);
@@ -553,9 +557,10 @@ int thc_factorize_batched(int device, int precision, thc_system* sys, int nsys, 
       thc_ctx* h = nullptr;
       int st = thc_ctx_create(device, precision, &h);
       if (st) return st;
-      // The systems already overlap across the workers' streams: each worker keeps its
-      // whole factorisation on its own stream (whatever the default of "overlap").
+      // The systems already overlap across the workers' streams: each worker keeps its whole
+      // factorisation on its own stream, the Cholesky's look-ahead included.
       h->c.overlap = 0;
+      h->c.one_stream = true;
       pool.push_back(h);
     }
     workers.assign(pool.begin(), pool.begin() + nstreams);

@@ -85,6 +85,9 @@ struct Ctx {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaEvent_t ev_panel = nullptr, ev_trail = nullptr;   // Cholesky look-ahead (dense64.cu)
   int overlap = 0;
+  // Every launch on the context's one stream (workers of a batch; option "one_stream"): the
+  // Cholesky's look-ahead keeps its order and its results, without the second stream.
+  bool one_stream = false;
   void* ws[WS_NSLOTS] = {};
   size_t ws_bytes[WS_NSLOTS] = {};
   std::map<std::tuple<int, int, int, int, int>, cufftHandle> plans;  // (n0,n1,n2,batch,type)

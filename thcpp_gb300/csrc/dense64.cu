@@ -599,7 +599,7 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
   // that update.  The diagonal blocks' one-SM chain then runs beside the FP64 GEMMs on the
   // other SMs instead of between them.
   const bool la = n >= 512 && c->aux_stream && c->aux_stream != s;
-  cudaStream_t s2 = la ? c->aux_stream : s;
+  cudaStream_t s2 = la && !c->one_stream ? c->aux_stream : s;
   bool trail_pending = false;
   for (int k0 = 0; k0 < n; k0 += NB) {
     int nb = std::min(NB, n - k0);
@@ -653,8 +653,10 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
     if (rest > nb1) {
       // The rest of the trailing triangle (rows below the next diagonal block, columns from
       // it on) on the second stream, after the panel.
-      THC_CUDA(c, cudaEventRecord(c->ev_panel, s));
-      THC_CUDA(c, cudaStreamWaitEvent(s2, c->ev_panel, 0));
+      if (s2 != s) {
+        THC_CUDA(c, cudaEventRecord(c->ev_panel, s));
+        THC_CUDA(c, cudaStreamWaitEvent(s2, c->ev_panel, 0));
+      }
       GemmArgs g{};
       g.M = rest - nb1; g.N = rest; g.K = nb;
       g.A = l21 + (long long)nb1 * ld; g.sam = ld; g.sak = 1;
@@ -669,8 +671,10 @@ int potrf_inv(Ctx* c, double* A, long long ld, int n, const double* thr, CholSta
         st = dgemm(c, g);
       }
       if (st) return st;
-      THC_CUDA(c, cudaEventRecord(c->ev_trail, s2));
-      trail_pending = true;
+      if (s2 != s) {
+        THC_CUDA(c, cudaEventRecord(c->ev_trail, s2));
+        trail_pending = true;
+      }
     }
   }
   if (trail_pending) THC_CUDA(c, cudaStreamWaitEvent(s, c->ev_trail, 0));

@@ -351,7 +351,7 @@ int isdf_run_mixed(Ctx* c, const double* phi_in, long long ng, int no, const int
   bool shifted = shift_rel > 0.0;
   bool cinv_tc = !shifted && nmu >= 512;
   CholStatus* hcs_p = (CholStatus*)c->pinned;      // pinned: the copy stays asynchronous
-  const cudaStream_t fs = c->overlap ? c->aux_stream : s;
+  const cudaStream_t fs = c->overlap && !c->one_stream ? c->aux_stream : s;
   {
     if (fs != s) {
       THC_CUDA(c, cudaEventRecord(c->ev_fork, s));
