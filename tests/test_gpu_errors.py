@@ -119,3 +119,20 @@ def test_index_outside_the_grid(gpu_ctx_fp64, bad):
         gpu_ctx_fp64.isdf_half_complex(phi, np.ascontiguousarray(phi[:, :3]), idx, (10, 10, 10),
                                        np.ones(1000))
     assert e.value.status == capi.THC_ERR_ARG
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("nmu", [5, 40])
+@pytest.mark.parametrize("bad", [-1, 2000])
+def test_initial_index_outside_the_grid(request, prec, nmu, bad):
+    ctx = request.getfixturevalue("gpu_ctx_fp64" if prec == "fp64" else "gpu_ctx_mixed")
+    r = np.random.default_rng(2)
+    g, rho = r.uniform(size=(2000, 3)), r.uniform(0.5, 2.0, size=2000)
+    init = np.arange(nmu, dtype=np.int32) * 3
+    init[nmu // 2] = bad
+    with pytest.raises(capi.ThcError, match="initial index out of range") as e:
+        ctx.kmeans(g, rho, nmu, init, 5, 1e-9)
+    assert e.value.status == capi.THC_ERR_ARG
+    init[nmu // 2] = 1999
+    idx, _, status = ctx.kmeans(g, rho, nmu, init, 5, 1e-9)
+    assert status == capi.THC_OK and len(idx) == nmu

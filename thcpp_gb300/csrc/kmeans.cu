@@ -73,7 +73,7 @@ struct KmState {
   double abound;        // |a| bound of the FP32 error estimate
   unsigned long long absmax[3];
   int bad_label;
-  int pad2;
+  int bad_init;         // an initial index that is no grid point
   unsigned long long bmin[3], bmax[3];   // grid bounding box (order-preserving bit patterns)
   int nbin[3];
   int nbins;
@@ -231,6 +231,10 @@ __global__ void km_prep(const double* __restrict__ grid, const double* __restric
   }
   if (i < b.nmu) {
     long long g = init_idx[i];
+    if (g < 0 || g >= b.ng) {
+      b.st->bad_init = 1;
+      g = 0;
+    }
     for (int d = 0; d < 3; d++) {
       double v = grid[3 * g + d];
       b.cen[d * b.nmu + i] = v;
@@ -420,6 +424,10 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
   long long t = blockIdx.x * (long long)kAssignThreads + threadIdx.x;
   bool valid = t < b.ng;
   long long i = valid ? b.perm[t] : 0;
+  if ((unsigned long long)i >= (unsigned long long)b.ng) {   // reported, not used as an index
+    st->bad_label = 1;
+    i = 0;
+  }
   float g[3] = {0, 0, 0};
   int before = 0;            // the label of the iteration before
   if (valid) {
@@ -2186,6 +2194,7 @@ int kmeans_run(Ctx* c, const double* grid_in, const double* rho_in, long long ng
   // overwrite: thc_kmeans_history reports none for it.
   c->km_last_iters = fixed ? 0 : hs.iter;
   c->km_last_max_it = max_it;
+  if (hs.bad_init) return set_error(c, THC_ERR_ARG, "thc_kmeans: initial index out of range");
   if (hs.bad_label) return set_error(c, THC_ERR_CUDA, "thc_kmeans: internal label out of range");
   if (hs.empty) {
     if (stats) stats->iterations = hs.iter;
