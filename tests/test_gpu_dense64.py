@@ -96,3 +96,30 @@ def test_breakdown_position(gpu_ctx_fp64, gpu_ctx_mixed, prec, pos):
     idx[pos] = idx[pos - 1]
     r = ctx.isdf(s.phi, idx, s.mesh, s.coulG)
     assert r["stats"].chol_c_info == pos + 1 and r["stats"].rank_deficient == 1
+
+
+@pytest.mark.parametrize("kind", ["real", "half", "complex"])
+def test_c_keeps_the_fma_kernels_rounding(gpu_ctx_fp64, kind):
+    """C = Z[:, idx] at a size whose other products are on the tensor cores: its factor, and so the
+    pivots, are the FMA route's to the last bit."""
+    r = np.random.default_rng(8)
+    mesh, no, nmu = (16, 16, 20), 64, 640
+    phi = r.standard_normal((int(np.prod(mesh)), no))
+    idx = np.sort(r.choice(len(phi), nmu, replace=False)).astype(np.int32)
+    v = np.ones(len(phi))
+    pivot = {}
+    for tc in (1, 0):
+        gpu_ctx_fp64.set_option("gemm_tc", tc)
+        try:
+            if kind == "half":
+                got = gpu_ctx_fp64.isdf_half(phi, np.ascontiguousarray(phi[:, :40]), idx, mesh, v)
+            elif kind == "complex":
+                pc = phi + 1j * np.roll(phi, 7, axis=0)
+                got = gpu_ctx_fp64.isdf_complex(np.ascontiguousarray(pc), idx, mesh, v)
+            else:
+                got = gpu_ctx_fp64.isdf(phi, idx, mesh, v)
+        finally:
+            gpu_ctx_fp64.set_option("gemm_tc", 1)
+        assert got["status"] == 0
+        pivot[tc] = got["stats"].c_min_pivot
+    assert pivot[1] == pivot[0] > 0
