@@ -85,3 +85,18 @@ def test_complex_half_rotated_solve(gpu_ctx_fp64, s):
         m = got["M"][..., 0] + 1j * got["M"][..., 1]
         err[tc] = np.linalg.norm(m * np.outer(d, d) - ref) / np.linalg.norm(ref)
     assert err[1] < 2 * err[0] + 2 * _tolerance(phi, idx, d)
+
+
+@pytest.mark.parametrize("binades", [-220, -100, 100, 220])
+def test_orbitals_of_any_size(gpu_ctx_fp64, binades):
+    """zeta does not change when all orbitals are scaled (C as the fourth power, Z with it)."""
+    phi, idx, d = _fragments(30, 5)
+    ng = len(phi)
+    zeta = []
+    for f in (1.0, 2.0 ** binades):
+        r = gpu_ctx_fp64.isdf(phi * f, idx, MESH, np.ones(ng), 0.0)
+        assert r["status"] == capi.THC_OK
+        zeta.append(gpu_ctx_fp64.interpolating_vectors(ng, NMU))
+    err = np.linalg.norm(d[:, None] * (zeta[1] - zeta[0]), axis=0)
+    err /= np.linalg.norm(d[:, None] * zeta[0], axis=0)
+    assert err.max() < 2 * _tolerance(phi, idx, d)

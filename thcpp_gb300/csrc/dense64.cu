@@ -1,5 +1,6 @@
-// FP64 dense linear algebra on CUDA cores: GEMM, blocked Cholesky and triangular
-// solves.  These carry the all-FP64 path, which replaces the reference's ScaLAPACK
+// FP64 dense linear algebra on CUDA cores: GEMM (products of little work, with known zeros or a
+// flag; the others go to dgemm_tc.cu), blocked Cholesky and the triangular inverse.  These and the
+// digit products carry the all-FP64 path, which replaces the reference's ScaLAPACK
 // calls one for one:
 //   pzgemm 'C','N'  (P = Phi_mu^H Phi, src/interpolating_vectors.cpp:117)  -> dgemm + square
 //   pzgels 'N'      (least squares C X = Z, :416)             -> potrf_inv + chol_inverse + dgemm

@@ -12,12 +12,15 @@
 // The tensor cores sum V_l in FP32, exactly for l <= 4: over the 192 k between two drains
 // |V_l| <= 5 192 2^14 < 2^24.  Levels 5 to 7 (weight <= 2^-40) could pass 2^24 only with
 // digits of one sign throughout, and then round by less than 2^-55 of the sum.  A drain adds the
-// sums to 96-bit integers in registers, which hold the sum over any K without rounding, so C is
-// the correctly rounded value of the truncated expansion: about 2^-57 sqrt(K) off relative to
-// 2^{eA+eB}, where a chain of FP64 FMAs over terms of that size is 2^-54 sqrt(K) and more.
+// sums to 96-bit integers in registers, which hold the sum over any K without rounding; it is
+// rounded once, half away from zero, a negative one taken one unit (2^-70 2^{eA+eB}) smaller.  C is
+// about 2^-57 sqrt(K) off relative to 2^{eA+eB}, where a chain of FP64 FMAs over terms of that
+// size is 2^-54 sqrt(K) and more.  Where a row's entries meet small ones of the other operand
+// only, the FMAs' error, relative to the terms, is the smaller one: operands that scale against
+// each other along k are balanced first (GemmArgs::kexp; kBalancedBinades in dense64.cuh).
 //
-// Measured against the FMA kernel of dense64.cu, cut and product together (random operands;
-// errors relative to |a||b| of an entry's row and column, root mean square):
+// Measured against the FMA kernel of dense64.cu, cut and product together (random operands of one
+// size; errors relative to |a||b| of an entry's row and column, root mean square):
 //     M x N x K                     FMA              tensor cores
 //     256 x 110592 x 256            11.8 ms 3.4e-17  0.54 ms 3.7e-18   (27 TFLOP/s)
 //     256 x 110592 x 32, squared    1.54 ms 3.5e-17  0.21 ms 9.9e-18
@@ -56,6 +59,10 @@ constexpr int kStgBytes = kEpiWarps * 32 * 8 * 8;   // results on their way to c
 constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + kStgBytes + 256 + 1024 + 8192;
 static_assert(kSmem <= 227 * 1024, "shared memory");
 static_assert(kStageBytes % 1024 == 0, "stage alignment");
+// Level 4 is exact in FP32 between two drains, and level 0 (|S T| <= 2^14 a term) stays within the
+// 2^22 that the epilogue's addition of 1.5 2^23 takes.
+static_assert(5LL * kPeriod * kBK * (1 << 14) < (1 << 24), "exact levels");
+static_assert((long long)kPeriod * kBK * (1 << 14) <= (1 << 22), "level 0");
 
 constexpr long long kPair = 0x8b400000LL;  // 257 x the bits of 1.5 2^23, modulo 2^32
 
@@ -344,7 +351,7 @@ __device__ __forceinline__ double to_double(unsigned w0, unsigned w1, unsigned w
 // and is issued alone: 0.996 ms for the zeta product at N_g 110592, N_mu 256, against 0.47 at
 // once with these and 0.38 now).  Stages of 32 k with the 64-byte swizzle are 5 % faster than
 // stages of 16 k with the 32-byte one.
-// Every 160 k the levels are drained from the highest down; the next stage multiplies the
+// Every kPeriod stages (192 k) the levels are drained from the highest down; the next stage multiplies the
 // lowest digits of A first and so follows the drain level by level instead of waiting for
 // all of it.  Every wait is bounded (spin_limit); after one gives up, the kernel sets the
 // error flag, waits for its own copies and MMAs, frees TMEM and returns.

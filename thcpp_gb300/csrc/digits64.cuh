@@ -85,7 +85,7 @@ __device__ __forceinline__ unsigned digit_pair(unsigned w0, unsigned w1, int n)
 }
 
 // Digit storage: [k / 32][digit][row][32] BF16, rows padded to 128 and k to 32 with zeros,
-// so that the 16-k tile of 128 rows and all digits is one box of a 3-D tensor map.
+// so that the 32-k tile of 128 rows and all digits is one box of a 3-D tensor map.
 struct Digits {
   __nv_bfloat16* s = nullptr;
   int* e = nullptr;

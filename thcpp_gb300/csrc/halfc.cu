@@ -11,9 +11,9 @@
 // M is HalfTransformedMuv, written without a Cholesky factor (dump_thc_data, :317-328).
 //
 // C has full rank for a sensible point set but no symmetry, so the reference's QR solve is
-// replaced by the inverse from Gauss-Jordan elimination with partial pivoting (one pivot
-// kernel and one elimination kernel per column, on [C | I]; N_mu^3 complex FMAs, small next
-// to the N_mu^2 N_g of the products), then X = C^{-1} Z.  Complex values are (re, im) pairs; P
+// replaced by the inverse from Gauss-Jordan elimination with partial pivoting (one kernel per
+// column, gj_step, on [C | I] from one buffer into another; N_mu^3 complex FMAs, small next to
+// the N_mu^2 N_g of the products), then X = C^{-1} Z.  Complex values are (re, im) pairs; P
 // and Z are kept as their real N_mu x N_g matrix and the imaginary one behind it, so that every
 // complex product is one real GEMM (of twice the rows, or the terms) with each operand cut
 // once.  IVMG(G) = IVG(-G), so one transform serves both.

@@ -11,11 +11,14 @@
 //
 // GPU formulation (all buffers resident in HBM, row-major):
 //   Phi (N_g x N_o) -> Phi_mu (N_mu x N_o) gather
-//   C  = (Phi_mu Phi_mu^T)^2              FP64 GEMM, square epilogue
+//   C  = (Phi_mu Phi_mu^T)^2              FP64 FMAs, square epilogue
 //   Z^T = (Phi_mu Phi^T)^2                 FP64 GEMM, square epilogue (N_mu x N_g)
-//   L_C = chol(C + shift I); C^{-1} by forward/backward substitution on I
+//   L_C = chol(C + shift I); X = L_C^{-1} by block rows, C^{-1} = X^T X
 //   zeta^T = C^{-1} Z^T                     (N_mu x N_g; each row is one 3-D field)
-//   zeta_hat = batched R2C (cuFFT D2Z)      (N_mu x N_c complex, N_c = n0 n1 (n2/2+1))
+//   zeta_hat = batched R2C                  (N_mu x N_c complex, N_c = n0 n1 (n2/2+1))
+// The FP64 GEMMs of enough work run as exact digit products on the tensor cores (dgemm_tc.cu), the
+// transforms as products with DFT matrices (fft_tc.cu) or cuFFT D2Z; zeta's operands are balanced
+// by powers of two first.
 //   M = sum_half w [v_sym Re(a) + i v_anti Im(a)],  a = conj(zh_mu) zh_nu,
 //       which equals the reference's full C2C sum for any v(G) (v_sym / v_anti are the
 //       even / odd parts of v under G -> -G; v_anti != 0 only where the fftfreq mesh

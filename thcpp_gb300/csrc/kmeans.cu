@@ -27,13 +27,15 @@
 //     bitmap per cluster, km_cluster), then each cluster's members are accumulated in
 //     that order by segment walks, which reproduce the sequential loop's rounding
 //     exactly (segsum.cuh, seqsum.cuh);
-//   * the normed difference that is reported is the sequential sum in index order (again
-//     warp_seqsum); the per-iteration convergence test uses a fixed-order approximation
-//     and falls back to the exact sum whenever the two could decide differently.
-// Mixed precision: an FP32 pass keeps the best and second-best squared distance and
-// accepts its argmin only when the gap exceeds a proven bound on the FP32 error;
-// every other point is queued and resolved by a warp-parallel FP64 scan with the exact
-// semantics above.  The labels, and hence every later result, equal the FP64 path's.
+//   * the normed difference that is reported for the last iteration is the sequential sum in
+//     index order (again warp_seqsum); the per-iteration convergence test uses an approximation
+//     from integer sums and falls back to the exact sum whenever the two could decide differently.
+// From 8 centroids on, in both precisions (km_assign_p): an FP32 pass over the centroids that a
+// tile's box leaves keeps the best and second-best squared distance and accepts its argmin only
+// when the gap exceeds a proven bound on the FP32 error; every other point is resolved at once by
+// its warp with the exact FP64 semantics above.  Below, or with km_prune = 0: the FP64 scan, or
+// (mixed precision) an FP32 pass whose near ties are queued for one.  The labels, and hence every
+// later result, are the same whichever is taken.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
@@ -389,12 +391,12 @@ constexpr int kWarpMax = 64;      // and per warp
 //
 // A tile is 256 consecutive points of the binned order, its bounding box (b.box) made once per
 // call.  With lb(c) / ub(c) the smallest / largest squared distance from centroid c to the box
-// and U = min_c ub(c), a centroid with lb(c) > U (1 + 1e-4) + slack, slack = 1e-4 |a|^2, is
+// and U = min_c ub(c), a centroid with lb(c) > U (1 + 1e-4) + slack, slack = 1e-4 |a|^2 + 1e-37, is
 // farther from every point of the tile than its nearest centroid by a margin far above the
 // rounding of the FP32 bounds and of the FP64 distance, so it can neither win nor tie after
 // sqrt.  Of the kept centroids, in ascending index order, each thread takes the nearest in FP32
 // with the gap to the second: with u = 2^-24,
-//   |d2_32 - d2_64| <= u (2 |d| |a| + 5 d2) + O(u^2),   a_i = |c_i| + |g_i|,
+//   |d2_32 - d2_64| <= u (2 |d| |a| + 5 d2) + O(u^2),   a_i = |c_i| + |g_i| from the box's corner,
 // so a gap above 2 E(m2), E(m) = 2u (2 sqrt(m) |a| + 5 m) (a factor 2 for the O(u^2)
 // terms), proves that every other centroid is strictly farther in FP64, hence also after sqrt.
 // Other points are resolved at once in FP64 by their whole warp, one at a time, with the
