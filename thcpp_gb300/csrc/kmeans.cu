@@ -426,10 +426,6 @@ __global__ void __launch_bounds__(kAssignThreads) km_assign_p(KmBufs b)
   long long t = blockIdx.x * (long long)kAssignThreads + threadIdx.x;
   bool valid = t < b.ng;
   long long i = valid ? b.perm[t] : 0;
-  if ((unsigned long long)i >= (unsigned long long)b.ng) {   // reported, not used as an index
-    st->bad_label = 1;
-    i = 0;
-  }
   float g[3] = {0, 0, 0};
   int before = 0;            // the label of the iteration before
   if (valid) {
@@ -1027,6 +1023,13 @@ __device__ __forceinline__ double old_coordinate(const KmBufs& b, int k, int it)
 {
   return threadIdx.x < 3 ? b.cen[((size_t)(it & 1) * 3 + threadIdx.x) * b.nmu + k] : 0.0;
 }
+// The FP32 coordinates' origin, for threads 0..2: loaded with the state at a kernel's start, it
+// waits for sums_finish in red[kOrg ..], past the warps' entries (in a register it spills).
+constexpr int kOrg = 29;
+__device__ __forceinline__ double origin(const KmState* st)
+{
+  return threadIdx.x < 3 ? st->org[threadIdx.x] : 0.0;
+}
 
 // End of an iteration's sums for cluster k (whole block; res[0..3] = w, x, y, z sums): the
 // new centroid, its squared move, and -- in the last block to finish, found by a ticket in
@@ -1043,14 +1046,17 @@ __device__ void sums_finish(const KmBufs& b, int k, int it, double* res, double*
   if (threadIdx.x < 3) {   // one coordinate each: c_d = sum_d / w (the reference's division)
     const int d = threadIdx.x;
     double* nc = b.cen + (size_t)((it + 1) & 1) * 3 * nmu;
-    float* nc32 = b.cen32 + (size_t)((it + 1) & 1) * 3 * nmu;
-    const double org = st->org[d];
     const double v = __ddiv_rn(res[1 + d], res[0]);
     nc[d * nmu + k] = v;
-    nc32[d * nmu + k] = (float)(v - org);
     red[d] = __dsub_rn(v, old);
+    red[kOrg - 3 + d] = v;
   }
   __syncthreads();
+  if (threadIdx.x - 32 < 3u) {   // another warp, beside the ticket
+    const int d = threadIdx.x - 32;
+    float* nc32 = b.cen32 + (size_t)((it + 1) & 1) * 3 * nmu;
+    nc32[d * nmu + k] = (float)(red[kOrg - 3 + d] - red[kOrg + d]);
+  }
   if (threadIdx.x == 0) {
     if (res[0] < 1e-8) atomicExch(&st->empty, 1);
     double sq = 0.0;
@@ -1173,6 +1179,7 @@ __global__ void __launch_bounds__(kSumThreads) km_sums(KmBufs b)
   const int tq = warp / kSumWins, tw = warp % kSumWins;   // this warp's window task
   const int k = blockIdx.x;
   const int s = b.start[k], n = b.total[k];
+  if (threadIdx.x < 3) red[kOrg + threadIdx.x] = origin(b.st);
   const double old = old_coordinate(b, k, it);
   if (threadIdx.x < 4) sm.acc[threadIdx.x] = 0.0;
   for (int base = 0; base < n; base += kSumCap) {
@@ -1274,12 +1281,14 @@ __global__ void __launch_bounds__(128 * NW, 1024 / (128 * NW)) km_cluster(KmBufs
   extern __shared__ __align__(16) unsigned char cl_smem[];
   ClusterSmem<NW, NWIN>& sm = *reinterpret_cast<ClusterSmem<NW, NWIN>*>(cl_smem);
   const int done = st->done, it = st->iter;
+  const double org = origin(st);
   const int k = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // This warp's quantity and first window.
   const int tq = warp & 3, tw = warp >> 2;
   unsigned* mk = b.mask + (size_t)k * b.nwt;
   unsigned word = lane < b.nwt ? mk[lane] : 0u;
   if (done) return;
+  if (tid < 3) sm.red[kOrg + tid] = org;
   const int* lab = b.labels + (size_t)(it & 1) * b.ng;
   const double old = old_coordinate(b, k, it);
   if (warp == 0) {
@@ -1591,6 +1600,7 @@ __global__ void __launch_bounds__(128) km_swalk(KmBufs b)
   const int it = st->iter;
   const int k = blockIdx.x, q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w0 = b.wbase[k], w1 = b.wbase[k + 1];
+  if (threadIdx.x < 3) red[kOrg + threadIdx.x] = origin(st);
   const double* t = b.sv + (size_t)q * b.ng;
   const double old = old_coordinate(b, k, it);
   double acc = 0.0;
