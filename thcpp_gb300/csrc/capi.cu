@@ -21,6 +21,29 @@
 
 namespace thc {
 
+// The pool keeps freed memory reserved (release threshold = max), possibly in pieces too small for
+// a request: returns what no allocation uses.  The whole device first: trimming may then release
+// nothing that a kernel of another stream or context still uses.
+static void trim_pool(Ctx* c)
+{
+  cudaMemPool_t pool;
+  if (cudaDeviceSynchronize() != cudaSuccess ||
+      cudaDeviceGetDefaultMemPool(&pool, c->device) != cudaSuccess ||
+      cudaMemPoolTrimTo(pool, 0) != cudaSuccess)
+    cudaGetLastError();
+}
+
+void digits_release(Ctx* c)
+{
+  for (Slot t : {WS_T64_A, WS_T64_B})
+    if (c->ws[t]) {
+      cudaFreeAsync(c->ws[t], c->stream);
+      c->ws[t] = nullptr;
+      c->ws_bytes[t] = 0;
+    }
+  trim_pool(c);
+}
+
 void* ws_get(Ctx* c, Slot s, size_t bytes)
 {
   // Stream-ordered allocation: growing a slot neither synchronises the device nor stalls
@@ -39,24 +62,13 @@ void* ws_get(Ctx* c, Slot s, size_t bytes)
     cudaGetLastError();
     if (cudaMallocAsync(&p, bytes, c->stream) != cudaSuccess) {
       cudaGetLastError();
-      // The digits of the FP64 tensor-core products are optional: what asks for anything else than
-      // they and what is used with them holds no pointer to them.
+      // What asks for anything else than the digits of the FP64 tensor-core products and what is
+      // used with them holds no pointer to them.
       if (s != WS_T64_A && s != WS_T64_B && s != WS_T64_E && s != WS_DPART && s != WS_FFTWORK)
-        for (Slot t : {WS_T64_A, WS_T64_B})
-          if (c->ws[t]) {
-            cudaFreeAsync(c->ws[t], c->stream);
-            c->ws[t] = nullptr;
-            c->ws_bytes[t] = 0;
-          }
-      // The pool keeps freed memory reserved (release threshold = max), possibly in pieces
-      // too small for this request: return what no allocation uses and try once more.
-      // The whole device first: trimming may then release nothing that a kernel of another
-      // stream or context still uses.
-      cudaMemPool_t pool;
-      if (cudaDeviceSynchronize() != cudaSuccess ||
-          cudaDeviceGetDefaultMemPool(&pool, c->device) != cudaSuccess ||
-          cudaMemPoolTrimTo(pool, 0) != cudaSuccess ||
-          cudaMallocAsync(&p, bytes, c->stream) != cudaSuccess) {
+        digits_release(c);
+      else
+        trim_pool(c);
+      if (cudaMallocAsync(&p, bytes, c->stream) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
       }

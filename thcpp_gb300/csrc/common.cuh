@@ -189,6 +189,10 @@ struct ProfScope {
 // Grow-only workspace slot; returns nullptr on allocation failure.
 void* ws_get(Ctx* c, Slot s, size_t bytes);
 
+// Gives the digits of the FP64 tensor-core products back (they are optional), and what the pool
+// holds unused: before a second try at an allocation that is not.
+void digits_release(Ctx* c);
+
 int set_error(Ctx* c, int status, const char* fmt, ...);
 
 // Record a CUDA error after launches (cudaGetLastError).

@@ -555,6 +555,10 @@ int dgemm(Ctx* c, const GemmArgs& g_in)
     choose_tile(g);
     if (g.ksplit > 1) {
       g.part = (double*)ws_get(c, WS_DPART, sizeof(double) * g.ksplit * g.M * g.N);
+      if (!g.part) {
+        digits_release(c);
+        g.part = (double*)ws_get(c, WS_DPART, sizeof(double) * g.ksplit * g.M * g.N);
+      }
       if (!g.part) return set_error(c, THC_ERR_NOMEM, "dgemm: split-K partials");
     }
   }

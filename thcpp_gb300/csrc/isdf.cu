@@ -208,8 +208,18 @@ int get_plan(Ctx* c, int n0, int n1, int n2, int batch, cufftType type, cufftHan
     size_t work = 0;
     // Real-to-complex outputs are half spectra; complex-to-complex ones full grids.
     const long long odist = type == CUFFT_Z2Z ? ng : nc;
-    cufftResult r = cufftMakePlanMany64(p, 3, n, nullptr, 1, ng, nullptr, 1, odist, type, batch,
-                                        &work);
+    auto make = [&]() {
+      return cufftMakePlanMany64(p, 3, n, nullptr, 1, ng, nullptr, 1, odist, type, batch, &work);
+    };
+    cufftResult r = make();
+    if (r == CUFFT_ALLOC_FAILED) {       // the plan's own tables: with the digits given back
+      cufftDestroy(p);
+      cudaGetLastError();
+      digits_release(c);
+      if (cufftCreate(&p) != CUFFT_SUCCESS) return set_error(c, THC_ERR_CUFFT, "cufftCreate failed");
+      cufftSetAutoAllocation(p, 0);
+      r = make();
+    }
     if (r != CUFFT_SUCCESS) {
       cufftDestroy(p);
       return set_error(c, THC_ERR_CUFFT, "cufftMakePlanMany64 failed (%d)", (int)r);
@@ -218,6 +228,10 @@ int get_plan(Ctx* c, int n0, int n1, int n2, int batch, cufftType type, cufftHan
     c->plan_work[key] = work;
   }
   void* wa = ws_get(c, WS_FFTWORK, c->plan_work[key]);
+  if (!wa) {
+    digits_release(c);
+    wa = ws_get(c, WS_FFTWORK, c->plan_work[key]);
+  }
   if (!wa) return set_error(c, THC_ERR_NOMEM, "cuFFT work area");
   if (cufftSetWorkArea(p, wa) != CUFFT_SUCCESS || cufftSetStream(p, c->stream) != CUFFT_SUCCESS)
     return set_error(c, THC_ERR_CUFFT, "cuFFT work area / stream");
