@@ -351,9 +351,9 @@ __device__ __forceinline__ double to_double(unsigned w0, unsigned w1, unsigned w
 // and is issued alone: 0.996 ms for the zeta product at N_g 110592, N_mu 256, against 0.47 at
 // once with these and 0.38 now).  Stages of 32 k with the 64-byte swizzle are 5 % faster than
 // stages of 16 k with the 32-byte one.
-// Every kPeriod stages (192 k) the levels are drained from the highest down; the next stage multiplies the
-// lowest digits of A first and so follows the drain level by level instead of waiting for
-// all of it.  Every wait is bounded (spin_limit); after one gives up, the kernel sets the
+// Every kPeriod stages (192 k) the levels are drained from the highest down; the next stage
+// multiplies the lowest digits of A first and so follows the drain level by level instead of
+// waiting for all of it.  Every wait is bounded (spin_limit); after one gives up, the kernel sets the
 // error flag, waits for its own copies and MMAs, frees TMEM and returns.
 // Digit i of A times digits j .. j + CNT - 1 of B, into levels i + j and up; a0 / b0 are the
 // low descriptor words of the stage's operands.
@@ -849,7 +849,8 @@ int digits_product(Ctx* c, const Digits& a, const Digits& b, const GemmArgs& g)
 
 bool dgemm_tc_fits(const Ctx* c, const GemmArgs& g)
 {
-  if (!c->gemm_tc || g.fma_only || (g.kexp && g.dk) || g.skip_flag || g.a_zero_below || g.b_zero_below ||
+  if (!c->gemm_tc || g.fma_only || (g.kexp && g.dk) || g.skip_flag || g.a_zero_below ||
+      g.b_zero_below ||
       g.lower_offset || g.no_split || g.ksplit > 1 || g.part || (g.lower_only && g.M != g.N))
     return false;
   return 2.0 * (double)g.M * (double)g.N * (double)g.K >= kDgemmTcFlops && g.K >= 8;

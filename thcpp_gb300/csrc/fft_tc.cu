@@ -195,7 +195,7 @@ int fft_tc(Ctx* c, int n0, int n1, int n2, int count, bool real, const double* i
   const long long kz = oz_pad_k(kin), ky = oz_pad_k(2 * n1), kx = oz_pad_k(2 * n0);
   const size_t per = kNS * sizeof(__nv_bfloat16);
   const long long dig = std::max({rz * kz, ry * ky, rx * kx});         // per field
-  const int F = (int)std::min<long long>(count, (long long)(c->digit_bytes / 4 / (dig * per)));
+  const int F = (int)std::min<long long>(count, (long long)(std::min(c->digit_bytes / 4, kFftTcChunk) / (dig * per)));
   if (F < 1) return THC_OK;
   auto padded = [&](long long rows, long long kp) { return (size_t)oz_pad_mn(F * rows) * kp * per; };
   const long long e_rows = oz_pad_mn(F * rz) + oz_pad_mn(F * ry) + oz_pad_mn(F * rx);
